@@ -16,7 +16,7 @@
 #include "b2e_csr.h"
 #include "b2e_roots.h"
 #include "b2e_fft.h"
-#include "b2e_elements.cuh"
+#include "b2e_fast.cuh"
 #include "b2e_kernels.h"
 #include "b2e_sg.h"
 #include "b2e_wakenet.h"
@@ -172,6 +172,50 @@ __global__ void csr_entry_kernel(DevParticles P, int64_t n, double *beta0, const
   beta0[i] = b0;
 }
 
+/* a slice of the bend from slopes to slopes: the general form, out of line (for
+ * other integration orders and particles near a limit), and the straight-line
+ * one, which leaves the particle alone where it does not apply */
+struct SlicePart {
+  double X, XP, Y, YP, DP, dist;
+};
+static __device__ __noinline__ int csr_slice_general(SlicePart *p, const DevElem *ep, const DevAperture *ap) {
+  const DevElem &e = *ep;
+  const double *c = e.c;
+  double f = (1 + p->DP) / sqrt((1 + p->XP * p->XP) + p->YP * p->YP);
+  double Q1 = p->XP * f, Q3 = p->YP * f;
+  const RadSite no_rad = {0, 0, 0, 0, 0, nullptr};
+  const int lost = csbend_integrate<false>(p->X, Q1, p->Y, Q3, p->dist, p->DP, c, 1, (int)c[CB_NSUB], false, ap, e,
+                                           no_rad);
+  f = 1 / sqrt(((1 + p->DP) * (1 + p->DP) - Q1 * Q1) - Q3 * Q3);
+  p->XP = Q1 * f;
+  p->YP = Q3 * f;
+  return lost;
+}
+
+__device__ __forceinline__ bool csr_slice_fast(SlicePart &pio, const DevElem &e, const DevAperture *ap) {
+  SlicePart p = pio;
+  const double A = 1 + p.DP;
+  double r, ir, f;
+  r = fp_sqrt_recip((1 + p.XP * p.XP) + p.YP * p.YP, ir);
+  bool ok = fp_abs_hi(p.X) < FP_HI_2P100 && fp_plain(p.XP, FP_HI_2) && fp_plain(p.YP, FP_HI_2) &&
+            fp_within(A, FP_HI_2M4, FP_HI_2P4) && !fp_edge(r);
+  f = fp_quot(A, r, ir);
+  p.XP = p.XP * f;
+  p.YP = p.YP * f;
+  /* a kick adds a zero to QY, which a negative zero would not survive */
+  ok = ok && fp_hi(p.YP) != 0x80000000u;
+  ok = bend_slices_fast<false, 4>(p.X, p.XP, p.Y, p.YP, p.dist, A, 0.0, e.c, 1, 4, ap, e) && ok;
+  const double d = (A * A - p.XP * p.XP) - p.YP * p.YP;
+  r = fp_sqrt_recip(d, ir);
+  ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10) && !fp_edge(r);
+  f = fp_quot(1.0, r, ir);
+  p.XP = p.XP * f;
+  p.YP = p.YP * f;
+  if (ok)
+    pio = p;
+  return ok;
+}
+
 /* one kick: optional wake kick of the previous kick, one integrator slice,
  * c*t update, min/max of c*t (csbend.c:2385-2450, :3066-3076) */
 /* 64 registers (4 blocks of 256 per SM): twice the resident warps of the
@@ -189,31 +233,27 @@ __global__ void __launch_bounds__(256, 4) csr_slice_kernel(DevParticles P, int64
   if (alive) {
     const DevElem &e = *ep;
     const double *c = e.c;
-    double X = P.x[i], XP = P.xp[i], Y = P.y[i], YP = P.yp[i], DP = P.dp[i], f, Q1, Q3, Q4;
+    SlicePart p = {P.x[i], P.xp[i], P.y[i], P.yp[i], P.dp[i], 0};
     CT = P.s[i];
     if (apply_kick)
-      DP = csr_kick(CT, X, DP, st, nBins, Po, c[CB_RHO0]);
-    f = (1 + DP) / sqrt((1 + XP * XP) + YP * YP);
-    Q1 = XP * f;
-    Q3 = YP * f;
-    const RadSite no_rad = {0, 0, 0, 0, 0, nullptr};
-    const int nsub = (int)c[CB_NSUB];
-    int lost = nsub == 4 ? csbend_integrate<false, 4>(X, Q1, Y, Q3, Q4, DP, c, 1, nsub, false, ap, e, no_rad)
-                         : csbend_integrate<false>(X, Q1, Y, Q3, Q4, DP, c, 1, nsub, false, ap, e, no_rad);
-    f = 1 / sqrt(((1 + DP) * (1 + DP) - Q1 * Q1) - Q3 * Q3);
-    Q1 = Q1 * f;
-    Q3 = Q3 * f;
-    P.x[i] = X;
-    P.xp[i] = Q1;
-    P.y[i] = Y;
-    P.yp[i] = Q3;
-    P.dp[i] = DP;
+      p.DP = csr_kick(CT, p.X, p.DP, st, nBins, Po, c[CB_RHO0]);
+    int lost = 0;
+    if (!((e.flags & EF_FAST) && c[CB_NSUB] == 4 && csr_slice_fast(p, e, ap))) {
+      SlicePart t = p;
+      lost = csr_slice_general(&t, &e, ap);
+      p = t;
+    }
+    P.x[i] = p.X;
+    P.xp[i] = p.XP;
+    P.y[i] = p.Y;
+    P.yp[i] = p.YP;
+    P.dp[i] = p.DP;
     if (lost) {
       P.lost_pass[i] = pass;
       P.lost_elem[i] = elem_index;
       alive = false;
     } else {
-      CT = CT + Q4 / beta0[i];
+      CT = CT + p.dist / beta0[i];
       P.s[i] = CT;
     }
   }

@@ -62,6 +62,9 @@ enum {
 #define EF_SKEW_KICK 0x100000   /* CSBEND with YKICK: the skew dipole term RB_SKEW0 in Fx */
 #define EF_EDGE1_SIMPLE 0x200000 /* CSBEND EDGE1_EFFECTS 3: applySimpleDipoleEdgeKick */
 #define EF_EDGE2_SIMPLE 0x400000 /* CSBEND EDGE2_EFFECTS 3 */
+#define EF_FAST 0x800000        /* KMULT / CSBEND / CSRCSBEND: the straight-line forms of b2e_fast.cuh apply */
+#define EF_EDGE1_FLAT 0x1000000 /* CSBEND: entrance edge of zero angle and no fringe */
+#define EF_EDGE2_FLAT 0x2000000 /* CSBEND: exit edge of zero angle and no fringe */
 
 /* KMULT constant slots */
 #define KM_ORDER 0       /* 1 quad, 2 sext */
@@ -210,6 +213,8 @@ typedef struct {
 typedef struct {
   double x_max, y_max;
   double a2, b2;        /* ipow(x_max, xe), ipow(y_max, ye) */
+  double inv_x, inv_y;  /* 1/x_max, 1/y_max for ap_surely_inside: 0 where a half-axis is not
+                         * checked, infinite where the quick test does not apply */
   int32_t elliptical, xe, ye;
   int32_t mode; /* check after the element: 0 none, 1 rectangular, 2 elliptical */
 } DevAperture;

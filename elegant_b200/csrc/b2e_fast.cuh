@@ -1,0 +1,444 @@
+/*
+ * Straight-line forms of the KQUAD/KSEXT and CSBEND maps for the particles
+ * that stay well inside every limit, which is nearly all of them on nearly
+ * every element.  Same expressions in the same order as kmult and csbend
+ * (b2e_elements.cuh), bit for bit, with the divisions and square roots of
+ * b2e_fp64.cuh, which share seeds and reciprocals and hold no branches.
+ *
+ * A form returns false, and leaves the particle untouched, when anything
+ * leaves the range it was written for: an aperture (or a place too near its
+ * edge to tell cheaply), a coordinate, slope or angle limit, a loss, a
+ * non-finite or extremely small value, a significand the reciprocals do not
+ * round correctly.  The caller then runs the general map from the element's
+ * entrance, which finds the loss or the value; a particle pays for that once
+ * or twice in its life.  Range tests compare the high words of the doubles on
+ * the integer pipe.
+ *
+ * Why: the general maps spend about 180 FP64-pipe operations per bend drift
+ * substep and kick, half of them in five separate divisions and a square root,
+ * each with its own range branch; these take about 85.
+ */
+#ifndef B2E_FAST_CUH
+#define B2E_FAST_CUH
+#include "b2e_elements.cuh"
+#include "b2e_fp64.cuh"
+
+/* high words of the limits */
+#define FP_HI_2M250 0x30500000u
+#define FP_HI_2M10 0x3f500000u
+#define FP_HI_2M4 0x3fb00000u
+#define FP_HI_2M3 0x3fc00000u
+#define FP_HI_2 0x40000000u
+#define FP_HI_2P4 0x40300000u
+#define FP_HI_2P10 0x40900000u
+#define FP_HI_2P100 0x46300000u
+
+/* v zero, or 2^-250 <= |v| below the value whose high word is `end`: products
+ * and remainders of such values stay clear of the subnormal range */
+__device__ __forceinline__ bool fp_plain(double v, unsigned end) {
+  const unsigned h = fp_abs_hi(v);
+  return h - FP_HI_2M250 < end - FP_HI_2M250 || (h | (unsigned)__double2loint(v)) == 0;
+}
+
+/* v in [value of lo, value of hi) by high words; negative and non-finite v are out */
+__device__ __forceinline__ bool fp_within(double v, unsigned lo, unsigned hi) { return fp_hi(v) - lo < hi - lo; }
+
+/* surely inside the aperture: (x/x_max)^2 + (y/y_max)^2 below 0.998 or so, a
+ * half-axis that is not checked counting as infinite.  Rectangles contain that
+ * ellipse, and so do the super-ellipses of exponents above 2.  False for
+ * non-finite x or y. */
+__device__ __forceinline__ bool ap_surely_inside(double x, double y, const DevAperture *ap) {
+  const double u = x * ap->inv_x, v = y * ap->inv_y;
+  return fp_abs_hi(fma(u, u, v * v)) < 0x3feff000u;
+}
+
+__device__ __forceinline__ bool ap_surely_inside(double x, double y, const DevAperture *ap, const DevElem &e) {
+  if (e.flags & EF_REVERSE_TILT) {
+    const double x0 = x, y0 = y;
+    x = x0 * e.rev_cos + y0 * e.rev_sin;
+    y = -x0 * e.rev_sin + y0 * e.rev_cos;
+  }
+  return ap_surely_inside(x, y, ap);
+}
+
+/* the exact test, out of line: only particles near or beyond the edge take it */
+static __device__ __noinline__ bool ap_inside_exact(double x, double y, const DevAperture *ap, const DevElem *e) {
+  return mult_aperture_ok(x, y, ap, *e);
+}
+
+__device__ __forceinline__ bool ap_inside(double x, double y, const DevAperture *ap, const DevElem &e) {
+  return ap_surely_inside(x, y, ap, e) || ap_inside_exact(x, y, ap, &e);
+}
+
+/* offset_misalign with the square root only where dz uses it: zero times a
+ * positive finite root is a zero of dz's sign */
+__device__ __forceinline__ void offset_misalign_fast(Part &p, double dx, double dy, double dz) {
+  const double r = dz == 0 ? 1.0 : fp_sqrt((1 + p.xp * p.xp) + p.yp * p.yp);
+  p.s = p.s + dz * r;
+  p.x = (p.x - dx) + dz * p.xp;
+  p.y = (p.y - dy) + dz * p.yp;
+}
+
+/* entrance and exit limits of kmult (coordinates, slopes), and slopes below 2 */
+__device__ __forceinline__ bool inside_limits(const Part &p, const DevGlobals &g) {
+  const unsigned cl = min(fp_hi(g.coord_limit), FP_HI_2P100), sl = min(fp_hi(g.slope_limit), FP_HI_2);
+  return fp_abs_hi(p.x) < cl && fp_abs_hi(p.y) < cl && fp_abs_hi(p.xp) < sl && fp_abs_hi(p.yp) < sl;
+}
+
+__device__ __forceinline__ bool plain_transverse(const Part &p) {
+  return fp_plain(p.x, FP_HI_2P100) && fp_plain(p.y, FP_HI_2P100) && fp_plain(p.xp, FP_HI_2) && fp_plain(p.yp, FP_HI_2);
+}
+
+/* ---- KQUAD / KSEXT without K1/J1, steering, fringes or radiation (EF_FAST).
+ * The radiation block's round trip always runs (EF_RADBLOCK).
+ * Per kick: the round trip of the momenta through 1 + delta, one square root
+ * whose reciprocal divides both momenta; per drift one square root. */
+__device__ __forceinline__ bool kmult_fast(Part &pio, const DevElem &e, const DevAperture *ap, const DevGlobals &g) {
+  const double *c = e.c;
+  const int order = (int)c[KM_ORDER], nSlices = (int)c[KM_NSLICES], nSub = (int)c[KM_NSUB];
+  const double dx = c[KM_DX], dy = c[KM_DY];
+  Part p = pio;
+  if (e.flags & EF_ENTRANCE_OFFSET)
+    offset_misalign_fast(p, dx, dy, c[KM_DZ]);
+  if (e.flags & EF_ENTRANCE_ROTATE)
+    rotate_misalign(p, c[KM_COS_TILT], c[KM_SIN_TILT]);
+  const double A = 1 + p.dp, A2 = A * A, inv_A = fp_polish(A, fp_recip(A));
+  bool ok = inside_limits(p, g) && plain_transverse(p) && fp_within(A, FP_HI_2M4, FP_HI_2P4) && !fp_edge(A);
+  double x = p.x, xp = p.xp, y = p.y, yp = p.yp, s = 0, r, ir, d, qx, qy;
+  r = fp_sqrt_recip((1 + xp * xp) + yp * yp, ir);
+  ok = ok && !fp_edge(r);
+  qx = fp_quot(A * xp, r, ir);
+  qy = fp_quot(A * yp, r, ir);
+  d = (A2 - qx * qx) - qy * qy;
+  r = fp_sqrt_recip(d, ir);
+  ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10) && !fp_edge(r);
+  xp = fp_quot(qx, r, ir);
+  yp = fp_quot(qy, r, ir);
+  for (int i = 0; i < nSlices && ok; i++) {
+    if (ap)
+      ok = ap_inside(x + dx, y + dy, ap, e);
+#pragma unroll 1
+    for (int step = 0;; step++) {
+      const double dsh = c[KM_DSH0 + step];
+      x = x + xp * dsh;
+      y = y + yp * dsh;
+      s = s + dsh * fp_sqrt((1 + xp * xp) + yp * yp);
+      if (step == nSub - 1)
+        break;
+      const double kick = c[KM_KICK0 + step];
+      double fx, fy;
+      if (order == 1) {
+        fx = y;
+        fy = x;
+      } else {
+        fx = x * y;
+        fy = 0.5 * (x * x);
+        fy = fy + -0.5 * (y * y);
+      }
+      qx = qx - kick * fy;
+      qy = qy + kick * fx;
+      qx = fp_quot(qx, A, inv_A) * A;
+      qy = fp_quot(qy, A, inv_A) * A;
+      /* the test of the momenta before the round trip differs from this one
+       * by rounding only, so it cannot fail where d is 2^-10 or more */
+      d = (A2 - qx * qx) - qy * qy;
+      r = fp_sqrt_recip(d, ir);
+      ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10) && !fp_edge(r);
+      xp = fp_quot(qx, r, ir);
+      yp = fp_quot(qy, r, ir);
+    }
+  }
+  if (!ok || (ap && !ap_inside(x + dx, y + dy, ap, e)))
+    return false;
+  /* the slopes are those of the last kick: the momenta have not changed since */
+  p.x = x;
+  p.xp = xp;
+  p.y = y;
+  p.yp = yp;
+  p.s = p.s + s;
+  if (!inside_limits(p, g))
+    return false;
+  if (e.flags & EF_EXIT_MISALIGN) {
+    if (e.flags & EF_ENTRANCE_ROTATE)
+      rotate_misalign(p, c[KM_COS_TILT], -c[KM_SIN_TILT]);
+    if (e.flags & EF_ENTRANCE_OFFSET)
+      offset_misalign_fast(p, -dx, -dy, -c[KM_DZ]);
+  }
+  pio = p;
+  return true;
+}
+
+/* sqrt((1 + delta)^2 - QY^2) of the bend drift and its reciprocal */
+__device__ __forceinline__ bool bend_root(double A, double QY, double &f, double &inv_f) {
+  const double d = A * A - QY * QY;
+  f = fp_sqrt_recip(d, inv_f);
+  return fp_within(d, FP_HI_2M10, FP_HI_2P10) && !fp_edge(f);
+}
+
+/* The series of b2e_asin (to n = 4 for |x| <= 2^-6, else to n = 10), b2e_sin and
+ * b2e_cos (short for |x| <= 2^-4, else long), where the long ones enter the
+ * short ones' Horner chains: the same operations, with the branch around the
+ * high-order terms only.  The coefficients are operands from constant memory;
+ * as literals each costs two moves in front of its fma. */
+static __constant__ double kAsinSeries[10] = {
+  (2.0 / 3.0) * 0x1p-2,       (6.0 / 5.0) * 0x1p-4,      (20.0 / 7.0) * 0x1p-6,    (70.0 / 9.0) * 0x1p-8,
+  (252.0 / 11.0) * 0x1p-10,   (924.0 / 13.0) * 0x1p-12,  (3432.0 / 15.0) * 0x1p-14, (12870.0 / 17.0) * 0x1p-16,
+  (48620.0 / 19.0) * 0x1p-18, (184756.0 / 21.0) * 0x1p-20};
+static __constant__ double kSinSeries[9] = { /* -1/3!, 1/5!, ..., -1/19! */
+  -1.0 / 6.0, 1.0 / 120.0, -1.0 / 5040.0, 1.0 / 362880.0, -1.0 / 39916800.0, 1.0 / 6227020800.0,
+  -1.0 / 1307674368000.0, 1.0 / 355687428096000.0, -1.0 / 121645100408832000.0};
+static __constant__ double kCosSeries[9] = { /* 1/4!, -1/6!, ..., 1/20! */
+  1.0 / 24.0, -1.0 / 720.0, 1.0 / 40320.0, -1.0 / 3628800.0, 1.0 / 479001600.0, -1.0 / 87178291200.0,
+  1.0 / 20922789888000.0, -1.0 / 6402373705728000.0, 1.0 / 2432902008176640000.0};
+
+__device__ __forceinline__ double asin_series(double x, bool tiny) {
+  const double w = x * x;
+  double p = kAsinSeries[3];
+  if (!tiny) {
+    double q = kAsinSeries[9];
+#pragma unroll
+    for (int k = 8; k >= 4; k--)
+      q = fma(q, w, kAsinSeries[k]);
+    p = fma(q, w, kAsinSeries[3]);
+  }
+#pragma unroll
+  for (int k = 2; k >= 0; k--)
+    p = fma(p, w, kAsinSeries[k]);
+  return fma(x * w, p, x);
+}
+
+__device__ __forceinline__ double sin_series(double r, double w, bool small) {
+  double p = kSinSeries[3];
+  if (!small) {
+    double q = kSinSeries[8];
+#pragma unroll
+    for (int k = 7; k >= 4; k--)
+      q = fma(q, w, kSinSeries[k]);
+    p = fma(q, w, kSinSeries[3]);
+  }
+#pragma unroll
+  for (int k = 2; k >= 0; k--)
+    p = fma(p, w, kSinSeries[k]);
+  return fma(r * w, p, r);
+}
+
+/* 0.5 w is exact, so the two differences with it are one fma each */
+__device__ __forceinline__ double cos_series(double w, bool small) {
+  double p = kCosSeries[2];
+  if (!small) {
+    double q = kCosSeries[8];
+#pragma unroll
+    for (int k = 7; k >= 3; k--)
+      q = fma(q, w, kCosSeries[k]);
+    p = fma(q, w, kCosSeries[2]);
+  }
+  p = fma(p, w, kCosSeries[1]);
+  p = fma(p, w, kCosSeries[0]);
+  const double t = fma(-0.5, w, 1.0);
+  return t + (fma(-0.5, w, 1.0 - t) + (w * w) * p);
+}
+
+/* |v| <= limit, on the integer pipe (NaN is above every limit) */
+__device__ __forceinline__ bool abs_at_most(double v, double limit) {
+  return (__double_as_longlong(v) & 0x7fffffffffffffffll) <= __double_as_longlong(limit);
+}
+
+/* what the drifts of a bend met: the largest |sin phi| (high word) and the
+ * largest low word of a cosine, tested once per element */
+struct BendExtremes {
+  unsigned sin_hi, cos_lo;
+};
+__device__ __forceinline__ bool bend_extremes_ok(const BendExtremes &m) {
+  return m.sin_hi < FP_HI_2M3 && m.cos_lo < 0xfffffff0u;
+}
+
+/* drift substep (bend_drift): f and inv_f as bend_root leaves them.  Angles
+ * beyond the series' range only make the extremes fail; with |sin phi| < 1/8
+ * and the slice angles EF_FAST admits, |arg| is below pi/4. */
+__device__ __forceinline__ void bend_drift_fast(double &X, double &QX, double &Y, double QY, double &dist, double A,
+                                                double f, double inv_f, double rho0, double dsh_rho0,
+                                                BendExtremes &m) {
+  const double sin_phi = fp_quot(QX, f, inv_f);
+  m.sin_hi = max(m.sin_hi, fp_abs_hi(sin_phi));
+  const double phi = asin_series(sin_phi, abs_at_most(sin_phi, 0x1p-6)), arg = dsh_rho0 + phi;
+  const double wa = arg * arg, wp = phi * phi;
+  const bool small = abs_at_most(arg, 0x1p-4);
+  const double sine = sin_series(arg, wa, small), cosi = cos_series(wa, small);
+  const double cos_phi = cos_series(wp, abs_at_most(phi, 0x1p-4));
+  const double ic = fp_recip(cosi), ip = fp_recip(cos_phi);
+  m.cos_lo = max(m.cos_lo, max((unsigned)__double2loint(cosi), (unsigned)__double2loint(cos_phi)));
+  const double tang = fp_quot(sine, cosi, ic), ratio = fp_quot(cos_phi, cosi, ic);
+  const double factor = fp_quot((rho0 + X) * cos_phi, f, inv_f) * (tang - fp_quot(sin_phi, cos_phi, ip));
+  QX = f * sine;
+  Y = Y + QY * factor;
+  dist = dist + factor * A;
+  X = rho0 * (ratio - 1) + ratio * X;
+}
+
+/* nSlices slices of the bend (csbend_integrate with neither field terms nor
+ * radiation).  QY changes only by rounding, in the round trip through 1 + delta
+ * after a kick (ROUND_TRIP), and stays put from the first trip that leaves it
+ * alone: the trip depends on nothing else.  So its trips stop there, and f and
+ * 1/f are formed again only while it moves. */
+template <bool ROUND_TRIP, int NSUB = 0>
+__device__ __forceinline__ bool bend_slices_fast(double &X, double &QX, double &Y, double &QY, double &dist, double A,
+                                                 double inv_A, const double *c, int nSlices, int nSub_rt,
+                                                 const DevAperture *ap, const DevElem &e) {
+  const double rho0 = c[CB_RHO0];
+  const int nSub = NSUB > 0 ? NSUB : nSub_rt;
+  double f, inv_f;
+  BendExtremes m = {0, 0};
+  bool ok = bend_root(A, QY, f, inv_f), moves = ROUND_TRIP;
+  dist = 0;
+  for (int i = 0; i < nSlices && ok; i++) {
+    if (ap)
+      ok = ap_inside(X, Y, ap, e);
+#pragma unroll(NSUB > 0 ? NSUB : 1)
+    for (int j = 0;; j++) {
+      bend_drift_fast(X, QX, Y, QY, dist, A, f, inv_f, rho0, c[CB_DSH0 + j], m);
+      if (j == nSub - 1)
+        break;
+      const double t = (-c[CB_DS0 + j]) * (1 + fp_quot(X, rho0, c[CB_INV_RHO0]));
+      QX = QX + fp_quot(t, c[CB_RHO_ACTUAL], c[CB_INV_RHO_ACTUAL]);
+      if (ROUND_TRIP) {
+        QX = fp_quot(QX, A, inv_A) * A;
+        if (moves) {
+          const double q = fp_quot(QY, A, inv_A) * A;
+          moves = q != QY;
+          if (moves) {
+            QY = q;
+            ok = bend_root(A, QY, f, inv_f) && ok;
+          }
+        }
+      }
+    }
+  }
+  return ok && bend_extremes_ok(m) && (!ap || ap_inside(X, Y, ap, e));
+}
+
+/* first-order edge with nonzero angles or fringe (csbend), out of line */
+struct EdgeSlopes {
+  double xp, yp;
+};
+static __device__ __noinline__ EdgeSlopes bend_edge_o1(double xp, double yp, double x, double y, double dp, double rho_actual,
+                                                       const double *tan_e) {
+  /* tan_e: CB_TAN_E, CB_E, CB_PSI of one face, in that order */
+  const double rho = (1 + dp) * rho_actual, delta_xp = (tan_e[0] / rho) * x;
+  EdgeSlopes r;
+  r.xp = xp + delta_xp;
+  r.yp = yp - (b2e_tan(tan_e[1] - tan_e[2] / (1 + dp)) / rho) * y;
+  return r;
+}
+
+/* ---- CSBEND without field terms, ETILT, second-order or simple edges and
+ * radiation (EF_FAST) */
+__device__ __forceinline__ bool csbend_fast(Part &pio, const DevElem &e, const DevAperture *ap, const DevGlobals &g) {
+  const double *c = e.c;
+  const double ct = c[CB_COS_TT], st = c[CB_SIN_TT];
+  Part p = pio;
+  double x, y, xp, yp, s, Q4, r, ir, f;
+  const double A = 1 + p.dp, inv_A = fp_polish(A, fp_recip(A));
+  bool ok = plain_transverse(p) && fp_plain(p.s, FP_HI_2P100) && fp_within(A, FP_HI_2M4, FP_HI_2P4) && !fp_edge(A);
+  s = p.s + c[CB_DZI] * (c[CB_DZI] == 0 ? 1.0 : fp_sqrt((1 + p.xp * p.xp) + p.yp * p.yp));
+  p.x = (p.x + c[CB_DXI]) + c[CB_DZI] * p.xp;
+  p.y = (p.y + c[CB_DYI]) + c[CB_DZI] * p.yp;
+  x = p.x * ct + p.y * st;
+  y = -p.x * st + p.y * ct;
+  xp = p.xp * ct + p.yp * st;
+  yp = -p.xp * st + p.yp * ct;
+  if (e.flags & EF_EDGE1) {
+    if (e.flags & EF_EDGE1_FLAT) {
+      /* no edge angle, no fringe: the zeros that the divisions by rho give */
+      const double rho = A * c[CB_RHO_ACTUAL], z = c[CB_TAN_E1] * rho;
+      xp = xp + z * x;
+      yp = yp - z * y;
+    } else {
+      const EdgeSlopes es = bend_edge_o1(xp, yp, x, y, p.dp, c[CB_RHO_ACTUAL], c + CB_TAN_E1);
+      xp = es.xp;
+      yp = es.yp;
+    }
+  }
+  r = fp_sqrt_recip((1 + xp * xp) + yp * yp, ir);
+  ok = ok && fp_plain(xp, FP_HI_2) && fp_plain(yp, FP_HI_2) && !fp_edge(r);
+  f = fp_quot(A, r, ir);
+  xp = xp * f;
+  yp = yp * f;
+  /* a kick adds a zero to QY, which a negative zero would not survive */
+  ok = ok && fp_hi(yp) != 0x80000000u;
+  if (!ok)
+    return false;
+  if (!bend_slices_fast<true>(x, xp, y, yp, Q4, A, inv_A, c, (int)c[CB_NSLICES], (int)c[CB_NSUB], ap, e))
+    return false;
+  {
+    const double d = (A * A - xp * xp) - yp * yp;
+    r = fp_sqrt_recip(d, ir);
+    ok = fp_within(d, FP_HI_2M10, FP_HI_2P10) && !fp_edge(r);
+  }
+  f = fp_quot(1.0, r, ir);
+  xp = xp * f;
+  yp = yp * f;
+  {
+    /* the velocity is the entrance's: beta s / beta rounds twice */
+    const double p0 = g.p_central * A, rb = fp_sqrt_recip(p0 * p0 + 1, ir), beta = fp_quot(p0, rb, ir);
+    ok = ok && fp_within(p0, FP_HI_2M10, FP_HI_2P100) && !fp_edge(rb) && !fp_edge(beta);
+    s = fp_quot(beta * s, beta, fp_polish(beta, fp_recip(beta))) + Q4;
+  }
+  if (e.flags & EF_EDGE2) {
+    if (e.flags & EF_EDGE2_FLAT) {
+      const double rho = A * c[CB_RHO_ACTUAL], z = c[CB_TAN_E2] * rho;
+      xp = xp + z * x;
+      yp = yp - z * y;
+    } else {
+      const EdgeSlopes es = bend_edge_o1(xp, yp, x, y, p.dp, c[CB_RHO_ACTUAL], c + CB_TAN_E2);
+      xp = es.xp;
+      yp = es.yp;
+    }
+  }
+  p.x = (x * ct - y * st) + 0.0;
+  p.y = (x * st + y * ct) + 0.0;
+  p.xp = (xp * ct - yp * st) + 0.0;
+  p.yp = (xp * st + yp * ct) + 0.0;
+  p.s = s + 0.0;
+  ok = ok && fp_abs_hi(p.xp) < FP_HI_2 && fp_abs_hi(p.yp) < FP_HI_2;
+  p.x = p.x + (c[CB_DXF] + c[CB_DZF] * p.xp);
+  p.y = p.y + (c[CB_DYF] + c[CB_DZF] * p.yp);
+  p.s = p.s + c[CB_DZF] * (c[CB_DZF] == 0 ? 1.0 : fp_sqrt((1 + p.xp * p.xp) + p.yp * p.yp));
+  if (!ok)
+    return false;
+  pio = p;
+  return true;
+}
+
+/* The general maps out of line, for elements or particles the forms above do
+ * not take.  The particle travels in a local copy, so that the caller's stays
+ * in registers on the other path. */
+template <bool RAD>
+static __device__ __noinline__ int kmult_call(Part *p, const DevElem *e, const DevAperture *ap, DevGlobals g,
+                                              const RadSite *rs) {
+  return kmult<RAD>(*p, *e, ap, g, *rs);
+}
+template <bool RAD>
+__device__ __forceinline__ int kmult_general(Part &p, const DevElem &e, const DevAperture *ap, const DevGlobals &g,
+                                             const RadSite &rs) {
+  Part t = p;
+  const RadSite site = rs;
+  const int lost = kmult_call<RAD>(&t, &e, ap, g, &site);
+  p = t;
+  return lost;
+}
+template <bool RAD>
+static __device__ __noinline__ int csbend_call(Part *p, const DevElem *e, const DevAperture *ap, DevGlobals g,
+                                               const RadSite *rs) {
+  return csbend<RAD>(*p, *e, ap, g, *rs);
+}
+template <bool RAD>
+__device__ __forceinline__ int csbend_general(Part &p, const DevElem &e, const DevAperture *ap, const DevGlobals &g,
+                                              const RadSite &rs) {
+  Part t = p;
+  const RadSite site = rs;
+  const int lost = csbend_call<RAD>(&t, &e, ap, g, &site);
+  p = t;
+  return lost;
+}
+
+#endif

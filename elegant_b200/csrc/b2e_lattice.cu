@@ -456,6 +456,49 @@ static void etilt_exit_offsets(double out[5], double rho0, double angle, double 
   out[3] = -xp * s + yp * c;
 }
 
+/* EF_FAST: the element is one of those the straight-line forms (b2e_fast.cuh)
+ * are written for, and its constants are zero or far from overflow and
+ * underflow in products with coordinates.  A CSRCSBEND's edges and exit
+ * offsets are the CSR entry and exit kernels' business. */
+static void mark_fast(DevElem &d) {
+  auto plain = [](double v) { return v == 0 || (fabs(v) >= 0x1p-60 && fabs(v) <= 0x1p60); };
+  /* a divisor by stored reciprocal: positive, its significand not among the
+   * last before 2 */
+  auto divisor = [&](double v) {
+    uint64_t bits;
+    memcpy(&bits, &v, sizeof(bits));
+    return v > 0 && plain(v) && (uint32_t)bits < 0xfffffff0u;
+  };
+  bool ok = true;
+  if (d.kind == K_KMULT) {
+    ok = (d.flags & EF_RADBLOCK) && !(d.flags & (EF_QUAD_ORDER2 | EF_SKEW_ORDER2 | EF_SR | EF_ISR | EF_STEERING | EF_QFRINGE1 | EF_QFRINGE2 |
+                      EF_END_DRIFT));
+    for (int j = 0; j < 8; j++)
+      ok = ok && plain(d.c[KM_DSH0 + j]) && plain(d.c[KM_KICK0 + j]);
+    ok = ok && plain(d.c[KM_DX]) && plain(d.c[KM_DY]) && plain(d.c[KM_DZ]);
+  } else if (d.kind == K_CSBEND || d.kind == K_CSRCSBEND) {
+    ok = !(d.flags & (EF_SR | EF_ISR | EF_FIELD | EF_SKEW_KICK | EF_EDGE1_SIMPLE | EF_EDGE2_SIMPLE));
+    if (d.kind == K_CSBEND)
+      ok = ok && (d.flags & EF_RADBLOCK) && !(d.flags & (EF_EDGE_ORDER2 | EF_ETILT));
+    /* a drift angle of 0.6 after one of asin(1/8) stays below pi/4 */
+    for (int j = 0; j < 8; j++)
+      ok = ok && plain(d.c[CB_DSH0 + j]) && fabs(d.c[CB_DSH0 + j]) < 0.6 && plain(d.c[CB_DS0 + j]);
+    ok = ok && divisor(d.c[CB_RHO0]) && divisor(d.c[CB_RHO_ACTUAL]);
+    for (int j = CB_DXI; j <= CB_DZF; j++)
+      ok = ok && plain(d.c[j]);
+    auto flat = [](const double *edge) { /* CB_TAN_E, CB_E, CB_PSI of one face */
+      return edge[0] == 0 && edge[1] == 0 && edge[2] == 0 && !std::signbit(edge[2]);
+    };
+    if (flat(d.c + CB_TAN_E1))
+      d.flags |= EF_EDGE1_FLAT;
+    if (flat(d.c + CB_TAN_E2))
+      d.flags |= EF_EDGE2_FLAT;
+  } else
+    return;
+  if (ok)
+    d.flags |= EF_FAST;
+}
+
 static std::string compile_csbend(const b2e_element &el, bool edge1, bool edge2, double Po, DevElem &d,
                                   DevRad &r) {
   const double *p = el.p;
@@ -793,6 +836,15 @@ std::string compile_lattice(const b2e_element *el, int n, const b2e_run_options 
           a.b2 = ipow_host(a.y_max, a.ye);
         }
       }
+      /* the quick test's bounds hold for exponents up to 8 and half-axes whose
+       * powers stay far from overflow and underflow */
+      auto inverse = [&](double half) {
+        if (half <= 0)
+          return 0.0;
+        return half >= 0x1p-100 && half <= 0x1p100 && a.xe <= 8 && a.ye <= 8 ? 1 / half : INFINITY;
+      };
+      a.inv_x = inverse(a.x_max);
+      a.inv_y = inverse(a.y_max);
       last_ap = (int)out.aps.size();
       out.aps.push_back(a);
       d.kind = K_MAXAMP;
@@ -866,6 +918,7 @@ std::string compile_lattice(const b2e_element *el, int n, const b2e_run_options 
     if (!err.empty())
       return std::string("element ") + std::to_string(i) + " (" + std::string(el[i].name, strnlen(el[i].name, 32)) +
              "): " + err;
+    mark_fast(d);
     d.ap_pass0 = last_ap;
     d.z_end = z;
   }

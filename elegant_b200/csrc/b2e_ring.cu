@@ -21,7 +21,7 @@
  * IDs are).
  */
 #include <cuda_runtime.h>
-#include "b2e_elements.cuh"
+#include "b2e_fast.cuh"
 #include "b2e_kernels.h"
 
 namespace b2e {
@@ -177,7 +177,8 @@ __global__ void __launch_bounds__(128 * TPB, MINB) ring_kernel(RingLaunch L) {
           rs.elem = ie;
           rs.rc = rads[ie].c;
         }
-        lost = kmult<RAD>(p, e, ap, L.g, rs);
+        if (!((e.flags & EF_FAST) && kmult_fast(p, e, ap, L.g)))
+          lost = kmult_general<RAD>(p, e, ap, L.g, rs);
         break;
       case K_CSBEND:
         if (RAD) {
@@ -185,7 +186,8 @@ __global__ void __launch_bounds__(128 * TPB, MINB) ring_kernel(RingLaunch L) {
           rs.elem = ie;
           rs.rc = rads[ie].c;
         }
-        lost = csbend<RAD>(p, e, ap, L.g, rs);
+        if (!((e.flags & EF_FAST) && csbend_fast(p, e, ap, L.g)))
+          lost = csbend_general<RAD>(p, e, ap, L.g, rs);
         break;
       case K_MALIGN: {
         const double *mc = e.c;
@@ -214,10 +216,12 @@ __global__ void __launch_bounds__(128 * TPB, MINB) ring_kernel(RingLaunch L) {
       default: /* MARK, CHARGE, WATCH (recorded between launches) */
         break;
       }
-      if (!lost && !(e.flags & EF_NO_APERTURE) && ap && !maxamp_ok(p, *ap))
-        lost = LOSS_APERTURE;
-      if (!lost && !finite_xy(p))
-        lost = LOSS_NAN;
+      if (!lost && !(ap && ap_surely_inside(p.x, p.y, ap))) {
+        if (!(e.flags & EF_NO_APERTURE) && ap && !maxamp_ok(p, *ap))
+          lost = LOSS_APERTURE;
+        else if (!finite_xy(p))
+          lost = LOSS_NAN;
+      }
       if (lost) {
         lost_pass = pass;
         lost_elem = ie;
@@ -690,5 +694,89 @@ extern "C" int b2e_selftest_division(const double *host_b, int32_t n_b, int64_t 
   if (e != cudaSuccess)
     return B2E_ERR_CUDA;
   *mismatches = (int64_t)hm;
+  return B2E_OK;
+}
+
+/* ---- rounding self-test (b2e_selftest_rounding) ------------------------- */
+namespace b2e {
+
+__device__ __forceinline__ uint64_t rounding_hash(uint64_t z) {
+  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull; /* SplitMix64 */
+  z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+  return z ^ (z >> 31);
+}
+
+/* an operand of one of four kinds: any significand over 60 binades, up to 2^40
+ * ulp either side of 1, the same around a power of two, and a short
+ * significand (exact quotients and squares) */
+__device__ __forceinline__ double rounding_operand(uint64_t z, int kind) {
+  const double m = __longlong_as_double((long long)(0x3ff0000000000000ull | (z >> 12)));
+  const int ex = (int)(z % 61) - 30;
+  const long long k = (long long)((z >> 20) >> (z % 41)); /* log-uniform below 2^44 */
+  switch (kind) {
+  case 0:
+    return ldexp(m, ex);
+  case 1:
+    return __longlong_as_double(0x3ff0000000000000ll + ((z & 64) ? k >> 4 : -(k >> 4)));
+  case 2:
+    return ldexp(__longlong_as_double(0x3ff0000000000000ll + ((z & 64) ? k >> 4 : -(k >> 4))), ex);
+  default:
+    return ldexp((double)(1 + (z >> 44)), ex - 20);
+  }
+}
+
+/* counts[0]: quotients through fp_recip, [1]: square roots, [2]: quotients
+ * through a root's reciprocal, [3]: fp_polish(fp_recip) against 1/b.  Every
+ * second numerator is placed next to the midpoint of two quotients, every
+ * second radicand next to the square of a midpoint. */
+__global__ void rounding_selftest_kernel(int64_t samples, uint64_t seed, unsigned long long *counts) {
+  unsigned long long bad[4] = {0, 0, 0, 0};
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < samples; k += (int64_t)gridDim.x * blockDim.x) {
+    const uint64_t z0 = rounding_hash(seed + 0x9E3779B97F4A7C15ull * (uint64_t)(2 * k + 1));
+    const uint64_t z1 = rounding_hash(seed + 0x9E3779B97F4A7C15ull * (uint64_t)(2 * k + 2));
+    const int kb = (int)(k & 3), ka = (int)((k >> 2) & 3);
+    const double b = rounding_operand(z0, kb), a0 = rounding_operand(z1, ka);
+    /* b times the midpoint above a0: the quotient lies next to that midpoint */
+    const double half_ulp = __longlong_as_double(((__double_as_longlong(a0) >> 52) - 53) << 52);
+    const double a = (k & 16) ? fma(a0, b, half_ulp * b) : (k & 32 ? -a0 : a0);
+    if (!fp_edge(b)) {
+      const double y = fp_recip(b), q = fp_quot(a, b, y);
+      bad[0] += __double_as_longlong(q) != __double_as_longlong(a / b);
+      bad[3] += __double_as_longlong(fp_polish(b, y)) != __double_as_longlong(1.0 / b);
+    }
+    const double d = (k & 16) ? fma(b, b, 2 * b * __longlong_as_double(((__double_as_longlong(b) >> 52) - 53) << 52)) : b;
+    double y;
+    const double s = fp_sqrt_recip(d, y);
+    bad[1] += __double_as_longlong(s) != __double_as_longlong(sqrt(d));
+    if (!fp_edge(s))
+      bad[2] += __double_as_longlong(fp_quot(a, s, y)) != __double_as_longlong(a / sqrt(d));
+  }
+  for (int c = 0; c < 4; c++) {
+    for (int off = 16; off > 0; off >>= 1)
+      bad[c] += __shfl_down_sync(0xffffffffu, bad[c], off);
+    if ((threadIdx.x & 31) == 0 && bad[c])
+      atomicAdd(counts + c, bad[c]);
+  }
+}
+
+} // namespace b2e
+
+extern "C" int b2e_selftest_rounding(int64_t samples, uint64_t seed, int64_t mismatches[4]) {
+  using namespace b2e;
+  if (samples < 1 || !mismatches)
+    return B2E_ERR_ARG;
+  unsigned long long *dm = nullptr, hm[4] = {0, 0, 0, 0};
+  if (cudaMalloc(&dm, sizeof(hm)) != cudaSuccess)
+    return B2E_ERR_NOMEM;
+  cudaMemset(dm, 0, sizeof(hm));
+  rounding_selftest_kernel<<<148 * 8, 256>>>(samples, seed, dm);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaMemcpy(hm, dm, sizeof(hm), cudaMemcpyDeviceToHost);
+  cudaFree(dm);
+  if (e != cudaSuccess)
+    return B2E_ERR_CUDA;
+  for (int c = 0; c < 4; c++)
+    mismatches[c] = (int64_t)hm[c];
   return B2E_OK;
 }

@@ -558,6 +558,15 @@ int b2e_umma_selftest(int mode, const void *dev_a, const void *dev_b, float *dev
  * the reference. */
 int b2e_selftest_division(const double *host_b, int32_t n_b, int64_t samples, uint64_t seed, int64_t *mismatches);
 
+/* ---- rounding self-test --------------------------------------------------
+ * Compares, on the device, the tracking maps' reciprocal, quotient and square
+ * root with the IEEE operators on `samples` operands drawn from `seed`: random
+ * significands, ones around 1 and around powers of two, short ones, and
+ * numerators and radicands placed next to rounding boundaries.  mismatches[0]:
+ * quotients by a reciprocal, [1] square roots, [2] quotients by a square root
+ * through its reciprocal, [3] reciprocals.  No counterpart in the reference. */
+int b2e_selftest_rounding(int64_t samples, uint64_t seed, int64_t mismatches[4]);
+
 /* ---- allocation-free CSR dipole ---------------------------------------
  * No counterpart in the reference: an addition for callers that cannot
  * allocate device memory when they track (a program whose memory pool owns
