@@ -73,6 +73,7 @@ struct b2e_ctx {
   DevBuf<DevElem> d_elems;
   DevBuf<DevAperture> d_aps;
   DevBuf<DevRfState> d_rf;
+  DevBuf<unsigned char> d_fiducial; /* accumulators of the fiducial sum, one per instance */
   DevBuf<DevTile> d_tiles;
   DevBuf<int64_t> d_inst_offsets;
   std::vector<DevTile> tiles;
@@ -176,6 +177,7 @@ extern "C" int b2e_destroy(b2e_ctx *ctx) {
   ctx->d_naff_bad.release();
   ctx->d_aps.release();
   ctx->d_rf.release();
+  ctx->d_fiducial.release();
   ctx->d_tiles.release();
   ctx->d_inst_offsets.release();
   for (auto &c : ctx->d_cols)
@@ -772,9 +774,10 @@ static int track_impl(b2e_ctx *ctx, double *effort) {
       ctx->launches++;
     } else if (stop_kind == 1) {
       ctx->launches++;
-      CUDA_TRY(ctx, launch_fiducial(particle_view(ctx), ctx->d_inst_offsets.ptr, ctx->n_inst, ctx->d_elems.ptr, ne,
-                                    stop_e, ctx->d_rf.ptr, ctx->lat.n_rf, ctx->opt.p_central,
-                                    ctx->opt.fiducial_particles, ctx->d_flag.ptr, ctx->stream));
+      CUDA_TRY(ctx, ctx->d_fiducial.ensure(fiducial_scratch_bytes(ctx->n_inst)));
+      CUDA_TRY(ctx, launch_fiducial(particle_view(ctx), ctx->d_inst_offsets.ptr, ctx->n_inst, ctx->n,
+                                    ctx->d_elems.ptr, ne, stop_e, ctx->d_rf.ptr, ctx->lat.n_rf, ctx->opt.p_central,
+                                    ctx->opt.fiducial_particles, ctx->d_fiducial.ptr, ctx->d_flag.ptr, ctx->stream));
       next_rf++;
       /* the RFCA itself is tracked by the next ring launch */
       int rc = run_ring_range(ctx, p, stop_e, p, stop_e + 1);

@@ -47,9 +47,11 @@ cudaError_t launch_ring(const RingLaunch &L, int n_tiles, bool staged, size_t sm
  * alive_out[inst] = survivors */
 cudaError_t launch_compact(DevParticles src, const int64_t *ids_src, DevParticles dst, int64_t *ids_dst,
                            const int64_t *offs, int n_inst, int *alive_out, cudaStream_t stream);
-cudaError_t launch_fiducial(DevParticles P, const int64_t *inst_offsets, int n_inst, const DevElem *elems,
+/* scratch: fiducial_scratch_bytes(n_inst) bytes of device memory */
+size_t fiducial_scratch_bytes(int n_inst);
+cudaError_t launch_fiducial(DevParticles P, const int64_t *inst_offsets, int n_inst, int64_t n, const DevElem *elems,
                             int n_elems, int elem_index, DevRfState *rf, int n_rf, double p_central,
-                            int64_t max_rows, unsigned int *error_flag, cudaStream_t stream);
+                            int64_t max_rows, void *scratch, unsigned int *error_flag, cudaStream_t stream);
 /* one WATCH record [7][n]: x..delta and ID (double) of the live rows */
 cudaError_t launch_watch_copy(DevParticles P, const int64_t *ids, int64_t n, double *out, cudaStream_t stream);
 /* turn-by-turn record 0: x, x', y, y' of every row */

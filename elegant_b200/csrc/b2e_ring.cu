@@ -316,48 +316,95 @@ cudaError_t launch_history_merge(const double *partials, int hist_passes, const 
 
 /* RFCA fiducial time (findFiducialTime, simple_rfca.c:62-257).  TMEAN:
  * Kahan-compensated mean of (s + sOffset)/(c*beta) over the particles that
- * reach the cavity on the first pass, summed in particle order.  One thread
- * per instance walks its particles sequentially so the sum is the
- * reference's serial Kahan sum, bit for bit, when no particle was lost
- * upstream on that pass (elegant's swap-to-tail would otherwise reorder the
- * survivors).  LIGHT: (zEnd - L + sOffset)/c (:97-100).  PMAXIMUM (:126-147):
- * the arrival time of the particle with the highest delta, found as the
- * reference's loop does: the first particle's delta is the starting best and
- * only a later, strictly higher one is taken, so a beam whose first particle
- * is highest has no fiducial particle (the reference stops there; here bit 2
- * of the error flag is set and the cavity stays unset). */
-__global__ void rf_fiducial_kernel(DevParticles P, const int64_t *inst_offsets, int n_inst, const DevElem *elems,
-                                   int n_elems, int elem_index, DevRfState *rf, int n_rf, double p_central,
-                                   int64_t max_rows, unsigned int *error_flag) {
-  const int inst = blockIdx.x * blockDim.x + threadIdx.x;
-  if (inst >= n_inst)
-    return;
-  const DevElem &e = elems[(size_t)inst * n_elems + elem_index];
-  const double sOffset = e.c[RF_SOFFSET];
-  const int slot = (int)e.c[RF_SLOT];
-  DevRfState &rs = rf[(size_t)inst * n_rf + slot];
+ * reach the cavity on the first pass, in particle order (the reference's
+ * serial sum, bit for bit, when no particle was lost upstream on that pass;
+ * elegant's swap-to-tail would otherwise reorder the survivors).  LIGHT:
+ * (zEnd - L + sOffset)/c (:97-100).  PMAXIMUM (:126-147): the arrival time of
+ * the particle with the highest delta, found as the reference's loop does: the
+ * first particle's delta is the starting best and only a later, strictly
+ * higher one is taken, so a beam whose first particle is highest has no
+ * fiducial particle (the reference stops there; here bit 2 of the error flag
+ * is set and the cavity stays unset).
+ *
+ * The Kahan sum in parallel.  Let all n terms be positive and of one binade,
+ * integers m_i q with q their common ulp.  Each step forms Y = b + error, sum =
+ * RN(tsum + Y) and error = tsum + Y - sum exactly (Fast2Sum: tsum has at least
+ * Y's exponent).  |error| is at most half an ulp of the sum, no more than n q,
+ * so while m_i <= 2^53 - 2n, Y too is an exact integer multiple of q below
+ * 2^53 q.  Nothing is then rounded away, sum + error is the exact sum of the
+ * terms so far, and sum is that sum rounded to nearest even: the result is
+ * RN(q sum m_i), an integer sum that any order gives.  Arrival times of a bunch
+ * behind the first metres of a line nearly always qualify; where they do not,
+ * one thread runs the reference's loop on tiles of terms formed by the block.
+ * (The loop with its own two divisions and square root per step took 530 ns
+ * per particle, 5.3 ms for 10,000.) */
+struct FidAcc {
+  unsigned long long lo, hi; /* sums of the significands' low 32 bits and of the rest */
+  unsigned long long n, done, m_max;
+  unsigned int e_max, e_min_c; /* largest exponent field; 2047 less the smallest */
+};
+
+__device__ __forceinline__ double arrival_time(const DevParticles &P, int64_t ip, double sOffset, double p_central) {
+  const double pp = p_central * (1 + P.dp[ip]);
+  const double beta = pp / sqrt(pp * pp + 1); /* beta_from_delta, do_tracking.c:95 */
+  return (P.s[ip] + sOffset) / (B2E_C_MKS * beta);
+}
+
+/* v 2^scale rounded to nearest even */
+__device__ double round_u128(unsigned __int128 v, int scale) {
+  int bits = 0;
+  for (unsigned __int128 t = v; t; t >>= 1)
+    bits++;
+  if (bits > 53) {
+    const int sh = bits - 53;
+    const unsigned __int128 rest = v & (((unsigned __int128)1 << sh) - 1), half = (unsigned __int128)1 << (sh - 1);
+    v >>= sh;
+    if (rest > half || (rest == half && (v & 1)))
+      v++;
+    scale += sh;
+  }
+  return ldexp((double)(unsigned long long)v, scale);
+}
+
+__device__ void fiducial_set(DevRfState &rs, const DevElem &e, double tsum, int64_t nsum) {
+  if (nsum > 0) {
+    const double omega = e.c[RF_OMEGA];
+    const double t0 = tsum / nsum, phase_fiducial = -omega * t0;
+    rs.phase_fiducial = phase_fiducial;
+    rs.phase = phase_fiducial + e.c[RF_PHASE_DEG_RAD];
+    rs.set = 1;
+  } else {
+    rs.set = 0;
+  }
+}
+
+/* cavities that need no sum: a group's later members, an explicit T_REFERENCE,
+ * LIGHT and PMAXIMUM */
+__device__ void fiducial_without_sum(const DevParticles &P, int64_t first, int64_t end, const DevElem &e, int mode,
+                                     DevRfState *rf, DevRfState &rs, double p_central, unsigned int *error_flag) {
   const int leader = (int)e.c[RF_LEADER];
   if (leader >= 0) {
     /* a later cavity of a PHASE_REFERENCE group: the group's phase
      * (REF_PHASE_RETURNED, simple_rfca.c:419-421) plus its own PHASE */
-    const DevRfState &ls = rf[(size_t)inst * n_rf + leader];
-    rs.phase_fiducial = ls.phase_fiducial;
-    rs.phase = ls.phase_fiducial + e.c[RF_PHASE_DEG_RAD];
-    rs.set = ls.set;
+    rs.phase_fiducial = rf[leader].phase_fiducial;
+    rs.phase = rf[leader].phase_fiducial + e.c[RF_PHASE_DEG_RAD];
+    rs.set = rf[leader].set;
     return;
   }
-  double tsum = 0, error = 0;
+  double tsum = 0;
   int64_t nsum = 0;
-  const int64_t first = inst_offsets[inst], end = inst_offsets[inst + 1];
-  const int mode = (int)e.c[RF_FID_MODE];
-  if (mode == B2E_FIDUCIAL_LIGHT) {
-    tsum = ((e.z_end - e.c[RF_L_TOTAL]) + sOffset) / B2E_C_MKS;
+  if (e.c[RF_T_REFERENCE] != -1) {
+    /* explicit T_REFERENCE replaces the fiducial search */
+    tsum = e.c[RF_T_REFERENCE];
     nsum = 1;
-  } else if (mode == B2E_FIDUCIAL_PMAXIMUM) {
+  } else if (mode == B2E_FIDUCIAL_LIGHT) {
+    tsum = ((e.z_end - e.c[RF_L_TOTAL]) + e.c[RF_SOFFSET]) / B2E_C_MKS;
+    nsum = 1;
+  } else {
     double best = 0;
     int64_t ibest = -1;
     bool seen = false;
-    for (int64_t ip = first; ip < end && (max_rows <= 0 || ip - first < max_rows); ip++) {
+    for (int64_t ip = first; ip < end; ip++) {
       if (P.lost_pass[ip] >= 0)
         continue;
       if (!seen) {
@@ -369,43 +416,107 @@ __global__ void rf_fiducial_kernel(DevParticles P, const int64_t *inst_offsets, 
       }
     }
     if (ibest >= 0) {
-      double pp = p_central * (1 + P.dp[ibest]);
-      double beta = pp / sqrt(pp * pp + 1);
-      tsum = (P.s[ibest] + sOffset) / (B2E_C_MKS * beta);
+      tsum = arrival_time(P, ibest, e.c[RF_SOFFSET], p_central);
       nsum = 1;
-    } else if (seen && e.c[RF_T_REFERENCE] == -1) {
+    } else if (seen) {
       atomicOr(error_flag, 2u);
     }
-  } else {
-    for (int64_t ip = first; ip < end && (max_rows <= 0 || ip - first < max_rows); ip++) {
-      if (P.lost_pass[ip] >= 0)
-        continue;
-      double pp = p_central * (1 + P.dp[ip]);
-      double beta = pp / sqrt(pp * pp + 1); /* beta_from_delta, do_tracking.c:95 */
-      double b = (P.s[ip] + sOffset) / (B2E_C_MKS * beta);
-      /* KahanPlus (kahan.c:28-35) */
-      double Y = b + error;
-      double sum = tsum + Y;
-      error = Y - (sum - tsum);
-      tsum = sum;
-      nsum++;
-    }
   }
-  if (e.c[RF_T_REFERENCE] != -1) {
-    /* explicit T_REFERENCE replaces the fiducial search */
-    tsum = e.c[RF_T_REFERENCE];
-    nsum = 1;
+  fiducial_set(rs, e, tsum, nsum);
+}
+
+constexpr int FID_THREADS = 256, FID_TILE = 1024;
+
+/* gx blocks per instance; the last one to finish its share forms the result.
+ * acc: one zeroed record per instance. */
+__global__ void __launch_bounds__(FID_THREADS)
+    rf_fiducial_kernel(DevParticles P, const int64_t *inst_offsets, int gx, const DevElem *elems, int n_elems,
+                       int elem_index, DevRfState *rf, int n_rf, double p_central, int64_t max_rows, FidAcc *acc_all,
+                       unsigned int *error_flag) {
+  __shared__ double tile[FID_TILE];
+  __shared__ int last;
+  const int inst = blockIdx.x / gx, part = blockIdx.x - inst * gx;
+  const DevElem &e = elems[(size_t)inst * n_elems + elem_index];
+  DevRfState *rf_inst = rf + (size_t)inst * n_rf;
+  DevRfState &rs = rf_inst[(int)e.c[RF_SLOT]];
+  const int64_t first = inst_offsets[inst];
+  int64_t end = inst_offsets[inst + 1];
+  if (max_rows > 0 && end - first > max_rows)
+    end = first + max_rows;
+  const int mode = (int)e.c[RF_FID_MODE];
+  if (e.c[RF_LEADER] >= 0 || e.c[RF_T_REFERENCE] != -1 || mode == B2E_FIDUCIAL_LIGHT ||
+      mode == B2E_FIDUCIAL_PMAXIMUM) {
+    if (part == 0 && threadIdx.x == 0)
+      fiducial_without_sum(P, first, end, e, mode, rf_inst, rs, p_central, error_flag);
+    return;
   }
-  if (nsum > 0) {
-    const double omega = e.c[RF_OMEGA];
-    double t0 = tsum / nsum;
-    double phase_fiducial = -omega * t0;
-    rs.phase_fiducial = phase_fiducial;
-    rs.phase = phase_fiducial + e.c[RF_PHASE_DEG_RAD];
-    rs.set = 1;
-  } else {
-    rs.set = 0;
+  const double sOffset = e.c[RF_SOFFSET];
+  FidAcc a = {0, 0, 0, 0, 0, 0, 0};
+  for (int64_t ip = first + part * FID_THREADS + threadIdx.x; ip < end; ip += (int64_t)gx * FID_THREADS) {
+    if (P.lost_pass[ip] >= 0)
+      continue;
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(arrival_time(P, ip, sOffset, p_central));
+    const unsigned long long m = (bits & 0xfffffffffffffull) | 0x10000000000000ull;
+    const unsigned int ex = (unsigned int)(bits >> 52); /* with the sign: beyond 2047 for a negative term */
+    a.lo += m & 0xffffffffull;
+    a.hi += m >> 32;
+    a.n++;
+    a.m_max = max(a.m_max, m);
+    a.e_max = max(a.e_max, ex);
+    a.e_min_c = max(a.e_min_c, 2047u - min(ex, 2047u));
   }
+  for (int off = 16; off > 0; off >>= 1) {
+    a.lo += __shfl_down_sync(0xffffffffu, a.lo, off);
+    a.hi += __shfl_down_sync(0xffffffffu, a.hi, off);
+    a.n += __shfl_down_sync(0xffffffffu, a.n, off);
+    a.m_max = max(a.m_max, __shfl_down_sync(0xffffffffu, a.m_max, off));
+    a.e_max = max(a.e_max, __shfl_down_sync(0xffffffffu, a.e_max, off));
+    a.e_min_c = max(a.e_min_c, __shfl_down_sync(0xffffffffu, a.e_min_c, off));
+  }
+  FidAcc *acc = acc_all + inst;
+  if ((threadIdx.x & 31) == 0 && a.n) {
+    atomicAdd(&acc->lo, a.lo);
+    atomicAdd(&acc->hi, a.hi);
+    atomicAdd(&acc->n, a.n);
+    atomicMax(&acc->m_max, a.m_max);
+    atomicMax(&acc->e_max, a.e_max);
+    atomicMax(&acc->e_min_c, a.e_min_c);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0)
+    last = atomicAdd(&acc->done, 1ull) == (unsigned long long)(gx - 1);
+  __syncthreads();
+  if (!last)
+    return;
+  __threadfence();
+  const unsigned long long lo = __ldcg(&acc->lo), hi = __ldcg(&acc->hi), n = __ldcg(&acc->n),
+                           m_max = __ldcg(&acc->m_max);
+  const unsigned int ex = __ldcg(&acc->e_max), exc = __ldcg(&acc->e_min_c);
+  if (n && n < (1ull << 31) && ex + exc == 2047u && ex > 100 && ex < 1900 && m_max <= (1ull << 53) - 2 * n) {
+    if (threadIdx.x == 0)
+      fiducial_set(rs, e, round_u128(((unsigned __int128)hi << 32) + lo, (int)ex - 1075), (int64_t)n);
+    return;
+  }
+  double tsum = 0, error = 0;
+  for (int64_t t0 = first; t0 < end; t0 += FID_TILE) {
+    const int len = (int)min((int64_t)FID_TILE, end - t0);
+    for (int k = threadIdx.x; k < len; k += FID_THREADS)
+      tile[k] = P.lost_pass[t0 + k] < 0 ? arrival_time(P, t0 + k, sOffset, p_central) : 0.0;
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int k = 0; k < len; k++) {
+        if (P.lost_pass[t0 + k] >= 0)
+          continue;
+        /* KahanPlus (kahan.c:28-35) */
+        const double Y = tile[k] + error, sum = tsum + Y;
+        error = Y - (sum - tsum);
+        tsum = sum;
+      }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0)
+    fiducial_set(rs, e, tsum, (int64_t)n);
 }
 
 /* Effort (particle-passes) and survivor count from the loss columns. */
@@ -580,12 +691,27 @@ cudaError_t launch_compact(DevParticles src, const int64_t *ids_src, DevParticle
   return cudaGetLastError();
 }
 
-cudaError_t launch_fiducial(DevParticles P, const int64_t *inst_offsets, int n_inst, const DevElem *elems,
+size_t fiducial_scratch_bytes(int n_inst) { return sizeof(FidAcc) * (size_t)n_inst; }
+
+cudaError_t launch_fiducial(DevParticles P, const int64_t *inst_offsets, int n_inst, int64_t n, const DevElem *elems,
                             int n_elems, int elem_index, DevRfState *rf, int n_rf, double p_central,
-                            int64_t max_rows, unsigned int *error_flag, cudaStream_t stream) {
-  int tpb = 64, nb = (n_inst + tpb - 1) / tpb;
-  rf_fiducial_kernel<<<nb, tpb, 0, stream>>>(P, inst_offsets, n_inst, elems, n_elems, elem_index, rf, n_rf,
-                                             p_central, max_rows, error_flag);
+                            int64_t max_rows, void *scratch, unsigned int *error_flag, cudaStream_t stream) {
+  if (n_inst <= 0)
+    return cudaSuccess;
+  /* blocks per instance: one per 1,024 rows of an average instance, at most
+   * four per SM over all instances */
+  int64_t rows = n / n_inst;
+  if (max_rows > 0 && rows > max_rows)
+    rows = max_rows;
+  int64_t gx = (rows + 1023) / 1024, cap = 148 * 4 / n_inst;
+  gx = gx > cap ? cap : gx;
+  gx = gx < 1 ? 1 : gx;
+  cudaError_t err = cudaMemsetAsync(scratch, 0, fiducial_scratch_bytes(n_inst), stream);
+  if (err != cudaSuccess)
+    return err;
+  rf_fiducial_kernel<<<(unsigned)(gx * n_inst), FID_THREADS, 0, stream>>>(P, inst_offsets, (int)gx, elems, n_elems, elem_index, rf,
+                                                                       n_rf, p_central, max_rows, (FidAcc *)scratch,
+                                                                       error_flag);
   return cudaGetLastError();
 }
 
