@@ -198,7 +198,7 @@ __device__ __forceinline__ bool csr_slice_fast(SlicePart &pio, const DevElem &e,
   double r, ir, f;
   r = fp_sqrt_recip((1 + p.XP * p.XP) + p.YP * p.YP, ir);
   bool ok = fp_abs_hi(p.X) < FP_HI_2P100 && fp_plain(p.XP, FP_HI_2) && fp_plain(p.YP, FP_HI_2) &&
-            fp_within(A, FP_HI_2M4, FP_HI_2P4) && !fp_edge(r);
+            fp_within(A, FP_HI_2M4, FP_HI_2P4);
   f = fp_quot(A, r, ir);
   p.XP = p.XP * f;
   p.YP = p.YP * f;
@@ -207,7 +207,7 @@ __device__ __forceinline__ bool csr_slice_fast(SlicePart &pio, const DevElem &e,
   ok = bend_slices_fast<false, 4>(p.X, p.XP, p.Y, p.YP, p.dist, A, 0.0, e.c, 1, 4, ap, e) && ok;
   const double d = (A * A - p.XP * p.XP) - p.YP * p.YP;
   r = fp_sqrt_recip(d, ir);
-  ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10) && !fp_edge(r);
+  ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10);
   f = fp_quot(1.0, r, ir);
   p.XP = p.XP * f;
   p.YP = p.YP * f;

@@ -8,8 +8,7 @@
  * A form returns false, and leaves the particle untouched, when anything
  * leaves the range it was written for: an aperture (or a place too near its
  * edge to tell cheaply), a coordinate, slope or angle limit, a loss, a
- * non-finite or extremely small value, a significand the reciprocals do not
- * round correctly.  The caller then runs the general map from the element's
+ * non-finite or extremely small value.  The caller then runs the general map from the element's
  * entrance, which finds the loss or the value; a particle pays for that once
  * or twice in its life.  Range tests compare the high words of the doubles on
  * the integer pipe.
@@ -102,16 +101,15 @@ __device__ __forceinline__ bool kmult_fast(Part &pio, const DevElem &e, const De
     offset_misalign_fast(p, dx, dy, c[KM_DZ]);
   if (e.flags & EF_ENTRANCE_ROTATE)
     rotate_misalign(p, c[KM_COS_TILT], c[KM_SIN_TILT]);
-  const double A = 1 + p.dp, A2 = A * A, inv_A = fp_polish(A, fp_recip(A));
-  bool ok = inside_limits(p, g) && plain_transverse(p) && fp_within(A, FP_HI_2M4, FP_HI_2P4) && !fp_edge(A);
+  const double A = 1 + p.dp, A2 = A * A, inv_A = fp_recip(A);
+  bool ok = inside_limits(p, g) && plain_transverse(p) && fp_within(A, FP_HI_2M4, FP_HI_2P4);
   double x = p.x, xp = p.xp, y = p.y, yp = p.yp, s = 0, r, ir, d, qx, qy;
   r = fp_sqrt_recip((1 + xp * xp) + yp * yp, ir);
-  ok = ok && !fp_edge(r);
   qx = fp_quot(A * xp, r, ir);
   qy = fp_quot(A * yp, r, ir);
   d = (A2 - qx * qx) - qy * qy;
   r = fp_sqrt_recip(d, ir);
-  ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10) && !fp_edge(r);
+  ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10);
   xp = fp_quot(qx, r, ir);
   yp = fp_quot(qy, r, ir);
   for (int i = 0; i < nSlices && ok; i++) {
@@ -143,7 +141,7 @@ __device__ __forceinline__ bool kmult_fast(Part &pio, const DevElem &e, const De
        * by rounding only, so it cannot fail where d is 2^-10 or more */
       d = (A2 - qx * qx) - qy * qy;
       r = fp_sqrt_recip(d, ir);
-      ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10) && !fp_edge(r);
+      ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10);
       xp = fp_quot(qx, r, ir);
       yp = fp_quot(qy, r, ir);
     }
@@ -172,7 +170,7 @@ __device__ __forceinline__ bool kmult_fast(Part &pio, const DevElem &e, const De
 __device__ __forceinline__ bool bend_root(double A, double QY, double &f, double &inv_f) {
   const double d = A * A - QY * QY;
   f = fp_sqrt_recip(d, inv_f);
-  return fp_within(d, FP_HI_2M10, FP_HI_2P10) && !fp_edge(f);
+  return fp_within(d, FP_HI_2M10, FP_HI_2P10);
 }
 
 /* The series of b2e_asin (to n = 4 for |x| <= 2^-6, else to n = 10), b2e_sin and
@@ -243,30 +241,21 @@ __device__ __forceinline__ bool abs_at_most(double v, double limit) {
   return (__double_as_longlong(v) & 0x7fffffffffffffffll) <= __double_as_longlong(limit);
 }
 
-/* what the drifts of a bend met: the largest |sin phi| (high word) and the
- * largest low word of a cosine, tested once per element */
-struct BendExtremes {
-  unsigned sin_hi, cos_lo;
-};
-__device__ __forceinline__ bool bend_extremes_ok(const BendExtremes &m) {
-  return m.sin_hi < FP_HI_2M3 && m.cos_lo < 0xfffffff0u;
-}
-
-/* drift substep (bend_drift): f and inv_f as bend_root leaves them.  Angles
- * beyond the series' range only make the extremes fail; with |sin phi| < 1/8
- * and the slice angles EF_FAST admits, |arg| is below pi/4. */
+/* drift substep (bend_drift): f and inv_f as bend_root leaves them.  sin_max
+ * collects the high word of the largest |sin phi|, for one test per element:
+ * below 1/8 the series hold, and with the slice angles EF_FAST admits |arg| is
+ * below pi/4. */
 __device__ __forceinline__ void bend_drift_fast(double &X, double &QX, double &Y, double QY, double &dist, double A,
                                                 double f, double inv_f, double rho0, double dsh_rho0,
-                                                BendExtremes &m) {
+                                                unsigned &sin_max) {
   const double sin_phi = fp_quot(QX, f, inv_f);
-  m.sin_hi = max(m.sin_hi, fp_abs_hi(sin_phi));
+  sin_max = max(sin_max, fp_abs_hi(sin_phi));
   const double phi = asin_series(sin_phi, abs_at_most(sin_phi, 0x1p-6)), arg = dsh_rho0 + phi;
   const double wa = arg * arg, wp = phi * phi;
   const bool small = abs_at_most(arg, 0x1p-4);
   const double sine = sin_series(arg, wa, small), cosi = cos_series(wa, small);
   const double cos_phi = cos_series(wp, abs_at_most(phi, 0x1p-4));
   const double ic = fp_recip(cosi), ip = fp_recip(cos_phi);
-  m.cos_lo = max(m.cos_lo, max((unsigned)__double2loint(cosi), (unsigned)__double2loint(cos_phi)));
   const double tang = fp_quot(sine, cosi, ic), ratio = fp_quot(cos_phi, cosi, ic);
   const double factor = fp_quot((rho0 + X) * cos_phi, f, inv_f) * (tang - fp_quot(sin_phi, cos_phi, ip));
   QX = f * sine;
@@ -287,7 +276,7 @@ __device__ __forceinline__ bool bend_slices_fast(double &X, double &QX, double &
   const double rho0 = c[CB_RHO0];
   const int nSub = NSUB > 0 ? NSUB : nSub_rt;
   double f, inv_f;
-  BendExtremes m = {0, 0};
+  unsigned sin_max = 0;
   bool ok = bend_root(A, QY, f, inv_f), moves = ROUND_TRIP;
   dist = 0;
   for (int i = 0; i < nSlices && ok; i++) {
@@ -295,7 +284,7 @@ __device__ __forceinline__ bool bend_slices_fast(double &X, double &QX, double &
       ok = ap_inside(X, Y, ap, e);
 #pragma unroll(NSUB > 0 ? NSUB : 1)
     for (int j = 0;; j++) {
-      bend_drift_fast(X, QX, Y, QY, dist, A, f, inv_f, rho0, c[CB_DSH0 + j], m);
+      bend_drift_fast(X, QX, Y, QY, dist, A, f, inv_f, rho0, c[CB_DSH0 + j], sin_max);
       if (j == nSub - 1)
         break;
       const double t = (-c[CB_DS0 + j]) * (1 + fp_quot(X, rho0, c[CB_INV_RHO0]));
@@ -313,7 +302,7 @@ __device__ __forceinline__ bool bend_slices_fast(double &X, double &QX, double &
       }
     }
   }
-  return ok && bend_extremes_ok(m) && (!ap || ap_inside(X, Y, ap, e));
+  return ok && sin_max < FP_HI_2M3 && (!ap || ap_inside(X, Y, ap, e));
 }
 
 /* first-order edge with nonzero angles or fringe (csbend), out of line */
@@ -337,8 +326,8 @@ __device__ __forceinline__ bool csbend_fast(Part &pio, const DevElem &e, const D
   const double ct = c[CB_COS_TT], st = c[CB_SIN_TT];
   Part p = pio;
   double x, y, xp, yp, s, Q4, r, ir, f;
-  const double A = 1 + p.dp, inv_A = fp_polish(A, fp_recip(A));
-  bool ok = plain_transverse(p) && fp_plain(p.s, FP_HI_2P100) && fp_within(A, FP_HI_2M4, FP_HI_2P4) && !fp_edge(A);
+  const double A = 1 + p.dp, inv_A = fp_recip(A);
+  bool ok = plain_transverse(p) && fp_plain(p.s, FP_HI_2P100) && fp_within(A, FP_HI_2M4, FP_HI_2P4);
   s = p.s + c[CB_DZI] * (c[CB_DZI] == 0 ? 1.0 : fp_sqrt((1 + p.xp * p.xp) + p.yp * p.yp));
   p.x = (p.x + c[CB_DXI]) + c[CB_DZI] * p.xp;
   p.y = (p.y + c[CB_DYI]) + c[CB_DZI] * p.yp;
@@ -359,7 +348,7 @@ __device__ __forceinline__ bool csbend_fast(Part &pio, const DevElem &e, const D
     }
   }
   r = fp_sqrt_recip((1 + xp * xp) + yp * yp, ir);
-  ok = ok && fp_plain(xp, FP_HI_2) && fp_plain(yp, FP_HI_2) && !fp_edge(r);
+  ok = ok && fp_plain(xp, FP_HI_2) && fp_plain(yp, FP_HI_2);
   f = fp_quot(A, r, ir);
   xp = xp * f;
   yp = yp * f;
@@ -372,7 +361,7 @@ __device__ __forceinline__ bool csbend_fast(Part &pio, const DevElem &e, const D
   {
     const double d = (A * A - xp * xp) - yp * yp;
     r = fp_sqrt_recip(d, ir);
-    ok = fp_within(d, FP_HI_2M10, FP_HI_2P10) && !fp_edge(r);
+    ok = fp_within(d, FP_HI_2M10, FP_HI_2P10);
   }
   f = fp_quot(1.0, r, ir);
   xp = xp * f;
@@ -380,8 +369,8 @@ __device__ __forceinline__ bool csbend_fast(Part &pio, const DevElem &e, const D
   {
     /* the velocity is the entrance's: beta s / beta rounds twice */
     const double p0 = g.p_central * A, rb = fp_sqrt_recip(p0 * p0 + 1, ir), beta = fp_quot(p0, rb, ir);
-    ok = ok && fp_within(p0, FP_HI_2M10, FP_HI_2P100) && !fp_edge(rb) && !fp_edge(beta);
-    s = fp_quot(beta * s, beta, fp_polish(beta, fp_recip(beta))) + Q4;
+    ok = ok && fp_within(p0, FP_HI_2M10, FP_HI_2P100);
+    s = fp_quot(beta * s, beta, fp_recip(beta)) + Q4;
   }
   if (e.flags & EF_EDGE2) {
     if (e.flags & EF_EDGE2_FLAT) {

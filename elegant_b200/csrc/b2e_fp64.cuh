@@ -20,16 +20,17 @@
  * (P. Markstein, IBM J. Res. Dev. 34, 1990).  Quotient: q = RN(a y), remainder
  * a - q b exact under fma, RN(q + r y), with y = RN(1/b) (the same paper).
  *
- * Why the roundings are right.  Quotient: a result can round wrongly only
- * where a/b lies within |r| |y - 1/b| of a midpoint; there q is one of the two
- * neighbours, so that term is at most half an ulp times the relative error of
- * y, which for y = RN(1/b) stays below the smallest distance a quotient can
- * have from a midpoint, except for the last few significands before 2
- * (fp_edge; the callers leave those to the IEEE operators).  Square root: with g
- * next to the midpoint the remainder is an integer multiple of ulp(g)^2, and
- * a relative error of the factor 1/(2g) below 1.5 2^-53 (here at most 1.32)
- * cannot move it across the rounding boundary.  b2e_selftest_rounding compares
- * all of them with the IEEE operators on the device.
+ * Why the roundings are right.  Quotient: with y = RN(1/b) the last step
+ * returns RN(a/b) for every a (the same paper); a result can round wrongly only
+ * where a/b lies within |r| |y - 1/b| of a midpoint, q is then one of the two
+ * neighbours, and half an ulp times the relative error of y is below the
+ * smallest distance a quotient can have from a midpoint.  The iterations give
+ * RN(1/b) but for the significand just below 2 (1/b a hair above a midpoint),
+ * which fp_fix sets.  Square root: with g next to the midpoint the remainder is
+ * an integer multiple of ulp(g)^2, and a relative error of the factor 1/(2g)
+ * below 1.5 2^-53 (here at most 1.32) cannot move it across the rounding
+ * boundary.  b2e_selftest_rounding compares all of them with the IEEE
+ * operators on the device.
  */
 #ifndef B2E_FP64_CUH
 #define B2E_FP64_CUH
@@ -45,8 +46,12 @@ __device__ __forceinline__ double fp_twice(double v) {
   return __hiloint2double(__double2hiint(v) + 0x00100000, __double2loint(v));
 }
 
-/* significand within 16 ulp of 2, or any whose low word looks like it */
-__device__ __forceinline__ bool fp_edge(double b) { return (unsigned)__double2loint(b) >= 0xfffffff0u; }
+/* RN(1/b) from y, which is that or, for a significand of all ones, may be the
+ * power of two below it: 1/(2^e (1 - 2^-53)) rounds to 2^-e (1 + 2^-52) */
+__device__ __forceinline__ double fp_fix(double b, double y) {
+  const unsigned ones = (fp_hi(b) | 0xfff00000u) & (unsigned)__double2loint(b);
+  return __hiloint2double(__double2hiint(y), ones == 0xffffffffu ? 1 : __double2loint(y));
+}
 
 __device__ __forceinline__ double fp_rcp_seed(double b) {
   double y;
@@ -60,12 +65,12 @@ __device__ __forceinline__ double fp_rsqrt_seed(double d) {
 }
 
 /* RN(1/b) from y within two ulp of it */
-__device__ __forceinline__ double fp_polish(double b, double y) { return fma(fma(-b, y, 1.0), y, y); }
+__device__ __forceinline__ double fp_polish(double b, double y) { return fp_fix(b, fma(fma(-b, y, 1.0), y, y)); }
 
-/* 1/b: four operations behind the seed */
+/* RN(1/b): four operations behind the seed */
 __device__ __forceinline__ double fp_recip(double b) {
   const double y0 = fp_rcp_seed(b), e = fma(-b, y0, 1.0), p = fma(e, e, e);
-  return fma(y0, fma(p, e, e), y0);
+  return fp_fix(b, fma(y0, fma(p, e, e), y0));
 }
 
 /* RN(a/b) from y = 1/b, b > 0.  The remainder is formed with its sign turned

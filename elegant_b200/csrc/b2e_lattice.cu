@@ -462,13 +462,6 @@ static void etilt_exit_offsets(double out[5], double rho0, double angle, double 
  * offsets are the CSR entry and exit kernels' business. */
 static void mark_fast(DevElem &d) {
   auto plain = [](double v) { return v == 0 || (fabs(v) >= 0x1p-60 && fabs(v) <= 0x1p60); };
-  /* a divisor by stored reciprocal: positive, its significand not among the
-   * last before 2 */
-  auto divisor = [&](double v) {
-    uint64_t bits;
-    memcpy(&bits, &v, sizeof(bits));
-    return v > 0 && plain(v) && (uint32_t)bits < 0xfffffff0u;
-  };
   bool ok = true;
   if (d.kind == K_KMULT) {
     ok = (d.flags & EF_RADBLOCK) && !(d.flags & (EF_QUAD_ORDER2 | EF_SKEW_ORDER2 | EF_SR | EF_ISR | EF_STEERING | EF_QFRINGE1 | EF_QFRINGE2 |
@@ -483,7 +476,8 @@ static void mark_fast(DevElem &d) {
     /* a drift angle of 0.6 after one of asin(1/8) stays below pi/4 */
     for (int j = 0; j < 8; j++)
       ok = ok && plain(d.c[CB_DSH0 + j]) && fabs(d.c[CB_DSH0 + j]) < 0.6 && plain(d.c[CB_DS0 + j]);
-    ok = ok && divisor(d.c[CB_RHO0]) && divisor(d.c[CB_RHO_ACTUAL]);
+    ok = ok && d.c[CB_RHO0] > 0 && plain(d.c[CB_RHO0]) && d.c[CB_RHO_ACTUAL] > 0 &&
+         plain(d.c[CB_RHO_ACTUAL]);
     for (int j = CB_DXI; j <= CB_DZF; j++)
       ok = ok && plain(d.c[j]);
     auto flat = [](const double *edge) { /* CB_TAN_E, CB_E, CB_PSI of one face */
@@ -750,6 +744,7 @@ const char *compile_single_csr_bend(const b2e_element &el, DevElem &d, BendExtra
   memcpy(bx.c, rad.c + RB_EXTRA0, sizeof(bx.c));
   if (d.kind != K_CSRCSBEND)
     return "CSRCSBEND with zero angle is a drift; nothing to do here";
+  mark_fast(d);
   d.z_end = el.p[B2E_BEND_L];
   return nullptr;
 }

@@ -865,17 +865,14 @@ __global__ void rounding_selftest_kernel(int64_t samples, uint64_t seed, unsigne
     /* b times the midpoint above a0: the quotient lies next to that midpoint */
     const double half_ulp = __longlong_as_double(((__double_as_longlong(a0) >> 52) - 53) << 52);
     const double a = (k & 16) ? fma(a0, b, half_ulp * b) : (k & 32 ? -a0 : a0);
-    if (!fp_edge(b)) {
-      const double y = fp_recip(b), q = fp_quot(a, b, y);
-      bad[0] += __double_as_longlong(q) != __double_as_longlong(a / b);
-      bad[3] += __double_as_longlong(fp_polish(b, y)) != __double_as_longlong(1.0 / b);
-    }
+    const double yb = fp_recip(b);
+    bad[0] += __double_as_longlong(fp_quot(a, b, yb)) != __double_as_longlong(a / b);
+    bad[3] += __double_as_longlong(fp_polish(b, yb)) != __double_as_longlong(1.0 / b);
     const double d = (k & 16) ? fma(b, b, 2 * b * __longlong_as_double(((__double_as_longlong(b) >> 52) - 53) << 52)) : b;
     double y;
     const double s = fp_sqrt_recip(d, y);
     bad[1] += __double_as_longlong(s) != __double_as_longlong(sqrt(d));
-    if (!fp_edge(s))
-      bad[2] += __double_as_longlong(fp_quot(a, s, y)) != __double_as_longlong(a / sqrt(d));
+    bad[2] += __double_as_longlong(fp_quot(a, s, y)) != __double_as_longlong(a / sqrt(d));
   }
   for (int c = 0; c < 4; c++) {
     for (int off = 16; off > 0; off >>= 1)
