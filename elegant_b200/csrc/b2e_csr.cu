@@ -172,92 +172,206 @@ __global__ void csr_entry_kernel(DevParticles P, int64_t n, double *beta0, const
   beta0[i] = b0;
 }
 
-/* a slice of the bend from slopes to slopes: the general form, out of line (for
- * other integration orders and particles near a limit), and the straight-line
- * one, which leaves the particle alone where it does not apply */
+/* one particle's kick: coordinates, c*t and the entrance velocity */
 struct SlicePart {
-  double X, XP, Y, YP, DP, dist;
+  double X, XP, Y, YP, CT, DP, beta0;
 };
-static __device__ __noinline__ int csr_slice_general(SlicePart *p, const DevElem *ep, const DevAperture *ap) {
+
+/* a bunch's wake as the kick reads it */
+struct SliceWake {
+  const double *dGamma;
+  double lower, dct;
+  int nBins, apply;
+};
+
+/* Optional wake kick of the previous kick, one integrator slice, c*t update
+ * (csbend.c:2385-2450), in the general form; out of line, for other integration
+ * orders and particles near a limit. */
+static __device__ __noinline__ int csr_slice_general(SlicePart *p, const DevElem *ep, const CsrDevState *st, int nBins,
+                                                     int apply, double Po) {
   const DevElem &e = *ep;
   const double *c = e.c;
-  double f = (1 + p->DP) / sqrt((1 + p->XP * p->XP) + p->YP * p->YP);
-  double Q1 = p->XP * f, Q3 = p->YP * f;
+  double f, Q1, Q3, Q4;
+  if (apply)
+    p->DP = csr_kick(p->CT, p->X, p->DP, st, nBins, Po, c[CB_RHO0]);
+  f = (1 + p->DP) / sqrt((1 + p->XP * p->XP) + p->YP * p->YP);
+  Q1 = p->XP * f;
+  Q3 = p->YP * f;
   const RadSite no_rad = {0, 0, 0, 0, 0, nullptr};
-  const int lost = csbend_integrate<false>(p->X, Q1, p->Y, Q3, p->dist, p->DP, c, 1, (int)c[CB_NSUB], false, ap, e,
-                                           no_rad);
+  const int lost =
+    csbend_integrate<false>(p->X, Q1, p->Y, Q3, Q4, p->DP, c, 1, (int)c[CB_NSUB], false, nullptr, e, no_rad);
   f = 1 / sqrt(((1 + p->DP) * (1 + p->DP) - Q1 * Q1) - Q3 * Q3);
   p->XP = Q1 * f;
   p->YP = Q3 * f;
+  if (!lost)
+    p->CT = p->CT + Q4 / p->beta0;
   return lost;
 }
 
-__device__ __forceinline__ bool csr_slice_fast(SlicePart &pio, const DevElem &e, const DevAperture *ap) {
+static __device__ __noinline__ double divide_ieee(double a, double b) { return a / b; }
+
+/* The same in the straight-line form of b2e_fast.cuh (four substeps); leaves
+ * the particle alone and returns false where that does not apply. */
+__device__ __forceinline__ bool csr_slice_fast(SlicePart &pio, const DevElem &e, const SliceWake &w, double inv_dct,
+                                               double Po, double inv_Po) {
   SlicePart p = pio;
+  const double *c = e.c;
+  double r, ir, f, dist;
+  if (w.apply) {
+    f = fp_quot(p.CT - w.lower, w.dct, inv_dct);
+    const long long iBin = (long long)f;
+    f -= iBin;
+    if (iBin >= 0 && iBin < w.nBins - 1) {
+      const double g = (1 - f) * w.dGamma[iBin] + f * w.dGamma[iBin + 1];
+      const double h = fp_plain(g, FP_HI_2P100) ? fp_quot(g, Po, inv_Po) : divide_ieee(g, Po);
+      p.DP += h * (1 + fp_quot(p.X, c[CB_RHO0], c[CB_INV_RHO0]));
+    }
+  }
   const double A = 1 + p.DP;
-  double r, ir, f;
   r = fp_sqrt_recip((1 + p.XP * p.XP) + p.YP * p.YP, ir);
   bool ok = fp_abs_hi(p.X) < FP_HI_2P100 && fp_plain(p.XP, FP_HI_2) && fp_plain(p.YP, FP_HI_2) &&
-            fp_within(A, FP_HI_2M4, FP_HI_2P4);
+            fp_within(A, FP_HI_2M4, FP_HI_2P4) && fp_within(p.beta0, FP_HI_2M10, FP_HI_2);
   f = fp_quot(A, r, ir);
   p.XP = p.XP * f;
   p.YP = p.YP * f;
   /* a kick adds a zero to QY, which a negative zero would not survive */
   ok = ok && fp_hi(p.YP) != 0x80000000u;
-  ok = bend_slices_fast<false, 4>(p.X, p.XP, p.Y, p.YP, p.dist, A, 0.0, e.c, 1, 4, ap, e) && ok;
+  ok = bend_slices_fast<false>(p.X, p.XP, p.Y, p.YP, dist, A, 0.0, c, 1, 4, nullptr, e) && ok;
   const double d = (A * A - p.XP * p.XP) - p.YP * p.YP;
   r = fp_sqrt_recip(d, ir);
-  ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10);
+  ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10) && fp_plain(dist, FP_HI_2P100);
   f = fp_quot(1.0, r, ir);
   p.XP = p.XP * f;
   p.YP = p.YP * f;
+  p.CT = p.CT + fp_quot(dist, p.beta0, fp_recip(p.beta0));
   if (ok)
     pio = p;
   return ok;
 }
 
-/* one kick: optional wake kick of the previous kick, one integrator slice,
- * c*t update, min/max of c*t (csbend.c:2385-2450, :3066-3076) */
-/* 64 registers (4 blocks of 256 per SM): twice the resident warps of the
- * unconstrained build, the FP64 chains' latency being what limits it */
-__global__ void __launch_bounds__(256, 4) csr_slice_kernel(DevParticles P, int64_t n, const double *beta0, const DevElem *ep,
-                                 const DevAperture *ap, CsrBunches B, int after_first_kick, int nBins, double Po,
-                                 int pass, int elem_index) {
+constexpr int SLICE_THREADS = 128, SLICE_COLS = 7;
+
+__device__ __forceinline__ void copy8_async(void *smem, const void *gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+               : "memory");
+}
+__device__ __forceinline__ void copy4_async(void *smem, const void *gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+               : "memory");
+}
+
+/* One kick of every particle, and min/max of c*t per bunch (csbend.c:3066-3076).
+ * Each block takes a run of 128-particle tiles; a thread copies its particle of
+ * the next tile into shared memory (its own words only, so no barrier) while it
+ * integrates the current one.  Bound by issue: about 840 warp instructions, 410
+ * of them FP64, per warp of particles.  Before, a block per 256 particles waited
+ * for the loss word, then for the coordinates, then for the velocity, and every
+ * warp sent two atomics to the bunch's range words; here the range stays in
+ * registers until the bunch changes. */
+__global__ void __launch_bounds__(SLICE_THREADS, 6)
+    csr_slice_kernel(DevParticles P, int64_t n, int64_t tiles_per_block, const double *beta0,
+                     const __grid_constant__ DevElem e, CsrBunches B, int after_first_kick, int nBins, double Po,
+                     double inv_Po, int pass, int elem_index) {
+  __shared__ double col[2][SLICE_COLS][SLICE_THREADS];
+  __shared__ int32_t lost_word[2][SLICE_THREADS];
   chain_enter();
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  bool alive = i < n && P.lost_pass[i] < 0;
-  const int b = i < n ? bunch_of(i, B) : B.n - 1;
-  const CsrDevState *st = B.st + b;
-  const int apply_kick = after_first_kick && B.csr_const[b] != 0;
-  double CT = 0;
-  if (alive) {
-    const DevElem &e = *ep;
-    const double *c = e.c;
-    SlicePart p = {P.x[i], P.xp[i], P.y[i], P.yp[i], P.dp[i], 0};
-    CT = P.s[i];
-    if (apply_kick)
-      p.DP = csr_kick(CT, p.X, p.DP, st, nBins, Po, c[CB_RHO0]);
-    int lost = 0;
-    if (!((e.flags & EF_FAST) && c[CB_NSUB] == 4 && csr_slice_fast(p, e, ap))) {
-      SlicePart t = p;
-      lost = csr_slice_general(&t, &e, ap);
-      p = t;
+  const int t = threadIdx.x;
+  const int64_t begin = blockIdx.x * tiles_per_block * SLICE_THREADS + t;
+  const int64_t end = min(n, (blockIdx.x + 1) * tiles_per_block * SLICE_THREADS);
+  const bool straight = (e.flags & EF_FAST) && e.c[CB_NSUB] == 4 && fp_within(Po, FP_HI_2M10, FP_HI_2P100);
+  auto fetch = [&](int64_t i, int slot) {
+    if (i < end) {
+      copy8_async(&col[slot][0][t], P.x + i);
+      copy8_async(&col[slot][1][t], P.xp + i);
+      copy8_async(&col[slot][2][t], P.y + i);
+      copy8_async(&col[slot][3][t], P.yp + i);
+      copy8_async(&col[slot][4][t], P.s + i);
+      copy8_async(&col[slot][5][t], P.dp + i);
+      copy8_async(&col[slot][6][t], beta0 + i);
+      copy4_async(&lost_word[slot][t], P.lost_pass + i);
     }
-    P.x[i] = p.X;
-    P.xp[i] = p.XP;
-    P.y[i] = p.Y;
-    P.yp[i] = p.YP;
-    P.dp[i] = p.DP;
-    if (lost) {
-      P.lost_pass[i] = pass;
-      P.lost_elem[i] = elem_index;
-      alive = false;
-    } else {
-      CT = CT + p.dist / beta0[i];
-      P.s[i] = CT;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  /* the warp's bunch so far and its range of c*t over this thread's particles */
+  int bunch = begin - t < n ? bunch_of(begin - t, B) : 0, cur = bunch;
+  int64_t bunch_end = B.n <= 1 ? n : B.offs[bunch + 1];
+  unsigned long long kmin = ~0ull, kmax = 0ull;
+  auto flush = [&]() {
+    for (int off = 16; off > 0; off >>= 1) {
+      kmin = min(kmin, __shfl_down_sync(0xffffffffu, kmin, off));
+      kmax = max(kmax, __shfl_down_sync(0xffffffffu, kmax, off));
+    }
+    if ((t & 31) == 0 && kmax != 0ull) {
+      atomicMin(&B.st[cur].ct_min_key, kmin);
+      atomicMax(&B.st[cur].ct_max_key, kmax);
+    }
+    kmin = ~0ull;
+    kmax = 0ull;
+  };
+  fetch(begin, 0);
+  int slot = 0;
+  /* the loop's bounds are the same for all threads of the block */
+  for (int64_t i = begin; i - t < end; i += SLICE_THREADS, slot ^= 1) {
+    fetch(i + SLICE_THREADS, slot ^ 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    while (i < end && i >= bunch_end && bunch < B.n - 1) {
+      bunch++;
+      bunch_end = B.offs[bunch + 1];
+    }
+    const CsrDevState *st = B.st + bunch;
+    bool alive = i < end && lost_word[slot][t] < 0;
+    SlicePart p;
+    if (alive) {
+      p = {col[slot][0][t], col[slot][1][t], col[slot][2][t], col[slot][3][t], col[slot][4][t], col[slot][5][t],
+           col[slot][6][t]};
+      const SliceWake w = {st->dGamma, st->ctLower, st->dct, nBins, after_first_kick && B.csr_const[bunch] != 0};
+      int lost = 0;
+      if (!(straight && (!w.apply || fp_within(w.dct, FP_HI_2M250, FP_HI_2P100)) &&
+            csr_slice_fast(p, e, w, fp_recip(w.dct), Po, inv_Po))) {
+        SlicePart q = p;
+        lost = csr_slice_general(&q, &e, st, nBins, w.apply, Po);
+        p = q;
+      }
+      P.x[i] = p.X;
+      P.xp[i] = p.XP;
+      P.y[i] = p.Y;
+      P.yp[i] = p.YP;
+      P.dp[i] = p.DP;
+      if (lost) {
+        P.lost_pass[i] = pass;
+        P.lost_elem[i] = elem_index;
+        alive = false;
+      } else {
+        P.s[i] = p.CT;
+      }
+    }
+    __syncwarp();
+    const int b0 = __shfl_sync(0xffffffffu, bunch, 0);
+    if (__all_sync(0xffffffffu, bunch == b0)) {
+      if (b0 != cur) {
+        flush();
+        cur = b0;
+      }
+      if (alive) {
+        const unsigned long long k = key_of(p.CT);
+        kmin = min(kmin, k);
+        kmax = max(kmax, k);
+      }
+    } else if (alive) {
+      /* the warp straddles bunches here */
+      atomicMin(&B.st[bunch].ct_min_key, key_of(p.CT));
+      atomicMax(&B.st[bunch].ct_max_key, key_of(p.CT));
     }
   }
-  bunch_minmax(CT, alive, b, B);
+  flush();
+}
+
+/* grid and tiles per block: as many blocks as the SMs hold at once, each with
+ * an equal run of tiles */
+static inline int slice_grid(int64_t n, int64_t *tiles_per_block) {
+  const int64_t tiles = std::max<int64_t>(1, (n + SLICE_THREADS - 1) / SLICE_THREADS);
+  *tiles_per_block = (tiles + 148 * 8 - 1) / (148 * 8);
+  return (int)((tiles + *tiles_per_block - 1) / *tiles_per_block);
 }
 
 /* histogram of c*t with the range of binParticleCoordinate (csbend.c:3047-3113):
@@ -1985,8 +2099,10 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
       csr_reset_keys_kernel<<<1, 32, 0, stream>>>(B);
       (*launches)++;
     }
-    CSR_CUDA(launch_chained(csr_slice_kernel, dim3(g), dim3(256), 0, stream, P, n, (const double *)st.d_beta0, d_e,
-                            (const DevAperture *)nullptr, B, (int)(kick > 0), ce.bins, Po, pass, elem));
+    int64_t per_block;
+    const int slice_blocks = slice_grid(n, &per_block);
+    CSR_CUDA(launch_chained(csr_slice_kernel, dim3(slice_blocks), dim3(SLICE_THREADS), 0, stream, P, n, per_block,
+                            (const double *)st.d_beta0, h_elem, B, (int)(kick > 0), ce.bins, Po, 1 / Po, pass, elem));
     (*launches)++;
     CSR_CUDA(cudaGetLastError());
     if (!any_active)
@@ -2459,7 +2575,10 @@ extern "C" int b2e_csr_bend_static(double *const dev_columns[6], int32_t *dev_lo
   double phiBend = 0;
   for (int kick = 0; kick < nSlices; kick++) {
     csr_reset_keys_kernel<<<1, 32, 0, s>>>(B);
-    csr_slice_kernel<<<g, 256, 0, s>>>(P, n, S->beta0, &S->elem, nullptr, B, kick > 0, bins, Po, 0, 0);
+    int64_t per_block;
+    const int slice_blocks = slice_grid(n, &per_block);
+    csr_slice_kernel<<<slice_blocks, SLICE_THREADS, 0, s>>>(P, n, per_block, S->beta0, d, B, kick > 0, bins, Po, 1 / Po,
+                                                            0, 0);
     STATIC_TRY(cudaGetLastError());
     STATIC_TRY(cudaMemsetAsync(S->counts, 0, sizeof(unsigned int) * bins, s));
     int hb = hist_blocks(n, 1);
