@@ -502,8 +502,8 @@ __global__ void csr_hist_kernel(DevParticles P, int64_t n, CsrBunches B, unsigne
 
 struct WakeArgs {
   int nBins, sgHalf, sgdHalf, trapz, steady, correct;
-  const double *sg_w, *sgd_w; /* [nBins][B2E_SG_MAX_WIDTH] */
-  const int *sg_lo, *sg_n, *sgd_lo, *sgd_n;
+  /* Savitzky-Golay weights of smoothing and derivative (sg_table) */
+  const double *sg_w, *sgd_w;
   double slippage, slippage13, c1, c2, csr_constant;
   double length, nSlices;   /* element length and kicks: c1 and c2 of each bunch */
   double *wakelog;          /* nBins values per bunch for this kick, or null */
@@ -566,13 +566,31 @@ __device__ void lh_pass_filters(const WakeArgs &a, double *sm) {
   }
 }
 
-/* Savitzky-Golay pass with precomputed per-bin weights (b2e_sg.h convention);
- * lo/wn point into an interleaved (start, width) table, stride 2 per bin. */
-__device__ void sg_apply(const double *in, double *out, int nBins, const double *w, const int *lo, const int *wn) {
-  for (int b = threadIdx.x; b < nBins; b += blockDim.x) {
+/* Savitzky-Golay weights of a filter over nb bins.  The window of bin b is
+ * width = min(2 half + 1, nb) bins from start = clamp(b - half, 0, nb - width)
+ * (b2e_sg_window), and its weights depend on b - start only: [row][width], row =
+ * b - start, width rows. */
+B2E_SG_FN int sg_width(int half, int nb) { return half <= 0 ? 1 : (2 * half + 1 < nb ? 2 * half + 1 : nb); }
+B2E_SG_FN void sg_row(int half, int order, int deriv, int nb, int row, double *w) {
+  const long width = sg_width(half, nb), ord = order < width - 1 ? order : width - 1;
+  double t[B2E_SG_MAX_WIDTH];
+  /* no window: the bin itself; the derivative of a constant fit is zero */
+  if (half <= 0 && deriv == 0)
+    w[0] = 1;
+  else if (deriv > ord || b2e_sg_weights(t, width, -(long)row, ord, deriv))
+    for (int k = 0; k < width; k++)
+      w[k] = 0;
+  else
+    for (int k = 0; k < width; k++)
+      w[k] = t[k];
+}
+
+__device__ void sg_apply(const double *in, double *out, int nb, int half, const double *w) {
+  const int width = sg_width(half, nb);
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
+    const int start = half <= 0 ? b : min(max(b - half, 0), nb - width);
+    const double *wb = w + (b - start) * width;
     double s = 0;
-    const double *wb = w + (size_t)b * B2E_SG_MAX_WIDTH;
-    const int start = lo[2 * b], width = wn[2 * b];
     for (int k = 0; k < width; k++)
       s += wb[k] * in[start + k];
     out[b] = s;
@@ -610,31 +628,35 @@ __device__ __forceinline__ double ordered_sum(const double *v, int n) {
   return s;
 }
 
-/* bring this thread's rows of both Savitzky-Golay tables toward L1 while the
- * counts load, so that the two filter passes do not wait on L2 */
-__device__ __forceinline__ void prefetch_sg_rows(const WakeArgs &a) {
-  for (int b = threadIdx.x; b < a.nBins; b += blockDim.x) {
-    if (a.sgHalf > 0) {
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(a.sg_w + (size_t)b * B2E_SG_MAX_WIDTH));
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(a.sg_lo + 2 * b));
-    }
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(a.sgd_w + (size_t)b * B2E_SG_MAX_WIDTH));
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(a.sgd_lo + 2 * b));
-  }
-}
+/* weights up to this many per table are staged in shared memory (windows of 17) */
+constexpr int SG_STAGE = 17 * 17;
 
 /* Filters of one kick's wake (csbend.c:2566-2591) on one CTA: Savitzky-Golay
  * smoothing of the counts, correctDistribution, density per unit ct, its
  * derivative filter and the (dct*b)^(1/3) denominators.  Leaves hist = sm,
- * deriv = sm + nBins, denom = sm + 2 nBins (tmp = sm + 3 nBins is scratch). */
-template <typename CountT, typename SumT>
-__device__ void wake_filters(const CountT *counts, const WakeArgs &a, const double dct, double *sm, SumT *nbinned_out) {
+ * deriv = sm + nBins, denom = sm + 2 nBins (tmp = sm + 3 nBins is scratch) and,
+ * with INVERSE, 1/denom at sm + 4 nBins + 8; returns whether the quotients
+ * deriv/denom may be formed with them (fp_quot): every value plain. */
+template <typename CountT, typename SumT, bool INVERSE = false>
+__device__ bool wake_filters(const CountT *counts, const WakeArgs &a, const double dct, double *sm, SumT *nbinned_out) {
   const int nb = a.nBins;
+  double *inv = sm + 4 * nb + 8;
   double *hist = sm, *deriv = sm + nb, *denom = sm + 2 * nb, *tmp = sm + 3 * nb;
   __shared__ double nBinnedD;
   __shared__ int skip;
   __shared__ SumT warp_sums[32];
-  prefetch_sg_rows(a);
+  __shared__ double stage[2][SG_STAGE];
+  /* the weights come in with the counts */
+  const int w0 = sg_width(a.sgHalf, nb), w1 = sg_width(a.sgdHalf, nb);
+  const double *sg_w = a.sg_w, *sgd_w = a.sgd_w;
+  if (w0 * w0 <= SG_STAGE && w1 * w1 <= SG_STAGE) {
+    for (int k = threadIdx.x; k < w0 * w0; k += blockDim.x)
+      stage[0][k] = sg_w[k];
+    for (int k = threadIdx.x; k < w1 * w1; k += blockDim.x)
+      stage[1][k] = sgd_w[k];
+    sg_w = stage[0];
+    sgd_w = stage[1];
+  }
   if constexpr (std::is_integral<SumT>::value) {
     /* integer counts: the total is exact in any order, so it is a block
      * reduction (per thread, warp shuffles, then the warps' totals) */
@@ -675,7 +697,7 @@ __device__ void wake_filters(const CountT *counts, const WakeArgs &a, const doub
   if (a.lh)
     lh_pass_filters(a, sm);
   if (a.sgHalf > 0) {
-    sg_apply(hist, tmp, nb, a.sg_w, a.sg_lo, a.sg_n);
+    sg_apply(hist, tmp, nb, a.sgHalf, sg_w);
     __syncthreads();
     /* correctDistribution (csbend.c:4705-4721): negative bins clipped in
      * parallel, then the sum in bin order, as the reference forms it */
@@ -691,8 +713,12 @@ __device__ void wake_filters(const CountT *counts, const WakeArgs &a, const doub
       else
         deriv[0] = nBinnedD / sum; /* factor, parked in deriv[0] */
     } else if (threadIdx.x >= 32) {
-      for (int b = threadIdx.x - 32; b < nb; b += blockDim.x - 32)
-        denom[b] = b2e_pow13(dct * b);
+      for (int b = threadIdx.x - 32; b < nb; b += blockDim.x - 32) {
+        const double v = b2e_pow13(dct * b);
+        denom[b] = v;
+        if (INVERSE)
+          inv[b] = fp_recip(v);
+      }
     }
     __syncthreads();
     const double factor = deriv[0];
@@ -703,17 +729,24 @@ __device__ void wake_filters(const CountT *counts, const WakeArgs &a, const doub
   }
   const bool denom_done = a.sgHalf > 0 && blockDim.x > 32;
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    if (!denom_done)
+    if (!denom_done) {
       denom[b] = b2e_pow13(dct * b);
+      if (INVERSE)
+        inv[b] = fp_recip(denom[b]);
+    }
     hist[b] = hist[b] / dct;
-    deriv[b] = hist[b];
   }
   __syncthreads();
-  sg_apply(deriv, tmp, nb, a.sgd_w, a.sgd_lo, a.sgd_n);
-  __syncthreads();
+  sg_apply(hist, deriv, nb, a.sgdHalf, sgd_w);
+  if (!INVERSE) {
+    __syncthreads();
+    return false;
+  }
+  /* each thread checks the values it wrote */
+  bool plain = fp_within(dct, FP_HI_2M250, FP_HI_2P100);
   for (int b = threadIdx.x; b < nb; b += blockDim.x)
-    deriv[b] = tmp[b];
-  __syncthreads();
+    plain = plain && fp_plain(deriv[b], FP_HI_2P700);
+  return __syncthreads_and(plain);
 }
 
 /* bins of slippage; clamped to [0, nb] so indexing stays in bounds for a
@@ -769,6 +802,58 @@ __device__ __forceinline__ void wake_terms(int ib, const WakeArgs &a, const doub
   *T2out = T2;
 }
 
+/* The same for the bins ib = first + m*stride, m < NI, of one thread, with the
+ * quotients deriv/denom through the stored reciprocals (three operations each)
+ * and each (denom, 1/denom) pair read once for all NI bins.  Every sum is in
+ * wake_terms' order; the steady and the transient integral differ in the
+ * length of the sum and in the halved first term. */
+template <int NI>
+__device__ void wake_terms_inverse(int first, int stride, const WakeArgs &a, const double dct, const double *hist,
+                                   const double *deriv, const double *denom, const double *inv, long long diS,
+                                   long long diS4, double *T1, double *T2) {
+  const int nb = a.nBins;
+  int len[NI]; /* terms of each sum; nonincreasing in m */
+  double last[NI];
+#pragma unroll
+  for (int m = 0; m < NI; m++) {
+    const int ib = first + m * stride;
+    const long long room = nb - 1 - ib;
+    len[m] = ib < nb ? (int)(a.steady || room < diS ? room : diS) : 0;
+    T1[m] = T2[m] = last[m] = 0;
+  }
+  int k = 1;
+#pragma unroll
+  for (int live = NI; live > 0; live--)
+    for (; k <= len[live - 1]; k++) {
+      const double b = denom[k], y = inv[k];
+#pragma unroll
+      for (int m = 0; m < live; m++) {
+        last[m] = fp_quot(deriv[first + m * stride + k], b, y);
+        T1[m] += last[m];
+      }
+    }
+#pragma unroll
+  for (int m = 0; m < NI; m++) {
+    const int ib = first + m * stride;
+    if (ib >= nb)
+      continue;
+    if (a.trapz) {
+      if ((a.steady || diS > 0) && ib + 1 < nb)
+        T1[m] += 0.3 * (denom[1] * denom[1]) * (2 * deriv[ib + 1] + 3 * deriv[ib]) / dct;
+      if (len[m] > 1) {
+        const double t = fp_quot(deriv[ib + 1], denom[1], inv[1]);
+        T1[m] -= ((a.steady ? t : t / 2) + last[m]) / 2;
+      }
+    }
+    if (!a.steady) {
+      if (ib + diS < nb)
+        T2[m] += hist[ib + diS];
+      if (ib + diS4 < nb)
+        T2[m] -= hist[ib + diS4];
+    }
+  }
+}
+
 /* Steady-state wake by the integrated Green's function (csbend.c:2593-2621,
  * :2676-2680, convolveArrays1 :5484-5491): chi(z) per bin, its second
  * difference, the one-sided convolution with the density (per-bin serial
@@ -820,16 +905,16 @@ __device__ void igf_wake(const WakeArgs &a, const double dct, const double *hist
 
 /* Wake of one kick (csbend.c:2566-2673) on one CTA, from a histogram of
  * counts (unsigned counts in tracking, real-valued counts for batched
- * profiles).  sm holds 4*nBins + 8 doubles.  Writes dgamma[nBins], the wake log
+ * profiles).  sm holds 5*nBins + 8 doubles.  NI: bins a thread takes at a time.  Writes dgamma[nBins], the wake log
  * when a.wakelog is set, the binned total when nbinned_out is set, and the
  * smoothed density (per unit ct) and its derivative when hist_out/deriv_out
  * are set. */
-template <typename CountT, typename SumT>
+template <typename CountT, typename SumT, int NI>
 __device__ void wake_body(const CountT *counts, const WakeArgs &a, const double dct, double *sm, double *dgamma,
                           SumT *nbinned_out, double *hist_out, double *deriv_out, double *page = nullptr) {
   const int nb = a.nBins;
-  wake_filters<CountT, SumT>(counts, a, dct, sm, nbinned_out);
-  const double *hist = sm, *deriv = sm + nb, *denom = sm + 2 * nb;
+  const bool inverse = wake_filters<CountT, SumT, true>(counts, a, dct, sm, nbinned_out);
+  const double *hist = sm, *deriv = sm + nb, *denom = sm + 2 * nb, *inv = sm + 4 * nb + 8;
   double *page_t1 = page ? page + 2 * nb : nullptr, *page_t2 = page ? page + 3 * nb : nullptr;
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     if (hist_out)
@@ -857,20 +942,31 @@ __device__ void wake_body(const CountT *counts, const WakeArgs &a, const double 
     igf_wake(a, dct, hist, sm + 3 * nb, sm + 2 * nb, dgamma);
     return;
   }
-  for (int ib = threadIdx.x; ib < nb; ib += blockDim.x) {
-    double T1 = 0, T2 = 0;
-    if (a.csr_constant) {
-      wake_terms(ib, a, dct, hist, deriv, denom, diS, diS4, &T1, &T2);
-      T1 *= a.c1;
-      T2 *= a.c2;
-    }
-    double dg = T1 + T2;
-    dgamma[ib] = dg;
-    if (a.wakelog)
-      a.wakelog[ib] = dg;
-    if (page) {
-      page_t1[ib] = T1;
-      page_t2[ib] = T2;
+  for (int i0 = threadIdx.x; i0 < nb; i0 += NI * blockDim.x) {
+    double T1[NI], T2[NI];
+    if (inverse && a.csr_constant)
+      wake_terms_inverse<NI>(i0, blockDim.x, a, dct, hist, deriv, denom, inv, diS, diS4, T1, T2);
+#pragma unroll
+    for (int m = 0; m < NI; m++) {
+      const int ib = i0 + m * blockDim.x;
+      if (ib >= nb)
+        break;
+      if (!a.csr_constant)
+        T1[m] = T2[m] = 0;
+      else {
+        if (!inverse)
+          wake_terms(ib, a, dct, hist, deriv, denom, diS, diS4, &T1[m], &T2[m]);
+        T1[m] *= a.c1;
+        T2[m] *= a.c2;
+      }
+      const double dg = T1[m] + T2[m];
+      dgamma[ib] = dg;
+      if (a.wakelog)
+        a.wakelog[ib] = dg;
+      if (page) {
+        page_t1[ib] = T1[m];
+        page_t2[ib] = T2[m];
+      }
     }
   }
 }
@@ -927,7 +1023,7 @@ __global__ void __launch_bounds__(1024, 1) csr_wake_kernel(CsrBunches B, unsigne
   w.igf_factor = igf_factor;
   w.wakelog = a.wakelog ? a.wakelog + (size_t)bunch * a.nBins : nullptr;
   unsigned int *counts = counts_all + (size_t)bunch * a.nBins;
-  wake_body<unsigned int, long long>(counts, w, dct, sm, st->dGamma, &st->nBinned, nullptr, nullptr, page);
+  wake_body<unsigned int, long long, 1>(counts, w, dct, sm, st->dGamma, &st->nBinned, nullptr, nullptr, page);
   if (recycle) /* the counts were copied to shared memory before the first barrier */
     for (int b = threadIdx.x; b < a.nBins; b += blockDim.x)
       counts[b] = 0;
@@ -1083,20 +1179,34 @@ __global__ void __launch_bounds__(1024, 1) csr_sur_combine_kernel(CsrBunches B, 
 
 /* Batched wake integral of many profiles in bin units (dct = 1), one CTA per
  * profile: out = T1 (c1 = 1, no T2 term) for the profile's slippage in bins;
- * hist_out/deriv_out receive the smoothed density and its derivative. */
-__global__ void wake_batch_kernel(const double *counts, const double *slippage_bins, WakeArgs a, double *t1_out,
-                                  double *hist_out, double *deriv_out) {
+ * hist_out/deriv_out receive the smoothed density and its derivative.  The
+ * filters' weights come as an argument (windows up to 17 bins: no table to
+ * allocate and fill per call) or, for wider windows, from a.sg_w.
+ * 256 threads with four bins each: the integral's 0.3 million terms per
+ * 1,024-bin profile are bound by the FP64 pipe (four operations a term), with
+ * 2.5 shared-memory words read per term instead of two per division. */
+constexpr int BATCH_THREADS = 256, BATCH_BINS = 4;
+struct SgTables {
+  double w[2][SG_STAGE];
+};
+__global__ void __launch_bounds__(BATCH_THREADS)
+    wake_batch_kernel(const double *counts, const double *slippage_bins, WakeArgs a, const __grid_constant__ SgTables sg,
+                      double *t1_out, double *hist_out, double *deriv_out) {
   extern __shared__ double sm[];
   const size_t off = (size_t)blockIdx.x * a.nBins;
   WakeArgs w = a;
+  if (!w.sg_w) {
+    w.sg_w = sg.w[0];
+    w.sgd_w = sg.w[1];
+  }
   w.slippage = slippage_bins[blockIdx.x];
   w.slippage13 = 1;
   w.c1 = 1;
   w.c2 = 0;
   w.csr_constant = 1;
   w.wakelog = nullptr;
-  wake_body<double, double>(counts + off, w, 1.0, sm, t1_out + off, (double *)nullptr, hist_out + off,
-                            deriv_out + off);
+  wake_body<double, double, BATCH_BINS>(counts + off, w, 1.0, sm, t1_out + off, (double *)nullptr, hist_out + off,
+                                        deriv_out + off);
 }
 
 /* after the last kick: its wake kick and the min/max for the exit binning */
@@ -1458,7 +1568,6 @@ int csr_configure(CsrState &st, const b2e_element *el, int n, const CompiledLatt
   if (!st.enabled)
     return B2E_OK;
   std::vector<double> sgw;
-  std::vector<int> sgi;
   st.sg_offset.clear();
   for (int idx : lat.csr_elements) {
     const b2e_element &e = el[idx];
@@ -1528,27 +1637,15 @@ int csr_configure(CsrState &st, const b2e_element *el, int n, const CompiledLatt
         if (el[j].type != B2E_MARK)
           break;
       }
-      /* per-bin Savitzky-Golay weights for smoothing (order sgOrder, derivative 0)
+      /* Savitzky-Golay weights for smoothing (order sgOrder, derivative 0)
        * and for the derivative (order sgdOrder, derivative 1) */
       st.sg_offset.push_back(sgw.size());
       for (int pass = 0; pass < 2; pass++) {
-        int half = pass == 0 ? ce.sgHalf : ce.sgdHalf, order = pass == 0 ? ce.sgOrder : ce.sgdOrder;
-        for (int b = 0; b < ce.bins; b++) {
-          double w[B2E_SG_MAX_WIDTH] = {0};
-          long width;
-          long lo = b2e_sg_window(b, ce.bins, half, half, &width);
-          long ord = order < width - 1 ? order : width - 1;
-          if (pass == 0 && half <= 0) {
-            width = 1;
-            lo = b;
-            w[0] = 1;
-          } else if ((pass == 1 && 1 > ord) || b2e_sg_weights(w, width, lo - b, ord, pass)) {
-            width = 0; /* derivative of a constant fit: zero */
-          }
-          for (int k = 0; k < B2E_SG_MAX_WIDTH; k++)
-            sgw.push_back(w[k]);
-          sgi.push_back((int)lo);
-          sgi.push_back((int)width);
+        const int half = pass == 0 ? ce.sgHalf : ce.sgdHalf, order = pass == 0 ? ce.sgOrder : ce.sgdOrder;
+        const int width = sg_width(half, ce.bins);
+        for (int row = 0; row < width; row++) {
+          sgw.resize(sgw.size() + width);
+          sg_row(half, order, pass, ce.bins, row, sgw.data() + sgw.size() - width);
         }
       }
     } else {
@@ -1587,15 +1684,12 @@ int csr_configure(CsrState &st, const b2e_element *el, int n, const CompiledLatt
   if (csr_set_bunches(st, 1, nullptr, err))
     return B2E_ERR_NOMEM;
   if (!sgw.empty()) {
-    if (cudaMalloc(&st.d_sg, sizeof(double) * sgw.size()) != cudaSuccess ||
-        cudaMalloc(&st.d_sg_idx, sizeof(int) * sgi.size()) != cudaSuccess) {
+    if (cudaMalloc(&st.d_sg, sizeof(double) * sgw.size()) != cudaSuccess) {
       err = "CSR weight allocation failed";
       return B2E_ERR_NOMEM;
     }
     cudaMemcpy(st.d_sg, sgw.data(), sizeof(double) * sgw.size(), cudaMemcpyHostToDevice);
-    cudaMemcpy(st.d_sg_idx, sgi.data(), sizeof(int) * sgi.size(), cudaMemcpyHostToDevice);
   }
-  /* the index array runs parallel to the weights: 2 ints per bin row */
   return B2E_OK;
 }
 
@@ -1862,7 +1956,6 @@ static int stupakov_drift(CsrState &st, const CsrElem &ce, const CsrBunches &B, 
   const double dz0 = length / nKicks;
   double dz = dz0 / 2, zTravel = zStart - st.z0;
   const double *sgw = st.d_sg + st.sg_offset[st.last_bend];
-  const int *sgi = st.d_sg_idx + st.sg_offset[st.last_bend] / B2E_SG_MAX_WIDTH * 2;
   WakeArgs a = {};
   a.nBins = nb;
   a.sgHalf = bend.sgHalf;
@@ -1870,11 +1963,7 @@ static int stupakov_drift(CsrState &st, const CsrElem &ce, const CsrBunches &B, 
   a.trapz = bend.trapz;
   a.correct = bend.sgHalf > 0;
   a.sg_w = sgw;
-  a.sgd_w = sgw + (size_t)nb * B2E_SG_MAX_WIDTH;
-  a.sg_lo = sgi;
-  a.sg_n = sgi + 1;
-  a.sgd_lo = sgi + 2 * nb;
-  a.sgd_n = sgi + 2 * nb + 1;
+  a.sgd_w = sgw + sg_width(bend.sgHalf, nb) * sg_width(bend.sgHalf, nb);
   set_filter_args(a, bend.lh, bend.clip, bend.lowCut0, bend.lowCut1, bend.highCut0, bend.highCut1);
   const size_t smem = sizeof(double) * (5 * nb + 8);
   CSR_CUDA(cudaFuncSetAttribute(stupakov_wake_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -2066,8 +2155,7 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
                            stream));
   CSR_CUDA(cudaMemcpyAsync(st.d_flags, flags.data(), flags.size(), cudaMemcpyHostToDevice, stream));
   const double *sgw = st.d_sg + st.sg_offset[k];
-  const int *sgi = st.d_sg_idx + st.sg_offset[k] / B2E_SG_MAX_WIDTH * 2;
-  const size_t wake_smem = sizeof(double) * (4 * ce.bins + 8);
+  const size_t wake_smem = sizeof(double) * (5 * ce.bins + 8);
   CSR_CUDA(cudaFuncSetAttribute(csr_wake_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wake_smem));
   /* learned wake: trained on the transient integral with trapezoid rule (the
    * CSRCSBEND defaults); other settings, or a bunch train larger than the
@@ -2132,11 +2220,7 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
     a.steady = ce.steady;
     a.correct = ce.sgHalf > 0;
     a.sg_w = sgw;
-    a.sgd_w = sgw + (size_t)ce.bins * B2E_SG_MAX_WIDTH;
-    a.sg_lo = sgi;
-    a.sg_n = sgi + 1;
-    a.sgd_lo = sgi + 2 * ce.bins;
-    a.sgd_n = sgi + 2 * ce.bins + 1;
+    a.sgd_w = sgw + sg_width(ce.sgHalf, ce.bins) * sg_width(ce.sgHalf, ce.bins);
     a.slippage = slippage;
     a.slippage13 = b2e_pow(slippage, 1. / 3.);
     a.length = ce.length;
@@ -2309,8 +2393,6 @@ void csr_release(CsrState &st) {
   st.sur_cap_bunches = st.gate_cap = st.gate_values = 0;
   if (st.d_sg)
     cudaFree(st.d_sg);
-  if (st.d_sg_idx)
-    cudaFree(st.d_sg_idx);
   if (st.d_wakelog)
     cudaFree(st.d_wakelog);
   if (st.d_pagelog)
@@ -2326,7 +2408,6 @@ void csr_release(CsrState &st) {
   st.d_state = nullptr;
   st.d_counts = nullptr;
   st.d_sg = nullptr;
-  st.d_sg_idx = nullptr;
   st.d_wakelog = nullptr;
   st.beta0_cap = 0;
   st.wakelog_cap = 0;
@@ -2367,8 +2448,7 @@ struct StaticCsrScratch {
   double beta0[B2E_STATIC_MAX_PARTICLES];
   CsrDevState state;
   unsigned int counts[B2E_STATIC_MAX_BINS];
-  double sg_w[2 * B2E_STATIC_MAX_BINS * B2E_SG_MAX_WIDTH];
-  int sg_idx[2 * B2E_STATIC_MAX_BINS * 2];
+  double sg_w[2 * B2E_SG_MAX_WIDTH * B2E_SG_MAX_WIDTH];
   DevElem elem;
   unsigned long long counters[2];
   double csr_const[2];    /* the one bunch's CSRConstant and IGF wake factor */
@@ -2411,9 +2491,6 @@ static StaticCsrScratch *static_scratch(char *err, int64_t errlen) {
 
 __global__ void static_set_elem_kernel(DevElem e, DevElem *dst) { *dst = e; }
 
-/* Savitzky-Golay weight tables for one element, on the device, with the same
- * helpers and layout as csr_configure (rows of B2E_SG_MAX_WIDTH weights;
- * interleaved (start, width) index pairs; smoothing rows then derivative rows). */
 /* The bunch's flags from the entrance count (S->counters[1] = particles alive
  * at the entrance; CSR only for more than one, csbend.c:1987), formed on the
  * device so that the host never waits for the count. */
@@ -2425,30 +2502,15 @@ __global__ void static_set_bunch_kernel(StaticCsrScratch *S, double csr_constant
   S->flags[1] = 0;
 }
 
-__global__ void static_sg_weights_kernel(int bins, int sgHalf, int sgOrder, int sgdHalf, int sgdOrder, double *w,
-                                         int *idx) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= 2 * bins)
-    return;
-  const int pass = row >= bins, b = row - pass * bins;
-  const int half = pass == 0 ? sgHalf : sgdHalf, order = pass == 0 ? sgOrder : sgdOrder;
-  double ww[B2E_SG_MAX_WIDTH];
-  for (int k = 0; k < B2E_SG_MAX_WIDTH; k++)
-    ww[k] = 0;
-  long width;
-  long lo = b2e_sg_window(b, bins, half, half, &width);
-  long ord = order < width - 1 ? order : width - 1;
-  if (pass == 0 && half <= 0) {
-    width = 1;
-    lo = b;
-    ww[0] = 1;
-  } else if ((pass == 1 && 1 > ord) || b2e_sg_weights(ww, width, lo - b, ord, pass)) {
-    width = 0;
-  }
-  for (int k = 0; k < B2E_SG_MAX_WIDTH; k++)
-    w[(size_t)row * B2E_SG_MAX_WIDTH + k] = ww[k];
-  idx[2 * row] = (int)lo;
-  idx[2 * row + 1] = (int)width;
+/* Savitzky-Golay weights for one element, on the device, with the same helpers
+ * and layout as csr_configure: smoothing rows, then derivative rows. */
+__global__ void static_sg_weights_kernel(int bins, int sgHalf, int sgOrder, int sgdHalf, int sgdOrder, double *w) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int w0 = sg_width(sgHalf, bins), w1 = sg_width(sgdHalf, bins);
+  if (t < w0)
+    sg_row(sgHalf, sgOrder, 0, bins, t, w + t * w0);
+  else if (t < w0 + w1)
+    sg_row(sgdHalf, sgdOrder, 1, bins, t - w0, w + w0 * w0 + (t - w0) * w1);
 }
 
 #define STATIC_TRY(call)                                                                                          \
@@ -2538,8 +2600,7 @@ extern "C" int b2e_csr_bend_static(double *const dev_columns[6], int32_t *dev_lo
   P.lost_elem = dev_lost_element;
 
   static_set_elem_kernel<<<1, 1, 0, s>>>(d, &S->elem);
-  static_sg_weights_kernel<<<(2 * bins + 127) / 128, 128, 0, s>>>(bins, sgHalf, sgOrder, sgdHalf, sgdOrder, S->sg_w,
-                                                                  S->sg_idx);
+  static_sg_weights_kernel<<<1, 2 * B2E_SG_MAX_WIDTH, 0, s>>>(bins, sgHalf, sgOrder, sgdHalf, sgdOrder, S->sg_w);
   STATIC_TRY(cudaGetLastError());
   /* particles alive at the entrance decide whether CSR is computed
    * (csbend.c:1987): counted and turned into the bunch's flags on the device;
@@ -2568,7 +2629,7 @@ extern "C" int b2e_csr_bend_static(double *const dev_columns[6], int32_t *dev_lo
 
   /* the wake kernel's shared-memory limit is a per-function setting that the
    * context path also changes: set it for this call's bin count */
-  const size_t wake_smem = sizeof(double) * (4 * bins + 8);
+  const size_t wake_smem = sizeof(double) * (5 * bins + 8);
   STATIC_TRY(cudaFuncSetAttribute(csr_wake_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wake_smem));
   csr_entry_kernel<<<g, 256, 0, s>>>(P, n, S->beta0, &S->elem, bx, Po);
   STATIC_TRY(cudaGetLastError());
@@ -2594,11 +2655,7 @@ extern "C" int b2e_csr_bend_static(double *const dev_columns[6], int32_t *dev_lo
     a.steady = p[B2E_BEND_STEADY_STATE] != 0;
     a.correct = sgHalf > 0;
     a.sg_w = S->sg_w;
-    a.sgd_w = S->sg_w + (size_t)bins * B2E_SG_MAX_WIDTH;
-    a.sg_lo = S->sg_idx;
-    a.sg_n = S->sg_idx + 1;
-    a.sgd_lo = S->sg_idx + 2 * bins;
-    a.sgd_n = S->sg_idx + 2 * bins + 1;
+    a.sgd_w = S->sg_w + sg_width(sgHalf, bins) * sg_width(sgHalf, bins);
     a.slippage = slippage;
     a.slippage13 = b2e_pow(slippage, 1. / 3.);
     a.length = length;
@@ -2707,6 +2764,11 @@ extern "C" int b2e_wake_t1_from_output(const float *dev_y, const double *dev_sca
 /* Batched wake integral for the wake-network data set: n_profiles histograms
  * of `bins` real-valued counts, each with its own slippage in bins. */
 using b2e::WakeArgs;
+using b2e::BATCH_THREADS;
+using b2e::sg_row;
+using b2e::sg_width;
+using b2e::SG_STAGE;
+using b2e::SgTables;
 using b2e::static_sg_weights_kernel;
 using b2e::wake_batch_kernel;
 extern "C" int b2e_csr_wake_batch(const double *dev_counts, const double *dev_slippage_bins, int32_t n_profiles,
@@ -2729,16 +2791,22 @@ extern "C" int b2e_csr_wake_batch(const double *dev_counts, const double *dev_sl
   if (n_profiles == 0)
     return B2E_OK;
   cudaStream_t s = (cudaStream_t)stream;
+  /* windows up to 17 bins: the weights travel as a kernel argument; wider
+   * ones through a table in device memory */
+  const int w0 = sg_width(sg_halfwidth, bins), w1 = sg_width(sgd_halfwidth, bins);
+  SgTables tables = {};
   double *w = nullptr;
-  int *idx = nullptr;
-  if (cudaMallocAsync((void **)&w, sizeof(double) * 2 * bins * B2E_SG_MAX_WIDTH, s) != cudaSuccess)
-    return B2E_ERR_NOMEM;
-  if (cudaMallocAsync((void **)&idx, sizeof(int) * 4 * bins, s) != cudaSuccess) {
-    cudaFreeAsync(w, s);
-    return B2E_ERR_NOMEM;
+  if (w0 * w0 <= SG_STAGE && w1 * w1 <= SG_STAGE) {
+    for (int row = 0; row < w0; row++)
+      sg_row(sg_halfwidth, sg_order, 0, bins, row, tables.w[0] + row * w0);
+    for (int row = 0; row < w1; row++)
+      sg_row(sgd_halfwidth, sgd_order, 1, bins, row, tables.w[1] + row * w1);
+  } else {
+    if (cudaMallocAsync((void **)&w, sizeof(double) * (w0 * w0 + w1 * w1), s) != cudaSuccess)
+      return B2E_ERR_NOMEM;
+    static_sg_weights_kernel<<<1, 2 * B2E_SG_MAX_WIDTH, 0, s>>>(bins, sg_halfwidth, sg_order, sgd_halfwidth, sgd_order,
+                                                                w);
   }
-  static_sg_weights_kernel<<<(2 * bins + 127) / 128, 128, 0, s>>>(bins, sg_halfwidth, sg_order, sgd_halfwidth,
-                                                                  sgd_order, w, idx);
   WakeArgs a = {};
   a.nBins = bins;
   a.sgHalf = sg_halfwidth;
@@ -2747,11 +2815,7 @@ extern "C" int b2e_csr_wake_batch(const double *dev_counts, const double *dev_sl
   a.steady = steady != 0;
   a.correct = sg_halfwidth > 0;
   a.sg_w = w;
-  a.sgd_w = w + (size_t)bins * B2E_SG_MAX_WIDTH;
-  a.sg_lo = idx;
-  a.sg_n = idx + 1;
-  a.sgd_lo = idx + 2 * bins;
-  a.sgd_n = idx + 2 * bins + 1;
+  a.sgd_w = w ? w + w0 * w0 : nullptr;
   a.slippage = 0;
   a.slippage13 = 1;
   a.c1 = 1;
@@ -2761,14 +2825,14 @@ extern "C" int b2e_csr_wake_batch(const double *dev_counts, const double *dev_sl
   a.length = a.nSlices = 1;
   a.igf = 0;
   a.gamma2 = a.gamma3 = a.rho0 = a.const1 = a.q4pe = a.igf_factor = 0;
-  const size_t smem = sizeof(double) * 4 * bins;
+  const size_t smem = sizeof(double) * (5 * bins + 8);
   cudaError_t e = cudaFuncSetAttribute(wake_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess) {
-    wake_batch_kernel<<<n_profiles, 512, smem, s>>>(dev_counts, dev_slippage_bins, a, dev_t1, dev_density,
-                                                    dev_derivative);
+    wake_batch_kernel<<<n_profiles, BATCH_THREADS, smem, s>>>(dev_counts, dev_slippage_bins, a, tables, dev_t1,
+                                                              dev_density, dev_derivative);
     e = cudaGetLastError();
   }
-  cudaFreeAsync(w, s);
-  cudaFreeAsync(idx, s);
+  if (w)
+    cudaFreeAsync(w, s);
   return e == cudaSuccess ? B2E_OK : B2E_ERR_CUDA;
 }

@@ -68,8 +68,7 @@ struct CsrState {
   void *reducer_user = nullptr;
   unsigned long long *d_keys = nullptr; /* [2][n_bunches]: gathered min, max keys */
   double *d_sg = nullptr;         /* weights of all elements, uploaded once */
-  int *d_sg_idx = nullptr;
-  std::vector<size_t> sg_offset;  /* per element: offset into d_sg / d_sg_idx */
+  std::vector<size_t> sg_offset;  /* per element: offset into d_sg */
   double *d_wakelog = nullptr;
   int64_t wakelog_cap = 0;
   /* optional page record of every plain-integral kick, for CSRCSBEND's

@@ -31,6 +31,7 @@
 #define FP_HI_2P4 0x40300000u
 #define FP_HI_2P10 0x40900000u
 #define FP_HI_2P100 0x46300000u
+#define FP_HI_2P700 0x6bb00000u
 
 /* v zero, or 2^-250 <= |v| below the value whose high word is `end`: products
  * and remainders of such values stay clear of the subnormal range */
