@@ -227,7 +227,7 @@ __device__ __forceinline__ bool csr_slice_fast(SlicePart &pio, const DevElem &e,
       p.DP += h * (1 + fp_quot(p.X, c[CB_RHO0], c[CB_INV_RHO0]));
     }
   }
-  const double A = 1 + p.DP;
+  double A = 1 + p.DP;
   r = fp_sqrt_recip((1 + p.XP * p.XP) + p.YP * p.YP, ir);
   bool ok = fp_abs_hi(p.X) < FP_HI_2P100 && fp_plain(p.XP, FP_HI_2) && fp_plain(p.YP, FP_HI_2) &&
             fp_within(A, FP_HI_2M4, FP_HI_2P4) && fp_within(p.beta0, FP_HI_2M10, FP_HI_2);
@@ -236,7 +236,7 @@ __device__ __forceinline__ bool csr_slice_fast(SlicePart &pio, const DevElem &e,
   p.YP = p.YP * f;
   /* a kick adds a zero to QY, which a negative zero would not survive */
   ok = ok && fp_hi(p.YP) != 0x80000000u;
-  ok = bend_slices_fast<false>(p.X, p.XP, p.Y, p.YP, dist, A, 0.0, c, 1, 4, nullptr, e) && ok;
+  ok = bend_slices_fast<TRIP_NONE>(p.X, p.XP, p.Y, p.YP, dist, A, 0.0, c, 1, 4, nullptr, e) && ok;
   const double d = (A * A - p.XP * p.XP) - p.YP * p.YP;
   r = fp_sqrt_recip(d, ir);
   ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10) && fp_plain(dist, FP_HI_2P100);

@@ -89,11 +89,23 @@ __device__ __forceinline__ bool plain_transverse(const Part &p) {
   return fp_plain(p.x, FP_HI_2P100) && fp_plain(p.y, FP_HI_2P100) && fp_plain(p.xp, FP_HI_2) && fp_plain(p.yp, FP_HI_2);
 }
 
-/* ---- KQUAD / KSEXT without K1/J1, steering, fringes or radiation (EF_FAST).
- * The radiation block's round trip always runs (EF_RADBLOCK).
- * Per kick: the round trip of the momenta through 1 + delta, one square root
- * whose reciprocal divides both momenta; per drift one square root. */
-__device__ __forceinline__ bool kmult_fast(Part &pio, const DevElem &e, const DevAperture *ap, const DevGlobals &g) {
+/* p/sqrt(p^2 + 1) */
+__device__ __forceinline__ bool beta_fast(double p, double &beta) {
+  double ir;
+  const double r = fp_sqrt_recip(p * p + 1, ir);
+  beta = fp_quot(p, r, ir);
+  return fp_within(p, FP_HI_2M10, FP_HI_2P100);
+}
+
+/* ---- KQUAD / KSEXT without K1/J1, steering, fringes or quantum excitation
+ * (EF_FAST).  The radiation block's round trip always runs (EF_RADBLOCK).  Per
+ * kick: the round trip of the momenta through 1 + delta, one square root whose
+ * reciprocal divides both momenta; per drift one square root.  SR adds the
+ * classical radiation of each kick (kmult_radiation), with delta changing
+ * inside the trip; rc: the element's DevRad constants. */
+template <bool SR>
+__device__ __forceinline__ bool kmult_fast(Part &pio, const DevElem &e, const DevAperture *ap, const DevGlobals &g,
+                                           const double *rc) {
   const double *c = e.c;
   const int order = (int)c[KM_ORDER], nSlices = (int)c[KM_NSLICES], nSub = (int)c[KM_NSUB];
   const double dx = c[KM_DX], dy = c[KM_DY];
@@ -102,7 +114,7 @@ __device__ __forceinline__ bool kmult_fast(Part &pio, const DevElem &e, const De
     offset_misalign_fast(p, dx, dy, c[KM_DZ]);
   if (e.flags & EF_ENTRANCE_ROTATE)
     rotate_misalign(p, c[KM_COS_TILT], c[KM_SIN_TILT]);
-  const double A = 1 + p.dp, A2 = A * A, inv_A = fp_recip(A);
+  double dp = p.dp, A = 1 + dp, A2 = A * A, inv_A = fp_recip(A);
   bool ok = inside_limits(p, g) && plain_transverse(p) && fp_within(A, FP_HI_2M4, FP_HI_2P4);
   double x = p.x, xp = p.xp, y = p.y, yp = p.yp, s = 0, r, ir, d, qx, qy;
   r = fp_sqrt_recip((1 + xp * xp) + yp * yp, ir);
@@ -134,12 +146,39 @@ __device__ __forceinline__ bool kmult_fast(Part &pio, const DevElem &e, const De
         fy = 0.5 * (x * x);
         fy = fy + -0.5 * (y * y);
       }
-      qx = qx - kick * fy;
-      qy = qy + kick * fx;
-      qx = fp_quot(qx, A, inv_A) * A;
-      qy = fp_quot(qy, A, inv_A) * A;
-      /* the test of the momenta before the round trip differs from this one
-       * by rounding only, so it cannot fail where d is 2^-10 or more */
+      const double kx = kick * fy, ky = kick * fx;
+      qx = qx - kx;
+      qy = qy + ky;
+      if (SR) {
+        /* slopes before the loss, the field squared from the kick over its
+         * share of the slice, the loss, and the momenta scaled to the new
+         * delta (zero kicks only enter squared, whatever their sign) */
+        d = (A2 - qx * qx) - qy * qy;
+        r = fp_sqrt_recip(d, ir);
+        ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10);
+        xp = fp_quot(qx, r, ir);
+        yp = fp_quot(qy, r, ir);
+        const double share = rc[RK_KFRAC0 + step], drift = rc[RK_DRIFT];
+        const double inv_share = fp_recip(share), inv_drift = fp_recip(drift);
+        const double a = fp_quot(fp_quot(kx, share, inv_share), drift, inv_drift);
+        const double b = fp_quot(fp_quot(ky, share, inv_share), drift, inv_drift);
+        const double ds = fp_sqrt((1 + xp * xp) + yp * yp) * (drift * share);
+        qx = fp_quot(qx, A, inv_A);
+        qy = fp_quot(qy, A, inv_A);
+        dp = dp - ((rc[RK_RAD] * A2) * (a * a + b * b)) * ds;
+        A = 1 + dp;
+        A2 = A * A;
+        inv_A = fp_recip(A);
+        ok = ok && fp_within(A, FP_HI_2M4, FP_HI_2P4);
+        qx = qx * A;
+        qy = qy * A;
+      } else {
+        qx = fp_quot(qx, A, inv_A) * A;
+        qy = fp_quot(qy, A, inv_A) * A;
+      }
+      /* without radiation the test of the momenta before the round trip
+       * differs from this one by rounding only, so it cannot fail where d is
+       * 2^-10 or more */
       d = (A2 - qx * qx) - qy * qy;
       r = fp_sqrt_recip(d, ir);
       ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10);
@@ -154,7 +193,17 @@ __device__ __forceinline__ bool kmult_fast(Part &pio, const DevElem &e, const De
   p.xp = xp;
   p.y = y;
   p.yp = yp;
-  p.s = p.s + s;
+  if (SR) {
+    /* path length at the changed velocity (multipole.c:1391-1394) */
+    double beta0, beta1;
+    if (!fp_plain(p.s, FP_HI_2P100) || !beta_fast(g.p_central * (1 + p.dp), beta0) ||
+        !beta_fast(g.p_central * A, beta1))
+      return false;
+    const double both = beta0 + beta1;
+    p.s = beta1 * (fp_quot(p.s, beta0, fp_recip(beta0)) + fp_quot(2 * s, both, fp_recip(both)));
+    p.dp = dp;
+  } else
+    p.s = p.s + s;
   if (!inside_limits(p, g))
     return false;
   if (e.flags & EF_EXIT_MISALIGN) {
@@ -265,20 +314,24 @@ __device__ __forceinline__ void bend_drift_fast(double &X, double &QX, double &Y
   X = rho0 * (ratio - 1) + ratio * X;
 }
 
-/* nSlices slices of the bend (csbend_integrate with neither field terms nor
- * radiation).  QY changes only by rounding, in the round trip through 1 + delta
- * after a kick (ROUND_TRIP), and stays put from the first trip that leaves it
- * alone: the trip depends on nothing else.  So its trips stop there, and f and
- * 1/f are formed again only while it moves. */
-template <bool ROUND_TRIP, int NSUB = 0>
-__device__ __forceinline__ bool bend_slices_fast(double &X, double &QX, double &Y, double &QY, double &dist, double A,
+/* nSlices slices of the bend (csbend_integrate without field terms).  QY changes
+ * only by rounding, in the round trip through 1 + delta after a kick (TRIP), and
+ * stays put from the first trip that leaves it alone: the trip depends on
+ * nothing else.  So its trips stop there, and f and 1/f are formed again only
+ * while it moves.  With radiation (TRIP_SR; rad_coef in rad, 1/rho0 as the
+ * radiation's formulas take it in inv_rho) delta changes inside every trip, and
+ * A, 1/A and f with it. */
+enum BendTrip { TRIP_NONE, TRIP, TRIP_SR };
+template <BendTrip MODE, int NSUB = 0>
+__device__ __forceinline__ bool bend_slices_fast(double &X, double &QX, double &Y, double &QY, double &dist, double &A,
                                                  double inv_A, const double *c, int nSlices, int nSub_rt,
-                                                 const DevAperture *ap, const DevElem &e) {
+                                                 const DevAperture *ap, const DevElem &e, double *delta = nullptr,
+                                                 double rad = 0, double inv_rho = 0) {
   const double rho0 = c[CB_RHO0];
   const int nSub = NSUB > 0 ? NSUB : nSub_rt;
-  double f, inv_f;
+  double f, inv_f, DP = MODE == TRIP_SR ? *delta : 0;
   unsigned sin_max = 0;
-  bool ok = bend_root(A, QY, f, inv_f), moves = ROUND_TRIP;
+  bool ok = bend_root(A, QY, f, inv_f), moves = MODE == TRIP;
   dist = 0;
   for (int i = 0; i < nSlices && ok; i++) {
     if (ap)
@@ -288,9 +341,9 @@ __device__ __forceinline__ bool bend_slices_fast(double &X, double &QX, double &
       bend_drift_fast(X, QX, Y, QY, dist, A, f, inv_f, rho0, c[CB_DSH0 + j], sin_max);
       if (j == nSub - 1)
         break;
-      const double t = (-c[CB_DS0 + j]) * (1 + fp_quot(X, rho0, c[CB_INV_RHO0]));
+      const double ds = c[CB_DS0 + j], t = (-ds) * (1 + fp_quot(X, rho0, c[CB_INV_RHO0]));
       QX = QX + fp_quot(t, c[CB_RHO_ACTUAL], c[CB_INV_RHO_ACTUAL]);
-      if (ROUND_TRIP) {
+      if (MODE == TRIP) {
         QX = fp_quot(QX, A, inv_A) * A;
         if (moves) {
           const double q = fp_quot(QY, A, inv_A) * A;
@@ -300,9 +353,26 @@ __device__ __forceinline__ bool bend_slices_fast(double &X, double &QX, double &
             ok = bend_root(A, QY, f, inv_f) && ok;
           }
         }
+      } else if (MODE == TRIP_SR) {
+        /* radiation after the kick (csbend.c:1603-1622) in the dipole field, F2 = 1 */
+        const double a = 1 + X * inv_rho, A2 = A * A, d = (A2 - QX * QX) - QY * QY;
+        double ir;
+        const double r = fp_sqrt_recip(d, ir), g = fp_quot(a, r, ir);
+        const double xp = QX * g, yp = QY * g, m = (a * a + xp * xp) + yp * yp;
+        ok = ok && fp_within(d, FP_HI_2M10, FP_HI_2P10) && fp_within(m, FP_HI_2M10, FP_HI_2P10);
+        QX = fp_quot(QX, A, inv_A);
+        QY = fp_quot(QY, A, inv_A);
+        DP = DP - ((rad * A2) * ds) * fp_sqrt(m);
+        A = 1 + DP;
+        inv_A = fp_recip(A);
+        QX = QX * A;
+        QY = QY * A;
+        ok = bend_root(A, QY, f, inv_f) && ok && fp_within(A, FP_HI_2M4, FP_HI_2P4);
       }
     }
   }
+  if (MODE == TRIP_SR)
+    *delta = DP;
   return ok && sin_max < FP_HI_2M3 && (!ap || ap_inside(X, Y, ap, e));
 }
 
@@ -321,13 +391,16 @@ static __device__ __noinline__ EdgeSlopes bend_edge_o1(double xp, double yp, dou
 }
 
 /* ---- CSBEND without field terms, ETILT, second-order or simple edges and
- * radiation (EF_FAST) */
-__device__ __forceinline__ bool csbend_fast(Part &pio, const DevElem &e, const DevAperture *ap, const DevGlobals &g) {
+ * quantum excitation (EF_FAST); with SR, classical radiation in the body and
+ * none at the edges, whose angles are zero; rc: the element's DevRad constants */
+template <bool SR>
+__device__ __forceinline__ bool csbend_fast(Part &pio, const DevElem &e, const DevAperture *ap, const DevGlobals &g,
+                                            const double *rc) {
   const double *c = e.c;
   const double ct = c[CB_COS_TT], st = c[CB_SIN_TT];
   Part p = pio;
-  double x, y, xp, yp, s, Q4, r, ir, f;
-  const double A = 1 + p.dp, inv_A = fp_recip(A);
+  double x, y, xp, yp, s, Q4, r, ir, f, A = 1 + p.dp;
+  const double inv_A = fp_recip(A);
   bool ok = plain_transverse(p) && fp_plain(p.s, FP_HI_2P100) && fp_within(A, FP_HI_2M4, FP_HI_2P4);
   s = p.s + c[CB_DZI] * (c[CB_DZI] == 0 ? 1.0 : fp_sqrt((1 + p.xp * p.xp) + p.yp * p.yp));
   p.x = (p.x + c[CB_DXI]) + c[CB_DZI] * p.xp;
@@ -357,7 +430,10 @@ __device__ __forceinline__ bool csbend_fast(Part &pio, const DevElem &e, const D
   ok = ok && fp_hi(yp) != 0x80000000u;
   if (!ok)
     return false;
-  if (!bend_slices_fast<true>(x, xp, y, yp, Q4, A, inv_A, c, (int)c[CB_NSLICES], (int)c[CB_NSUB], ap, e))
+  double dp = p.dp;
+  if (!(SR ? bend_slices_fast<TRIP_SR>(x, xp, y, yp, Q4, A, inv_A, c, (int)c[CB_NSLICES], (int)c[CB_NSUB], ap, e, &dp,
+                                       rc[RB_RAD], rc[RB_INV_RHO0])
+           : bend_slices_fast<TRIP>(x, xp, y, yp, Q4, A, inv_A, c, (int)c[CB_NSLICES], (int)c[CB_NSUB], ap, e)))
     return false;
   {
     const double d = (A * A - xp * xp) - yp * yp;
@@ -368,10 +444,14 @@ __device__ __forceinline__ bool csbend_fast(Part &pio, const DevElem &e, const D
   xp = xp * f;
   yp = yp * f;
   {
-    /* the velocity is the entrance's: beta s / beta rounds twice */
-    const double p0 = g.p_central * A, rb = fp_sqrt_recip(p0 * p0 + 1, ir), beta = fp_quot(p0, rb, ir);
-    ok = ok && fp_within(p0, FP_HI_2M10, FP_HI_2P100);
-    s = fp_quot(beta * s, beta, fp_recip(beta)) + Q4;
+    /* time-of-flight velocity fix (csbend.c:1278-1288); without radiation the
+     * exit velocity is the entrance's, and beta s / beta rounds twice */
+    double beta0, beta1;
+    ok = beta_fast(g.p_central * (1 + p.dp), beta0) && ok;
+    beta1 = beta0;
+    if (SR)
+      ok = beta_fast(g.p_central * A, beta1) && ok;
+    s = fp_quot(beta1 * s, beta0, fp_recip(beta0)) + Q4;
   }
   if (e.flags & EF_EDGE2) {
     if (e.flags & EF_EDGE2_FLAT) {
@@ -379,7 +459,7 @@ __device__ __forceinline__ bool csbend_fast(Part &pio, const DevElem &e, const D
       xp = xp + z * x;
       yp = yp - z * y;
     } else {
-      const EdgeSlopes es = bend_edge_o1(xp, yp, x, y, p.dp, c[CB_RHO_ACTUAL], c + CB_TAN_E2);
+      const EdgeSlopes es = bend_edge_o1(xp, yp, x, y, dp, c[CB_RHO_ACTUAL], c + CB_TAN_E2);
       xp = es.xp;
       yp = es.yp;
     }
@@ -389,6 +469,7 @@ __device__ __forceinline__ bool csbend_fast(Part &pio, const DevElem &e, const D
   p.xp = (xp * ct - yp * st) + 0.0;
   p.yp = (xp * st + yp * ct) + 0.0;
   p.s = s + 0.0;
+  p.dp = dp;
   ok = ok && fp_abs_hi(p.xp) < FP_HI_2 && fp_abs_hi(p.yp) < FP_HI_2;
   p.x = p.x + (c[CB_DXF] + c[CB_DZF] * p.xp);
   p.y = p.y + (c[CB_DYF] + c[CB_DZF] * p.yp);

@@ -460,17 +460,25 @@ static void etilt_exit_offsets(double out[5], double rho0, double angle, double 
  * are written for, and its constants are zero or far from overflow and
  * underflow in products with coordinates.  A CSRCSBEND's edges and exit
  * offsets are the CSR entry and exit kernels' business. */
-static void mark_fast(DevElem &d) {
+static void mark_fast(DevElem &d, const DevRad &r) {
   auto plain = [](double v) { return v == 0 || (fabs(v) >= 0x1p-60 && fabs(v) <= 0x1p60); };
   bool ok = true;
   if (d.kind == K_KMULT) {
-    ok = (d.flags & EF_RADBLOCK) && !(d.flags & (EF_QUAD_ORDER2 | EF_SKEW_ORDER2 | EF_SR | EF_ISR | EF_STEERING | EF_QFRINGE1 | EF_QFRINGE2 |
+    ok = (d.flags & EF_RADBLOCK) && !(d.flags & (EF_QUAD_ORDER2 | EF_SKEW_ORDER2 | EF_ISR | EF_STEERING | EF_QFRINGE1 | EF_QFRINGE2 |
                       EF_END_DRIFT));
     for (int j = 0; j < 8; j++)
       ok = ok && plain(d.c[KM_DSH0 + j]) && plain(d.c[KM_KICK0 + j]);
     ok = ok && plain(d.c[KM_DX]) && plain(d.c[KM_DY]) && plain(d.c[KM_DZ]);
+    if (d.flags & EF_SR) {
+      ok = ok && r.c[RK_DRIFT] > 0 && plain(r.c[RK_DRIFT]) && r.c[RK_XKICK] == 0 && r.c[RK_YKICK] == 0;
+      for (int j = 0; j < (int)d.c[KM_NSUB] - 1; j++)
+        ok = ok && r.c[RK_KFRAC0 + j] != 0 && plain(r.c[RK_KFRAC0 + j]);
+    }
   } else if (d.kind == K_CSBEND || d.kind == K_CSRCSBEND) {
-    ok = !(d.flags & (EF_SR | EF_ISR | EF_FIELD | EF_SKEW_KICK | EF_EDGE1_SIMPLE | EF_EDGE2_SIMPLE));
+    ok = !(d.flags & (EF_ISR | EF_FIELD | EF_SKEW_KICK | EF_EDGE1_SIMPLE | EF_EDGE2_SIMPLE));
+    /* radiation at an edge goes with its angle (csbend.c:1211, :1265) */
+    if (d.flags & EF_SR)
+      ok = ok && (!(d.flags & EF_EDGE1) || d.c[CB_E1] == 0) && (!(d.flags & EF_EDGE2) || d.c[CB_E2] == 0);
     if (d.kind == K_CSBEND)
       ok = ok && (d.flags & EF_RADBLOCK) && !(d.flags & (EF_EDGE_ORDER2 | EF_ETILT));
     /* a drift angle of 0.6 after one of asin(1/8) stays below pi/4 */
@@ -744,7 +752,7 @@ const char *compile_single_csr_bend(const b2e_element &el, DevElem &d, BendExtra
   memcpy(bx.c, rad.c + RB_EXTRA0, sizeof(bx.c));
   if (d.kind != K_CSRCSBEND)
     return "CSRCSBEND with zero angle is a drift; nothing to do here";
-  mark_fast(d);
+  mark_fast(d, rad);
   d.z_end = el.p[B2E_BEND_L];
   return nullptr;
 }
@@ -913,7 +921,7 @@ std::string compile_lattice(const b2e_element *el, int n, const b2e_run_options 
     if (!err.empty())
       return std::string("element ") + std::to_string(i) + " (" + std::string(el[i].name, strnlen(el[i].name, 32)) +
              "): " + err;
-    mark_fast(d);
+    mark_fast(d, out.rads[i]);
     d.ap_pass0 = last_ap;
     d.z_end = z;
   }

@@ -177,7 +177,8 @@ __global__ void __launch_bounds__(128 * TPB, MINB) ring_kernel(RingLaunch L) {
           rs.elem = ie;
           rs.rc = rads[ie].c;
         }
-        if (!((e.flags & EF_FAST) && kmult_fast(p, e, ap, L.g)))
+        if (!((e.flags & EF_FAST) && (RAD && (e.flags & EF_SR) ? kmult_fast<true>(p, e, ap, L.g, rs.rc)
+                                                               : kmult_fast<false>(p, e, ap, L.g, nullptr))))
           lost = kmult_general<RAD>(p, e, ap, L.g, rs);
         break;
       case K_CSBEND:
@@ -186,7 +187,8 @@ __global__ void __launch_bounds__(128 * TPB, MINB) ring_kernel(RingLaunch L) {
           rs.elem = ie;
           rs.rc = rads[ie].c;
         }
-        if (!((e.flags & EF_FAST) && csbend_fast(p, e, ap, L.g)))
+        if (!((e.flags & EF_FAST) && (RAD && (e.flags & EF_SR) ? csbend_fast<true>(p, e, ap, L.g, rs.rc)
+                                                               : csbend_fast<false>(p, e, ap, L.g, nullptr))))
           lost = csbend_general<RAD>(p, e, ap, L.g, rs);
         break;
       case K_MALIGN: {
