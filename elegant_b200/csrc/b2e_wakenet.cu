@@ -332,10 +332,15 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
  * and the dZ box as an MN-major B operand (N = co), K = the 128 bins in
  * steps of 16, accumulating three 128x64 FP32 tiles in TMEM over all tiles
  * of the block.  The epilogue writes the block's partial sums
- * [5][64 ci][64 co]. */
+ * [5][64 ci][64 co].
+ *
+ * The fifth tap's partner in the third pair is a constant block whose channel
+ * 0 is one in every bin: its accumulator row is the sum of dZ over the bins, the
+ * bias gradient.  The tensor cores form it beside products they do anyway; a
+ * kernel of its own read dZ again, 19 us per layer at 256 profiles. */
 constexpr int WG_STAGES = 2;
 constexpr size_t WG_STAGE_BYTES = 6 * CONV_STAGE_BYTES; /* 96 KB */
-constexpr size_t WG_SMEM = 1024 + WG_STAGES * WG_STAGE_BYTES;
+constexpr size_t WG_SMEM = 1024 + WG_STAGES * WG_STAGE_BYTES + CONV_STAGE_BYTES;
 
 __global__ void __launch_bounds__(WG_THREADS, 1)
     wgrad_kernel(const __grid_constant__ CUtensorMap t_in, const __grid_constant__ CUtensorMap t_dz, WgradArgs a) {
@@ -355,6 +360,14 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     mbar_init(&done, 1);
     fence_barrier_init();
   }
+  unsigned char *ones = sm + WG_STAGES * WG_STAGE_BYTES;
+  for (int k = threadIdx.x; k < (int)(CONV_STAGE_BYTES / 16); k += WG_THREADS) {
+    /* 16-byte chunk k & 7 of bin k >> 3; the 128-byte swizzle puts channels 0-7
+     * of a bin in chunk (bin & 7) */
+    const int bin = k >> 3;
+    reinterpret_cast<uint4 *>(ones)[k] = make_uint4((k & 7) == (bin & 7) ? 0x3f80u : 0u, 0u, 0u, 0u);
+  }
+  fence_proxy_async(); /* the MMA reads it through the async proxy */
   if (warp == 0) {
     tmem_alloc(&tmem_base, 256);
     tmem_relinquish();
@@ -398,9 +411,12 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
         const uint32_t st = smem_u32(sm + s * WG_STAGE_BYTES);
         const uint32_t bz = st + 5 * (uint32_t)CONV_STAGE_BYTES;
         for (int p = 0; p < 3; p++) {
+          /* the two 64-channel blocks of A: taps 2p and 2p + 1, the last tap and
+           * the ones */
           const uint32_t ax = st + 2 * p * (uint32_t)CONV_STAGE_BYTES;
+          const uint32_t step = p < 2 ? (uint32_t)CONV_STAGE_BYTES : smem_u32(ones) - ax;
           for (int k = 0; k < 8; k++)
-            mma_bf16(tmem + 64 * p, sw128_desc(ax + 2048 * k, (uint32_t)CONV_STAGE_BYTES, 1024),
+            mma_bf16(tmem + 64 * p, sw128_desc(ax + 2048 * k, step, 1024),
                      sw128_desc(bz + 2048 * k, (uint32_t)CONV_STAGE_BYTES, 1024), IDESC, it > 0 || k > 0);
         }
         mma_commit(&empty[s]);
@@ -432,6 +448,11 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
       }
       if (t < WN_TAPS) {
         float4 *o = reinterpret_cast<float4 *>(a.partial + (((size_t)blockIdx.x * WN_TAPS + t) * 64 + ci) * 64);
+#pragma unroll
+        for (int c = 0; c < 64; c += 4)
+          o[c / 4] = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+      } else if (ci == 0) {
+        float4 *o = reinterpret_cast<float4 *>(a.bias_partial + (size_t)blockIdx.x * 64);
 #pragma unroll
         for (int c = 0; c < 64; c += 4)
           o[c / 4] = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
@@ -526,20 +547,20 @@ extern "C" int b2e_umma_selftest(int mode, const void *dev_a, const void *dev_b,
 /* ======================================================== network context */
 namespace b2e {
 
-/* inputs [n][WN_IN][L] FP32 -> X0 [n][L][64] BF16 (channels WN_IN..63 zero) */
+/* inputs [n][WN_IN][L] FP32 -> channels 0-7 of X0 [n][L][64] BF16; channels
+ * 8-63 hold the zeros they were created with */
 __global__ void wn_pack_kernel(const float *in, int L, int64_t rows, __nv_bfloat16 *x0) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r >= rows)
     return;
   const int64_t p = r / L, i = r - p * L;
   const float *src = in + p * WN_IN * L + i;
-  uint4 *dst = reinterpret_cast<uint4 *>(x0 + r * 64);
-  dst[0] = make_uint4(pack_bf16(src[0], src[L]), pack_bf16(src[2 * L], src[3 * L]), 0u, 0u);
-  for (int c = 1; c < 8; c++)
-    dst[c] = make_uint4(0u, 0u, 0u, 0u);
+  *reinterpret_cast<uint4 *>(x0 + r * 64) =
+    make_uint4(pack_bf16(src[0], src[L]), pack_bf16(src[2 * L], src[3 * L]), 0u, 0u);
 }
 
-/* residual y - target into channel 0 of dZ6; per-block sums of squares */
+/* residual y - target into channel 0 of dZ6 (channels 8-63 hold the zeros they
+ * were created with); per-block sums of squares */
 __global__ void wn_loss_kernel(const float *y, const float *target, int64_t rows, __nv_bfloat16 *dz6, double *partial) {
   __shared__ double red[256];
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -547,10 +568,7 @@ __global__ void wn_loss_kernel(const float *y, const float *target, int64_t rows
   if (r < rows) {
     const float d = y[r] - target[r];
     sq = (double)d * d;
-    uint4 *dst = reinterpret_cast<uint4 *>(dz6 + r * 64);
-    dst[0] = make_uint4(pack_bf16(d, 0.f), 0u, 0u, 0u);
-    for (int c = 1; c < 8; c++)
-      dst[c] = make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4 *>(dz6 + r * 64) = make_uint4(pack_bf16(d, 0.f), 0u, 0u, 0u);
   }
   red[threadIdx.x] = sq;
   __syncthreads();
@@ -563,48 +581,34 @@ __global__ void wn_loss_kernel(const float *y, const float *target, int64_t rows
     partial[blockIdx.x] = red[0];
 }
 
-/* per-block channel sums of dZ [rows][64]: thread (chunk of 8 channels, row lane) */
-__global__ void wn_bias_grad_kernel(const __nv_bfloat16 *dz, int64_t rows, float *partial) {
-  __shared__ float red[32][65];
-  const int chunk = threadIdx.x & 7, lane = threadIdx.x >> 3; /* 8 x 32 */
-  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int64_t r = blockIdx.x * 32 + lane; r < rows; r += (int64_t)gridDim.x * 32) {
-    uint4 v = reinterpret_cast<const uint4 *>(dz + r * 64)[chunk];
-    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&v);
-    for (int i = 0; i < 4; i++) {
-      float2 f = __bfloat1622float2(h[i]);
-      acc[2 * i] += f.x;
-      acc[2 * i + 1] += f.y;
-    }
-  }
-  for (int i = 0; i < 8; i++)
-    red[lane][chunk * 8 + i] = acc[i];
+/* grad[t][co][ci] = scale * sum_block wpart[block][t][ci][co]; grad_b[co]
+ * likewise from bpart.  A block takes 64 consecutive sums, four threads each
+ * (blocks b, b + 4, ... of the partials, then the four in order): four times the
+ * loads in flight of one thread per sum. */
+constexpr int REDUCE_SPLIT = 4;
+__global__ void __launch_bounds__(64 * REDUCE_SPLIT)
+    wn_reduce_kernel(const float *wpart, int n_wblocks, const float *bpart, float scale, float *grad_w,
+                     float *grad_b) {
+  __shared__ float part[REDUCE_SPLIT][64];
+  const int c = threadIdx.x & 63, g = threadIdx.x >> 6;
+  const int idx = blockIdx.x * 64 + c; /* (t, ci, co), then the 64 biases */
+  const bool weights = idx < WN_WSIZE;
+  const float *src = weights ? wpart + idx : bpart + c;
+  const size_t stride = weights ? WN_WSIZE : 64;
+  float s = 0;
+#pragma unroll 8
+  for (int b = g; b < n_wblocks; b += REDUCE_SPLIT)
+    s += src[b * stride];
+  part[g][c] = s;
   __syncthreads();
-  if (threadIdx.x < 64) {
-    float s = 0;
-    for (int l = 0; l < 32; l++)
-      s += red[l][threadIdx.x];
-    partial[blockIdx.x * 64 + threadIdx.x] = s;
-  }
-}
-
-/* grad[t][co][ci] = scale * sum_block wpart[block][t][ci][co]; grad_b[co] likewise */
-__global__ void wn_reduce_kernel(const float *wpart, int n_wblocks, const float *bpart, int n_bblocks, float scale,
-                                 float *grad_w, float *grad_b) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx < WN_WSIZE) {
-    const int co = idx & 63, ci = (idx >> 6) & 63, t = idx >> 12; /* idx = (t, ci, co) */
-    float s = 0;
-    for (int b = 0; b < n_wblocks; b++)
-      s += wpart[(size_t)b * WN_WSIZE + idx];
+  if (g)
+    return;
+  s = ((part[0][c] + part[1][c]) + part[2][c]) + part[3][c];
+  if (weights) {
+    const int co = idx & 63, ci = (idx >> 6) & 63, t = idx >> 12;
     grad_w[(t * 64 + co) * 64 + ci] = s * scale;
-  } else if (idx < WN_WSIZE + 64) {
-    const int co = idx - WN_WSIZE;
-    float s = 0;
-    for (int b = 0; b < n_bblocks; b++)
-      s += bpart[b * 64 + co];
-    grad_b[co] = s * scale;
-  }
+  } else
+    grad_b[c] = s * scale;
 }
 
 /* Adam (Kingma & Ba 2015) on the flat FP32 parameters, then the BF16 weight
@@ -644,7 +648,7 @@ struct b2e_wakenet {
   double *lpart = nullptr;
   unsigned int *status = nullptr;
   CUtensorMap t_x0, t_act[WN_LAYERS], t_dz[WN_LAYERS], t_wk[WN_LAYERS], t_wt[WN_LAYERS];
-  int conv_grid_max = 296, wgrad_grid_max = 148, bias_blocks = 148;
+  int conv_grid_max = 296, wgrad_grid_max = 148;
   std::string err;
 };
 
@@ -716,13 +720,11 @@ int backward(b2e_wakenet *n, const float *targets, int n_prof, double *loss, cud
     w.n_prof = n_prof;
     w.dilation = n->dil[l];
     w.partial = n->wpart;
+    w.bias_partial = n->bpart;
     w.status = n->status;
     WN_TRY(n, launch_wgrad(l == 0 ? n->t_x0 : n->t_act[l - 1], n->t_dz[l], w, wgrid, s));
-    wn_bias_grad_kernel<<<n->bias_blocks, 256, 0, s>>>(n->dz[l], rows, n->bpart);
-    WN_TRY(n, cudaGetLastError());
-    wn_reduce_kernel<<<(WN_WSIZE + 64 + 255) / 256, 256, 0, s>>>(
-        n->wpart, wgrid, n->bpart, n->bias_blocks, scale, n->grads + l * WN_WSIZE,
-        n->grads + WN_LAYERS * WN_WSIZE + l * WN_CH);
+    wn_reduce_kernel<<<WN_WSIZE / 64 + 1, 64 * REDUCE_SPLIT, 0, s>>>(
+        n->wpart, wgrid, n->bpart, scale, n->grads + l * WN_WSIZE, n->grads + WN_LAYERS * WN_WSIZE + l * WN_CH);
     WN_TRY(n, cudaGetLastError());
     if (l > 0) {
       ConvArgs a{};
@@ -818,7 +820,7 @@ extern "C" int b2e_wakenet_create(b2e_wakenet **out, int32_t bins, int32_t max_b
   }
   ok(dalloc(&n->y, (size_t)max_batch * bins));
   ok(dalloc(&n->wpart, (size_t)n->wgrad_grid_max * WN_WSIZE));
-  ok(dalloc(&n->bpart, (size_t)n->bias_blocks * 64));
+  ok(dalloc(&n->bpart, (size_t)n->wgrad_grid_max * 64));
   ok(dalloc(&n->lpart, (size_t)((int64_t)max_batch * bins + 255) / 256));
   ok(dalloc(&n->status, 1));
   if (e == cudaSuccess) {
@@ -827,6 +829,9 @@ extern "C" int b2e_wakenet_create(b2e_wakenet **out, int32_t bins, int32_t max_b
     ok(cudaMemset(n->adam_m, 0, sizeof(float) * WN_NPARAM));
     ok(cudaMemset(n->adam_v, 0, sizeof(float) * WN_NPARAM));
     ok(cudaMemset(n->status, 0, sizeof(unsigned int)));
+    /* the dead channels of the network's input and of the output's gradient */
+    ok(cudaMemset(n->x0, 0, sizeof(__nv_bfloat16) * act));
+    ok(cudaMemset(n->dz[WN_LAYERS - 1], 0, sizeof(__nv_bfloat16) * act));
   }
   if (e == cudaSuccess) {
     ok(make_tmap_rows64(&n->t_x0, n->x0, bins, max_batch, 128));

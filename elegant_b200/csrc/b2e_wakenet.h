@@ -37,7 +37,8 @@ struct ConvArgs {
 
 struct WgradArgs {
   int L, n_prof, dilation;
-  float *partial; /* [gridDim.x][5][64 ci][64 co] */
+  float *partial;      /* [gridDim.x][5][64 ci][64 co] */
+  float *bias_partial; /* [gridDim.x][64 co] */
   unsigned int *status;
 };
 
