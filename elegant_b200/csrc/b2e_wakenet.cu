@@ -129,16 +129,19 @@ __global__ void __launch_bounds__(128, 1)
  *            shifted 128x64 activation boxes through a WN_STAGES-deep ring;
  *   warp 1   one thread issues UMMA 128x64x16 (4 per tap, 20 per tile) into
  *            one of two TMEM accumulators and commits to free the stage;
- *   warps 2-9 epilogue: TMEM -> registers (warp w reads lanes 32*(w%4)..;
- *            warps 2-5 take channels 0-31, warps 6-9 channels 32-63),
+ *   warps 2-17 epilogue: TMEM -> registers (warp w reads lanes 32*(w%4)..;
+ *            four warps per lane quadrant, 16 of the 64 channels each),
  *            bias + GELU (hidden), output channel 0 (output), or times
- *            GELU'(z) of the previous layer (backward data), BF16 stores.
- *            The erf/exp of GELU and GELU' bound the epilogue, hence two
- *            warps per lane quadrant; launch bounds of two CTAs per SM
- *            (96 registers, no spills) keep 16 epilogue warps per SM.
+ *            GELU'(z) of the previous layer (backward data), BF16.
+ *            The erf/exp of GELU and GELU' bound the epilogue: with 32
+ *            channels per warp, 16 epilogue warps per SM, the issue slots were
+ *            48 % busy; 16 channels need few enough registers (56) for 32
+ *            warps.  A thread's 16 channels are one 32-byte sector, moved by
+ *            one 256-bit access; in 16-byte pieces each sector was written
+ *            twice.
  * Bounded waits everywhere; a timeout sets the status word and every role
  * leaves its loop. */
-constexpr int CONV_EPI_WARPS = 8;
+constexpr int CONV_EPI_WARPS = 16;
 constexpr int CONV_THREADS = 64 + 32 * CONV_EPI_WARPS;
 constexpr int WG_THREADS = 192;
 constexpr size_t CONV_W_BYTES = (size_t)WN_TAPS * 64 * 128;  /* 40 KB */
@@ -153,6 +156,24 @@ __device__ __forceinline__ float gelu_grad_f(float z) {
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t *>(&h);
+}
+
+/* 16 BF16 values of one row, a 32-byte sector */
+struct Row16 {
+  uint32_t w[8];
+};
+__device__ __forceinline__ void store_row16(__nv_bfloat16 *p, const Row16 &r) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r.w[0]), "r"(r.w[1]),
+               "r"(r.w[2]), "r"(r.w[3]), "r"(r.w[4]), "r"(r.w[5]), "r"(r.w[6]), "r"(r.w[7])
+               : "memory");
+}
+__device__ __forceinline__ Row16 load_row16(const __nv_bfloat16 *p) {
+  Row16 r;
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]), "=r"(r.w[6]),
+                 "=r"(r.w[7])
+               : "l"(p));
+  return r;
 }
 
 template <int EPI>
@@ -252,23 +273,24 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
     }
   } else {
     const int q = warp & 3;               /* the TMEM lane quadrant this warp may read */
-    const int half = (warp - 2) >> 2;     /* channels [32 half, 32 half + 32) */
-    constexpr int NC = N == 64 ? 32 : N;  /* channels per thread */
-    const int c0 = N == 64 ? 32 * half : 0;
-    const bool works = N == 64 || half == 0; /* the output layer's channel 0: one warp per quadrant */
+    const int part = (warp - 2) >> 2;     /* channels [16 part, 16 part + 16) */
+    const int c0 = 16 * part;
+    const bool works = N == 64 || part == 0; /* the output layer's channel 0: one warp per quadrant */
     const int r = q * 32 + lane;           /* row of the tile this thread owns */
     uint32_t j = 0;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, j++) {
       const uint32_t acc = j & 1;
+      const int b = tile / tpp, l0 = (tile - b * tpp) << 7;
+      const size_t row = (size_t)b * a.L + l0 + r;
+      Row16 zz;
+      if (EPI == EPI_BWD) /* arrives while the accumulator fills */
+        zz = load_row16(a.z_prev + row * 64 + c0);
       if (!mbar_wait(&tfull[acc], (j >> 1) & 1, a.status, ST_TIMEOUT_EPI))
         break;
       tc_fence_after();
-      float v[NC];
+      float v[16];
       if (works) {
-        const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + acc * 64 + c0;
-#pragma unroll
-        for (int c = 0; c < NC; c += 16)
-          tmem_ld16(base + c, v + c);
+        tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + acc * 64 + c0, v);
         tmem_wait_ld();
       }
       tc_fence_before();
@@ -277,42 +299,27 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
         mbar_arrive(&tempty[acc]);
       if (!works)
         continue;
-      const int b = tile / tpp, l0 = (tile - b * tpp) << 7;
-      const size_t row = (size_t)b * a.L + l0 + r;
       if (EPI == EPI_OUTPUT) {
         a.y_out[row] = v[0] + sbias[0];
       } else if (EPI == EPI_HIDDEN) {
-        uint4 *zo = a.z_out ? reinterpret_cast<uint4 *>(a.z_out + row * 64 + c0) : nullptr;
-        uint4 *ao = reinterpret_cast<uint4 *>(a.a_out + row * 64 + c0);
+        Row16 zo, ao;
 #pragma unroll
-        for (int c = 0; c < NC; c += 8) {
-          float z[8];
-#pragma unroll
-          for (int i = 0; i < 8; i++)
-            z[i] = v[c + i] + sbias[c0 + c + i];
-          if (zo)
-            zo[c / 8] = make_uint4(pack_bf16(z[0], z[1]), pack_bf16(z[2], z[3]), pack_bf16(z[4], z[5]),
-                                   pack_bf16(z[6], z[7]));
-          ao[c / 8] = make_uint4(pack_bf16(gelu_f(z[0]), gelu_f(z[1])), pack_bf16(gelu_f(z[2]), gelu_f(z[3])),
-                                 pack_bf16(gelu_f(z[4]), gelu_f(z[5])), pack_bf16(gelu_f(z[6]), gelu_f(z[7])));
+        for (int i = 0; i < 8; i++) {
+          const float z0 = v[2 * i] + sbias[c0 + 2 * i], z1 = v[2 * i + 1] + sbias[c0 + 2 * i + 1];
+          zo.w[i] = pack_bf16(z0, z1);
+          ao.w[i] = pack_bf16(gelu_f(z0), gelu_f(z1));
         }
+        if (a.z_out)
+          store_row16(a.z_out + row * 64 + c0, zo);
+        store_row16(a.a_out + row * 64 + c0, ao);
       } else {
-        const uint4 *zp = reinterpret_cast<const uint4 *>(a.z_prev + row * 64 + c0);
-        uint4 *go = reinterpret_cast<uint4 *>(a.a_out + row * 64 + c0);
+        Row16 go;
 #pragma unroll
-        for (int c = 0; c < NC; c += 8) {
-          uint4 zz = zp[c / 8];
-          const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&zz);
-          float g[8];
-#pragma unroll
-          for (int i = 0; i < 4; i++) {
-            float2 f = __bfloat1622float2(h[i]);
-            g[2 * i] = v[c + 2 * i] * gelu_grad_f(f.x);
-            g[2 * i + 1] = v[c + 2 * i + 1] * gelu_grad_f(f.y);
-          }
-          go[c / 8] = make_uint4(pack_bf16(g[0], g[1]), pack_bf16(g[2], g[3]), pack_bf16(g[4], g[5]),
-                                 pack_bf16(g[6], g[7]));
+        for (int i = 0; i < 8; i++) {
+          const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&zz.w[i]));
+          go.w[i] = pack_bf16(v[2 * i] * gelu_grad_f(f.x), v[2 * i + 1] * gelu_grad_f(f.y));
         }
+        store_row16(a.a_out + row * 64 + c0, go);
       }
     }
   }
