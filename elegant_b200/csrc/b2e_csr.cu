@@ -127,9 +127,11 @@ __device__ __forceinline__ double csr_kick(double CT, double X, double DP, const
  * CTAs have started), then waits until the predecessor grid has completed
  * and its memory is visible, before touching any memory.  In a kernel
  * launched without the attribute both instructions return at once. */
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_enter() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  chain_release();
+  chain_wait();
 }
 
 /* entrance: offsets, tilt, c*t = s/beta, entrance edge (csbend.c:2286-2377) */
@@ -210,15 +212,15 @@ static __device__ __noinline__ int csr_slice_general(SlicePart *p, const DevElem
 
 static __device__ __noinline__ double divide_ieee(double a, double b) { return a / b; }
 
-/* The same in the straight-line form of b2e_fast.cuh (four substeps); leaves
- * the particle alone and returns false where that does not apply. */
-__device__ __forceinline__ bool csr_slice_fast(SlicePart &pio, const DevElem &e, const SliceWake &w, double inv_dct,
-                                               double Po, double inv_Po) {
-  SlicePart p = pio;
+/* The same in the straight-line form of b2e_fast.cuh (four substeps).  Returns
+ * false where that does not apply; the caller then reads the particle again.
+ * ct0 and beta0 are read where they are used, from shared memory. */
+__device__ __forceinline__ bool csr_slice_fast(SlicePart &p, const DevElem &e, const SliceWake &w, const double *ct0,
+                                               const double *beta0, double Po, double inv_Po) {
   const double *c = e.c;
   double r, ir, f, dist;
   if (w.apply) {
-    f = fp_quot(p.CT - w.lower, w.dct, inv_dct);
+    f = fp_quot(*ct0 - w.lower, w.dct, fp_recip(w.dct));
     const long long iBin = (long long)f;
     f -= iBin;
     if (iBin >= 0 && iBin < w.nBins - 1) {
@@ -230,7 +232,7 @@ __device__ __forceinline__ bool csr_slice_fast(SlicePart &pio, const DevElem &e,
   double A = 1 + p.DP;
   r = fp_sqrt_recip((1 + p.XP * p.XP) + p.YP * p.YP, ir);
   bool ok = fp_abs_hi(p.X) < FP_HI_2P100 && fp_plain(p.XP, FP_HI_2) && fp_plain(p.YP, FP_HI_2) &&
-            fp_within(A, FP_HI_2M4, FP_HI_2P4) && fp_within(p.beta0, FP_HI_2M10, FP_HI_2);
+            fp_within(A, FP_HI_2M4, FP_HI_2P4);
   f = fp_quot(A, r, ir);
   p.XP = p.XP * f;
   p.YP = p.YP * f;
@@ -243,13 +245,12 @@ __device__ __forceinline__ bool csr_slice_fast(SlicePart &pio, const DevElem &e,
   f = fp_quot(1.0, r, ir);
   p.XP = p.XP * f;
   p.YP = p.YP * f;
-  p.CT = p.CT + fp_quot(dist, p.beta0, fp_recip(p.beta0));
-  if (ok)
-    pio = p;
-  return ok;
+  const double b0 = *beta0;
+  p.CT = *ct0 + fp_quot(dist, b0, fp_recip(b0));
+  return ok && fp_within(b0, FP_HI_2M10, FP_HI_2);
 }
 
-constexpr int SLICE_THREADS = 128, SLICE_COLS = 7;
+constexpr int SLICE_THREADS = 128, SLICE_COLS = 7, SLICE_BLOCKS_PER_SM = 6;
 
 __device__ __forceinline__ void copy8_async(void *smem, const void *gmem) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
@@ -263,12 +264,15 @@ __device__ __forceinline__ void copy4_async(void *smem, const void *gmem) {
 /* One kick of every particle, and min/max of c*t per bunch (csbend.c:3066-3076).
  * Each block takes a run of 128-particle tiles; a thread copies its particle of
  * the next tile into shared memory (its own words only, so no barrier) while it
- * integrates the current one.  Bound by issue: about 840 warp instructions, 410
- * of them FP64, per warp of particles.  Before, a block per 256 particles waited
- * for the loss word, then for the coordinates, then for the velocity, and every
- * warp sent two atomics to the bunch's range words; here the range stays in
- * registers until the bunch changes. */
-__global__ void __launch_bounds__(SLICE_THREADS, 6)
+ * integrates the current one.  Bound by the FP64 pipe and its register ports:
+ * of about 920 warp instructions per 32 particles 430 are FP64, and an fma of
+ * three different registers issues every third cycle, not every second.  20 to
+ * 32 warps per SM, and two particles per thread, all measured within 2 %.
+ * Before, a block per 256 particles waited for the loss word, then for the
+ * coordinates, then for the velocity, and every warp sent two atomics to the
+ * bunch's range words; here the range stays in registers until the bunch
+ * changes. */
+__global__ void __launch_bounds__(SLICE_THREADS, SLICE_BLOCKS_PER_SM)
     csr_slice_kernel(DevParticles P, int64_t n, int64_t tiles_per_block, const double *beta0,
                      const __grid_constant__ DevElem e, CsrBunches B, int after_first_kick, int nBins, double Po,
                      double inv_Po, int pass, int elem_index) {
@@ -322,13 +326,17 @@ __global__ void __launch_bounds__(SLICE_THREADS, 6)
     bool alive = i < end && lost_word[slot][t] < 0;
     SlicePart p;
     if (alive) {
-      p = {col[slot][0][t], col[slot][1][t], col[slot][2][t], col[slot][3][t], col[slot][4][t], col[slot][5][t],
-           col[slot][6][t]};
+      const double(*v)[SLICE_THREADS] = col[slot];
       const SliceWake w = {st->dGamma, st->ctLower, st->dct, nBins, after_first_kick && B.csr_const[bunch] != 0};
       int lost = 0;
+      p.X = v[0][t];
+      p.XP = v[1][t];
+      p.Y = v[2][t];
+      p.YP = v[3][t];
+      p.DP = v[5][t];
       if (!(straight && (!w.apply || fp_within(w.dct, FP_HI_2M250, FP_HI_2P100)) &&
-            csr_slice_fast(p, e, w, fp_recip(w.dct), Po, inv_Po))) {
-        SlicePart q = p;
+            csr_slice_fast(p, e, w, &v[4][t], &v[6][t], Po, inv_Po))) {
+        SlicePart q = {v[0][t], v[1][t], v[2][t], v[3][t], v[4][t], v[5][t], v[6][t]};
         lost = csr_slice_general(&q, &e, st, nBins, w.apply, Po);
         p = q;
       }
@@ -370,7 +378,8 @@ __global__ void __launch_bounds__(SLICE_THREADS, 6)
  * an equal run of tiles */
 static inline int slice_grid(int64_t n, int64_t *tiles_per_block) {
   const int64_t tiles = std::max<int64_t>(1, (n + SLICE_THREADS - 1) / SLICE_THREADS);
-  *tiles_per_block = (tiles + 148 * 8 - 1) / (148 * 8);
+  const int64_t slots = 148 * SLICE_BLOCKS_PER_SM;
+  *tiles_per_block = (tiles + slots - 1) / slots;
   return (int)((tiles + *tiles_per_block - 1) / *tiles_per_block);
 }
 
@@ -395,11 +404,11 @@ static inline size_t hist_smem(int nBins) {
   return copies * one;
 }
 
-/* histogram CTAs (1024 threads) per bunch: one per 1024 particles, at most two
- * resident CTAs per SM over all bunches (each thread then takes up to
- * kHistUnroll particles per sweep) */
+/* histogram CTAs (1024 threads) per bunch: one per 1024 particles, at most one
+ * per SM over all bunches (two take 1.2 us more per kick at 1e6 particles, for
+ * the atomics with which each adds its counts to the bunch's) */
 static inline int hist_blocks(int64_t per_bunch, int nbunch) {
-  return (int)std::min<int64_t>(std::max<int64_t>(1, 148 * 2 / std::max(nbunch, 1)),
+  return (int)std::min<int64_t>(std::max<int64_t>(1, 148 / std::max(nbunch, 1)),
                                 std::max<int64_t>(1, (per_bunch + 1023) / 1024));
 }
 
@@ -424,7 +433,16 @@ static cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
 __global__ void csr_hist_kernel(DevParticles P, int64_t n, CsrBunches B, unsigned int *counts_all, int nBins,
                                 double factor) {
   extern __shared__ unsigned int scount[];
-  chain_enter();
+  chain_release();
+  /* the launch gives copies x nBins counters (hist_smem) */
+  unsigned int smem_bytes;
+  asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(smem_bytes));
+  const int copies = (int)(smem_bytes / (sizeof(unsigned int) * nBins));
+  unsigned int *mycount = scount + (size_t)((threadIdx.x >> 5) % copies) * nBins;
+  for (int b = threadIdx.x; b < copies * nBins; b += blockDim.x)
+    scount[b] = 0;
+  __syncthreads();
+  chain_wait(); /* so far only this block's shared memory */
   const int bunch = blockIdx.y;
   if (!B.active[bunch])
     return;
@@ -434,14 +452,6 @@ __global__ void csr_hist_kernel(DevParticles P, int64_t n, CsrBunches B, unsigne
   double lower = value_of(st->ct_min_key), upper = value_of(st->ct_max_key), dct;
   expand_range(&lower, &upper, factor);
   dct = (upper - lower) / nBins;
-  /* the launch gives copies x nBins counters (hist_smem) */
-  unsigned int smem_bytes;
-  asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(smem_bytes));
-  const int copies = (int)(smem_bytes / (sizeof(unsigned int) * nBins));
-  unsigned int *mycount = scount + (size_t)((threadIdx.x >> 5) % copies) * nBins;
-  for (int b = threadIdx.x; b < copies * nBins; b += blockDim.x)
-    scount[b] = 0;
-  __syncthreads();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->ctLower = lower;
     st->ctUpper = upper;
@@ -450,11 +460,9 @@ __global__ void csr_hist_kernel(DevParticles P, int64_t n, CsrBunches B, unsigne
   /* kHistUnroll particles per thread and sweep, their loads issued together
    * (the loss word and c*t are read unconditionally within the range, so
    * neither waits on the other); the loop bounds are uniform over the block */
-  /* (c*t - lower)/dct through the stored reciprocal, correctly rounded as the
-   * division (div_rn_recip), while dct is a normal number well inside the
-   * range where 1/dct and the remainder stay normal */
-  const double inv_dct = 1.0 / dct;
-  const bool recip_ok = dct > 1e-280 && dct < 1e280;
+  /* (c*t - lower)/dct through the reciprocal, rounded as the division */
+  const double inv_dct = fp_recip(dct);
+  const bool recip_ok = fp_within(dct, FP_HI_2M250, FP_HI_2P100);
   /* chunks of blockDim.x particles, chunk c to CTA c mod gridDim.x */
   const int64_t G = gridDim.x, D = blockDim.x;
   for (int64_t c0 = blockIdx.x; first + c0 * D < end; c0 += G * kHistUnroll) {
@@ -466,27 +474,27 @@ __global__ void csr_hist_kernel(DevParticles P, int64_t n, CsrBunches B, unsigne
       lp[u] = i < end ? P.lost_pass[i] : 0;
       ct[u] = i < end ? P.s[i] : 0.0;
     }
+    int bin[kHistUnroll];
 #pragma unroll
     for (int u = 0; u < kHistUnroll; u++) {
-      const int64_t i = first + (c0 + u * G) * D + threadIdx.x;
-      int bin = -1;
-      if (i < end && lp[u] < 0) {
-        const double a = ct[u] - lower;
-        long long b = (long long)(recip_ok ? div_rn_recip(a, dct, inv_dct) : a / dct);
-        if (b >= 0 && b <= nBins - 1)
-          bin = (int)b;
-      }
-      /* one shared-memory atomic per particle, unless neighbouring lanes
-       * share a bin (a beam stored in c*t order, where a warp's particles
-       * would queue on one counter): then one atomic per distinct bin */
-      const int lane = threadIdx.x & 31;
-      const int prev = __shfl_up_sync(0xffffffffu, bin, 1);
-      if (__any_sync(0xffffffffu, lane > 0 && bin >= 0 && bin == prev)) {
-        const unsigned int peers = __match_any_sync(0xffffffffu, bin);
-        if (bin >= 0 && lane == __ffs(peers) - 1)
-          atomicAdd(&mycount[bin], (unsigned int)__popc(peers));
-      } else if (bin >= 0) {
-        atomicAdd(&mycount[bin], 1u);
+      const double a = ct[u] - lower, q = recip_ok ? fp_quot(a, dct, inv_dct) : a / dct;
+      /* the truncated quotient in [0, nBins); out of it for NaN */
+      bin[u] = lp[u] < 0 && q > -1 && q < nBins ? (int)q : -1;
+    }
+    /* one shared-memory atomic per particle, unless neighbouring lanes share a
+     * bin (a beam stored in c*t order, where a warp's particles would queue on
+     * one counter; looked for in the sweep's first particles): then one atomic
+     * per distinct bin */
+    const int lane = threadIdx.x & 31, prev = __shfl_up_sync(0xffffffffu, bin[0], 1);
+    const bool shared_bins = __any_sync(0xffffffffu, lane > 0 && bin[0] >= 0 && bin[0] == prev);
+#pragma unroll
+    for (int u = 0; u < kHistUnroll; u++) {
+      if (shared_bins) {
+        const unsigned int peers = __match_any_sync(0xffffffffu, bin[u]);
+        if (bin[u] >= 0 && lane == __ffs(peers) - 1)
+          atomicAdd(&mycount[bin[u]], (unsigned int)__popc(peers));
+      } else if (bin[u] >= 0) {
+        atomicAdd(&mycount[bin[u]], 1u);
       }
     }
   }
@@ -631,6 +639,21 @@ __device__ __forceinline__ double ordered_sum(const double *v, int n) {
 /* weights up to this many per table are staged in shared memory (windows of 17) */
 constexpr int SG_STAGE = 17 * 17;
 
+/* both tables into stage, which a then points to; wider ones stay where they
+ * are.  The tables are older than any kernel in flight: a chained kernel stages
+ * them before it waits for its predecessor. */
+__device__ __forceinline__ void stage_weights(WakeArgs &a, double (&stage)[2][SG_STAGE]) {
+  const int w0 = sg_width(a.sgHalf, a.nBins), w1 = sg_width(a.sgdHalf, a.nBins);
+  if (w0 * w0 > SG_STAGE || w1 * w1 > SG_STAGE)
+    return;
+  for (int k = threadIdx.x; k < w0 * w0; k += blockDim.x)
+    stage[0][k] = a.sg_w[k];
+  for (int k = threadIdx.x; k < w1 * w1; k += blockDim.x)
+    stage[1][k] = a.sgd_w[k];
+  a.sg_w = stage[0];
+  a.sgd_w = stage[1];
+}
+
 /* Filters of one kick's wake (csbend.c:2566-2591) on one CTA: Savitzky-Golay
  * smoothing of the counts, correctDistribution, density per unit ct, its
  * derivative filter and the (dct*b)^(1/3) denominators.  Leaves hist = sm,
@@ -645,18 +668,6 @@ __device__ bool wake_filters(const CountT *counts, const WakeArgs &a, const doub
   __shared__ double nBinnedD;
   __shared__ int skip;
   __shared__ SumT warp_sums[32];
-  __shared__ double stage[2][SG_STAGE];
-  /* the weights come in with the counts */
-  const int w0 = sg_width(a.sgHalf, nb), w1 = sg_width(a.sgdHalf, nb);
-  const double *sg_w = a.sg_w, *sgd_w = a.sgd_w;
-  if (w0 * w0 <= SG_STAGE && w1 * w1 <= SG_STAGE) {
-    for (int k = threadIdx.x; k < w0 * w0; k += blockDim.x)
-      stage[0][k] = sg_w[k];
-    for (int k = threadIdx.x; k < w1 * w1; k += blockDim.x)
-      stage[1][k] = sgd_w[k];
-    sg_w = stage[0];
-    sgd_w = stage[1];
-  }
   if constexpr (std::is_integral<SumT>::value) {
     /* integer counts: the total is exact in any order, so it is a block
      * reduction (per thread, warp shuffles, then the warps' totals) */
@@ -697,7 +708,7 @@ __device__ bool wake_filters(const CountT *counts, const WakeArgs &a, const doub
   if (a.lh)
     lh_pass_filters(a, sm);
   if (a.sgHalf > 0) {
-    sg_apply(hist, tmp, nb, a.sgHalf, sg_w);
+    sg_apply(hist, tmp, nb, a.sgHalf, a.sg_w);
     __syncthreads();
     /* correctDistribution (csbend.c:4705-4721): negative bins clipped in
      * parallel, then the sum in bin order, as the reference forms it */
@@ -737,7 +748,7 @@ __device__ bool wake_filters(const CountT *counts, const WakeArgs &a, const doub
     hist[b] = hist[b] / dct;
   }
   __syncthreads();
-  sg_apply(hist, deriv, nb, a.sgdHalf, sgd_w);
+  sg_apply(hist, deriv, nb, a.sgdHalf, a.sgd_w);
   if (!INVERSE) {
     __syncthreads();
     return false;
@@ -979,7 +990,10 @@ __device__ void wake_body(const CountT *counts, const WakeArgs &a, const double 
 __global__ void __launch_bounds__(1024, 1) csr_wake_kernel(CsrBunches B, unsigned int *counts_all, WakeArgs a,
                                                            int recycle) {
   extern __shared__ double sm[];
-  chain_enter();
+  __shared__ double stage[2][SG_STAGE];
+  chain_release();
+  stage_weights(a, stage);
+  chain_wait();
   const int bunch = blockIdx.x;
   /* the bunch's scalars load together with its active flag (all in bounds) */
   const int active = B.active[bunch];
@@ -1052,6 +1066,8 @@ __device__ double block_sum(double v, double *red) {
 __global__ void __launch_bounds__(1024, 1) csr_sur_filter_kernel(CsrBunches B, const unsigned int *counts_all, WakeArgs a, int L, float sc_dens,
                                       float sc_deriv, double *tab, double *scal, float *inputs) {
   extern __shared__ double sm[];
+  __shared__ double stage[2][SG_STAGE];
+  stage_weights(a, stage);
   const int b = blockIdx.x, nb = a.nBins;
   float *in = inputs + (size_t)b * 4 * L;
   if (!B.active[b]) {
@@ -1199,6 +1215,8 @@ __global__ void __launch_bounds__(BATCH_THREADS)
     w.sg_w = sg.w[0];
     w.sgd_w = sg.w[1];
   }
+  __shared__ double stage[2][SG_STAGE];
+  stage_weights(w, stage);
   w.slippage = slippage_bins[blockIdx.x];
   w.slippage13 = 1;
   w.c1 = 1;
@@ -1408,7 +1426,10 @@ __device__ __forceinline__ long long clamp_bins(double d, int nb) {
  * memory: 4 nBins + 8 doubles for the filters, nBins for phi. */
 __global__ void __launch_bounds__(1024, 1) stupakov_wake_kernel(CsrBunches B, const unsigned int *counts_all, WakeArgs a, StupakovArgs sa) {
   extern __shared__ double sm[];
-  chain_enter();
+  __shared__ double stage[2][SG_STAGE];
+  chain_release();
+  stage_weights(a, stage);
+  chain_wait();
   const int bunch = blockIdx.x;
   if (!B.mode[bunch])
     return;

@@ -265,6 +265,9 @@ B2E_HD double b2e_cbrt_dd(double x, double *c, double *mout, int *qout) {
   r = e - 3 * q; /* 0, 1, 2 */
   m = ldexp(m, r); /* in [1/2, 4) */
   y = 0.65 + 0.25 * m - 0.0185 * m * m; /* within 6% on [1/2, 4) */
+#ifdef __CUDACC__
+#pragma unroll 1 /* one copy of the division: callers are short of instruction cache, not of issue slots */
+#endif
   for (int i = 0; i < 6; i++)
     y = y - (y * y * y - m) / (3.0 * y * y);
   /* residual m - y^3 with y^3 as an unevaluated sum */
