@@ -21,6 +21,7 @@
 #include <string.h>
 #include <algorithm>
 #include <string>
+#include <utility>
 #include <vector>
 #include "b2e_tmap.h"
 #include "b2e_umma.cuh"
@@ -176,6 +177,30 @@ __device__ __forceinline__ Row16 load_row16(const __nv_bfloat16 *p) {
   return r;
 }
 
+/* Programmatic dependent launch: the network's kernels follow one another on
+ * one stream, each with a prologue (barriers, tensor memory, weights) that needs
+ * nothing of its predecessor.  chain_release lets the next kernel's CTAs start
+ * where this one's have left, chain_wait holds them before they touch what the
+ * predecessor writes. */
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_chained(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t stream,
+                                  Args &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
 template <int EPI>
 __global__ void __launch_bounds__(CONV_THREADS, 2)
     conv_kernel(const __grid_constant__ CUtensorMap t_in, const __grid_constant__ CUtensorMap t_w, ConvArgs a) {
@@ -187,6 +212,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
   __shared__ uint32_t tmem_base;
   __shared__ float sbias[64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  chain_release();
   const int tpp = a.L >> 7, n_tiles = a.n_prof * tpp;
   constexpr int N = EPI == EPI_OUTPUT ? 16 : 64;
   constexpr uint32_t IDESC = umma::idesc_bf16(128, N, false, false);
@@ -208,19 +234,24 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
   if (warp == 0) {
     tmem_alloc(&tmem_base, 128);
     tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tmem_base;
-
-  if (warp == 0) {
     if (lane == 0) {
+      /* the weights are older than any kernel of the pass */
       prefetch_tmap(&t_in);
       prefetch_tmap(&t_w);
       mbar_expect_tx(&wbar, (uint32_t)CONV_W_BYTES);
       for (int t = 0; t < WN_TAPS; t++)
         tma_load_3d(sw + t * 8192, &t_w, &wbar, 0, t * 64, 0);
+    }
+    __syncwarp();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_base;
+  chain_wait();
+
+  if (warp == 0) {
+    if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
@@ -356,6 +387,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   __shared__ __align__(8) uint64_t full[WG_STAGES], empty[WG_STAGES], done;
   __shared__ uint32_t tmem_base;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  chain_release();
   const int tpp = a.L >> 7, n_tiles = a.n_prof * tpp;
   constexpr uint32_t IDESC = umma::idesc_bf16(128, 64, true, true);
 
@@ -384,6 +416,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem = tmem_base;
   bool any = false;
+  chain_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -481,17 +514,17 @@ cudaError_t launch_conv(int epi, const CUtensorMap &t_in, const CUtensorMap &t_w
   case EPI_HIDDEN:
     e = cudaFuncSetAttribute(conv_kernel<EPI_HIDDEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
     if (e == cudaSuccess)
-      conv_kernel<EPI_HIDDEN><<<grid, CONV_THREADS, CONV_SMEM, s>>>(t_in, t_w, a);
+      e = launch_chained(conv_kernel<EPI_HIDDEN>, grid, CONV_THREADS, CONV_SMEM, s, t_in, t_w, a);
     break;
   case EPI_OUTPUT:
     e = cudaFuncSetAttribute(conv_kernel<EPI_OUTPUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
     if (e == cudaSuccess)
-      conv_kernel<EPI_OUTPUT><<<grid, CONV_THREADS, CONV_SMEM, s>>>(t_in, t_w, a);
+      e = launch_chained(conv_kernel<EPI_OUTPUT>, grid, CONV_THREADS, CONV_SMEM, s, t_in, t_w, a);
     break;
   default:
     e = cudaFuncSetAttribute(conv_kernel<EPI_BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
     if (e == cudaSuccess)
-      conv_kernel<EPI_BWD><<<grid, CONV_THREADS, CONV_SMEM, s>>>(t_in, t_w, a);
+      e = launch_chained(conv_kernel<EPI_BWD>, grid, CONV_THREADS, CONV_SMEM, s, t_in, t_w, a);
     break;
   }
   return e == cudaSuccess ? cudaGetLastError() : e;
@@ -502,8 +535,7 @@ cudaError_t launch_wgrad(const CUtensorMap &t_in, const CUtensorMap &t_dz, const
   cudaError_t e = cudaFuncSetAttribute(wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WG_SMEM);
   if (e != cudaSuccess)
     return e;
-  wgrad_kernel<<<grid, WG_THREADS, WG_SMEM, s>>>(t_in, t_dz, a);
-  return cudaGetLastError();
+  return launch_chained(wgrad_kernel, grid, WG_THREADS, WG_SMEM, s, t_in, t_dz, a);
 }
 
 } // namespace b2e
@@ -597,6 +629,8 @@ __global__ void __launch_bounds__(64 * REDUCE_SPLIT)
     wn_reduce_kernel(const float *wpart, int n_wblocks, const float *bpart, float scale, float *grad_w,
                      float *grad_b) {
   __shared__ float part[REDUCE_SPLIT][64];
+  chain_release();
+  chain_wait();
   const int c = threadIdx.x & 63, g = threadIdx.x >> 6;
   const int idx = blockIdx.x * 64 + c; /* (t, ci, co), then the 64 biases */
   const bool weights = idx < WN_WSIZE;
@@ -730,9 +764,9 @@ int backward(b2e_wakenet *n, const float *targets, int n_prof, double *loss, cud
     w.bias_partial = n->bpart;
     w.status = n->status;
     WN_TRY(n, launch_wgrad(l == 0 ? n->t_x0 : n->t_act[l - 1], n->t_dz[l], w, wgrid, s));
-    wn_reduce_kernel<<<WN_WSIZE / 64 + 1, 64 * REDUCE_SPLIT, 0, s>>>(
-        n->wpart, wgrid, n->bpart, scale, n->grads + l * WN_WSIZE, n->grads + WN_LAYERS * WN_WSIZE + l * WN_CH);
-    WN_TRY(n, cudaGetLastError());
+    WN_TRY(n, launch_chained(wn_reduce_kernel, WN_WSIZE / 64 + 1, 64 * REDUCE_SPLIT, 0, s, (const float *)n->wpart, wgrid,
+                             (const float *)n->bpart, scale, n->grads + l * WN_WSIZE,
+                             n->grads + WN_LAYERS * WN_WSIZE + l * WN_CH));
     if (l > 0) {
       ConvArgs a{};
       a.L = n->L;
