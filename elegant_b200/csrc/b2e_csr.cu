@@ -982,6 +982,9 @@ __device__ void wake_body(const CountT *counts, const WakeArgs &a, const double 
   }
 }
 
+/* threads of a wake CTA: a warp for the serial sum beside one thread per bin */
+static inline int wake_threads(int bins) { return std::min(1024, (bins + 31) / 32 * 32 + 32); }
+
 /* wake of one kick, one CTA per bunch; c1 and c2 from the bunch's CSRConstant
  * in the host expression's order (csbend.c:2664-2667).  With recycle set the
  * CTA also readies its bunch for the next binning pass once this one's inputs
@@ -2021,7 +2024,7 @@ static int stupakov_drift(CsrState &st, const CsrElem &ce, const CsrBunches &B, 
       err = "CSR: the all-rank reduction of the histogram failed";
       return B2E_ERR_CUDA;
     }
-    CSR_CUDA(launch_chained(stupakov_wake_kernel, dim3(nbunch), dim3(1024), smem, stream, B,
+    CSR_CUDA(launch_chained(stupakov_wake_kernel, dim3(nbunch), dim3(wake_threads(nb)), smem, stream, B,
                             (const unsigned int *)st.d_counts, a, sa));
     CSR_CUDA(launch_chained(stupakov_kick_kernel, dim3(g), dim3(256), 0, stream, P, n, B, nb, Po));
     (*launches) += 2;
@@ -2297,7 +2300,7 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
       st.gate_values += nbunch;
       (*launches) += 3 + 7; /* filter, pack + 6 convolutions, combine */
     } else {
-      CSR_CUDA(launch_chained(csr_wake_kernel, dim3(nbunch), dim3(1024), wake_smem, stream, B, st.d_counts, a,
+      CSR_CUDA(launch_chained(csr_wake_kernel, dim3(nbunch), dim3(wake_threads(ce.bins)), wake_smem, stream, B, st.d_counts, a,
                               recycle ? 1 : 0));
       (*launches)++;
       CSR_CUDA(cudaGetLastError());
@@ -2694,7 +2697,7 @@ extern "C" int b2e_csr_bend_static(double *const dev_columns[6], int32_t *dev_lo
     a.const1 = 6.0 - b2e_log(27.0 / 4.0);
     a.q4pe = kE / (4 * kPI * eps0);
     a.igf_factor = 0;
-    csr_wake_kernel<<<1, 1024, wake_smem, s>>>(B, S->counts, a, 0);
+    csr_wake_kernel<<<1, wake_threads(bins), wake_smem, s>>>(B, S->counts, a, 0);
     STATIC_TRY(cudaGetLastError());
   }
   csr_reset_keys_kernel<<<1, 32, 0, s>>>(B);

@@ -255,15 +255,24 @@ __device__ __forceinline__ double asin_series(double x, bool tiny) {
   return fma(x * w, p, x);
 }
 
-__device__ __forceinline__ double sin_series(double r, double w, bool small) {
-  double p = kSinSeries[3];
-  if (!small) {
-    double q = kSinSeries[8];
+/* the high-order terms of both, which enter the Horner chains below in the
+ * place of their leading coefficients */
+__device__ __forceinline__ double sin_prefix(double w) {
+  double q = kSinSeries[8];
 #pragma unroll
-    for (int k = 7; k >= 4; k--)
-      q = fma(q, w, kSinSeries[k]);
-    p = fma(q, w, kSinSeries[3]);
-  }
+  for (int k = 7; k >= 3; k--)
+    q = fma(q, w, kSinSeries[k]);
+  return q;
+}
+__device__ __forceinline__ double cos_prefix(double w) {
+  double q = kCosSeries[8];
+#pragma unroll
+  for (int k = 7; k >= 2; k--)
+    q = fma(q, w, kCosSeries[k]);
+  return q;
+}
+
+__device__ __forceinline__ double sin_tail(double r, double w, double p) {
 #pragma unroll
   for (int k = 2; k >= 0; k--)
     p = fma(p, w, kSinSeries[k]);
@@ -271,15 +280,7 @@ __device__ __forceinline__ double sin_series(double r, double w, bool small) {
 }
 
 /* 0.5 w is exact, so the two differences with it are one fma each */
-__device__ __forceinline__ double cos_series(double w, bool small) {
-  double p = kCosSeries[2];
-  if (!small) {
-    double q = kCosSeries[8];
-#pragma unroll
-    for (int k = 7; k >= 3; k--)
-      q = fma(q, w, kCosSeries[k]);
-    p = fma(q, w, kCosSeries[2]);
-  }
+__device__ __forceinline__ double cos_tail(double w, double p) {
   p = fma(p, w, kCosSeries[1]);
   p = fma(p, w, kCosSeries[0]);
   const double t = fma(-0.5, w, 1.0);
@@ -302,9 +303,14 @@ __device__ __forceinline__ void bend_drift_fast(double &X, double &QX, double &Y
   sin_max = max(sin_max, fp_abs_hi(sin_phi));
   const double phi = asin_series(sin_phi, abs_at_most(sin_phi, 0x1p-6)), arg = dsh_rho0 + phi;
   const double wa = arg * arg, wp = phi * phi;
-  const bool small = abs_at_most(arg, 0x1p-4);
-  const double sine = sin_series(arg, wa, small), cosi = cos_series(wa, small);
-  const double cos_phi = cos_series(wp, abs_at_most(phi, 0x1p-4));
+  double ps = kSinSeries[3], pc = kCosSeries[2], pp = kCosSeries[2];
+  const bool small = abs_at_most(arg, 0x1p-4), small_phi = abs_at_most(phi, 0x1p-4);
+  if (!(small && small_phi)) { /* one branch for the three series */
+    ps = small ? ps : sin_prefix(wa);
+    pc = small ? pc : cos_prefix(wa);
+    pp = small_phi ? pp : cos_prefix(wp);
+  }
+  const double sine = sin_tail(arg, wa, ps), cosi = cos_tail(wa, pc), cos_phi = cos_tail(wp, pp);
   const double ic = fp_recip(cosi), ip = fp_recip(cos_phi);
   const double tang = fp_quot(sine, cosi, ic), ratio = fp_quot(cos_phi, cosi, ic);
   const double factor = fp_quot((rho0 + X) * cos_phi, f, inv_f) * (tang - fp_quot(sin_phi, cos_phi, ip));
