@@ -1394,26 +1394,98 @@ struct StupakovFn {
   __device__ double operator()(double phi) const { return phi * phi * phi * (phi + x4) / (phi + x); }
 };
 
-/* SolveForPhiStupakov (csbend.c:4169-4202); *phi_last carries the start
- * value from one solve to the next */
-__device__ double stupakov_phi(double x, double ds, double phim, double *phi_last) {
-  if (ds < 0)
-    return -1;
-  if (ds == 0)
-    return 0;
-  ds *= 24;
-  StupakovFn fn;
-  fn.x = x;
-  fn.x4 = 4 * x;
-  if (*phi_last == -1)
-    *phi_last = phim / 2;
-  if (fabs(ds - fn(phim)) < ds / 1e4) {
-    *phi_last = phim;
-    return phim;
+/* The grid of b2e_zero_interp's scan for SolveForPhiStupakov and the function
+ * on it: neither depends on the distance, so a kick's solutions share them.
+ * The scan takes steps of phim/100 from 0 and ends beyond 1.01 phim. */
+#define PHI_SCAN 128
+struct PhiScan {
+  double x[PHI_SCAN + 1], f[PHI_SCAN + 1];
+};
+
+__device__ __forceinline__ void phi_scan_fill(PhiScan &scan, const StupakovFn &fn, double phim) {
+  const double dx = phim / 100;
+  for (int k = threadIdx.x; k <= PHI_SCAN; k += blockDim.x) {
+    double x = 0;
+    for (int j = 0; j < k; j++) /* the scan's own sums */
+      x = x + dx;
+    scan.x[k] = x;
+    scan.f[k] = fn(x);
   }
-  double phi = b2e_zero_newton(fn, ds, *phi_last, phim / 1000, 3, ds / 1e4);
-  if (phi < 0 || phi > phim || fabs(ds - fn(phi)) > ds / 1e4)
-    phi = b2e_zero_interp(fn, ds, 0, phim * 1.01, phim / 100, ds / 1e4);
+}
+
+/* b2e_zero_interp(fn, value, 0, phim * 1.01, phim / 100, tol) by one warp: the
+ * scan for a hit or a change of sign 32 steps at a time, the refinement in
+ * every lane alike */
+__device__ double phi_interp(const PhiScan &scan, const StupakovFn &fn, double value, double phim, double tol) {
+  const double x_f = phim * 1.01, dx = phim / 100;
+  if (!(dx > 0) || !(scan.x[PHI_SCAN] > x_f))
+    return b2e_zero_interp(fn, value, 0, x_f, dx, tol);
+  if (fabs(scan.f[0] - value) < tol)
+    return 0;
+  int found = 0;
+  for (int base = 1; base <= PHI_SCAN && found == 0; base += 32) {
+    const int k = base + (threadIdx.x & 31);
+    const double ga = scan.f[k - 1] - value, gb = scan.f[k] - value;
+    const bool here =
+        scan.x[k] > x_f || fabs(gb) < tol || (ga == ga && gb == gb && (ga < 0) != (gb < 0));
+    const unsigned any = __ballot_sync(0xffffffffu, here);
+    if (any)
+      found = base + __ffs(any) - 1;
+  }
+  double xa = scan.x[found - 1], xb = scan.x[found], xm = xa;
+  double ga = scan.f[found - 1] - value, gb = scan.f[found] - value;
+  if (xb > x_f)
+    return x_f + dx;
+  if (fabs(gb) < tol)
+    return xb;
+  for (int k = 0, side = 0; k < B2E_ROOT_MAX_REFINE; k++) {
+    xm = xa - ga * (xb - xa) / (gb - ga);
+    const double gm = fn(xm) - value;
+    if (fabs(gm) < tol)
+      return xm;
+    if ((gm < 0) == (ga < 0)) {
+      xa = xm;
+      ga = gm;
+      if (side == -1)
+        gb = gb / 2;
+      side = -1;
+    } else {
+      xb = xm;
+      gb = gm;
+      if (side == 1)
+        ga = ga / 2;
+      side = 1;
+    }
+  }
+  return xm;
+}
+
+/* The solving part of SolveForPhiStupakov (csbend.c:4169-4202) by one warp:
+ * phi for the scaled distance ds (> 0) from the previous solution phi_last.
+ * b2e_zero_newton's passes with the two values of a pass formed by even and
+ * odd lanes; a pass that ends within the tolerance has made the check of its
+ * answer. */
+__device__ double stupakov_phi(const PhiScan &scan, const StupakovFn &fn, double ds, double tol, double phim,
+                               double *phi_last) {
+  const double dx = phim / 1000;
+  double phi = *phi_last, x_diff = phi;
+  bool fits;
+#pragma unroll 1
+  for (int pass = 0;; pass++) {
+    const double next = phi + dx, g_lane = fn(threadIdx.x & 1 ? next : phi) - ds;
+    const double g = __shfl_sync(0xffffffffu, g_lane, 0), g_diff = __shfl_sync(0xffffffffu, g_lane, 1);
+    fits = fabs(g) < tol;
+    if (fits)
+      break;
+    if (pass == 2) {
+      phi = (phi + x_diff) / 2;
+      break;
+    }
+    x_diff = next;
+    phi = phi - g / ((g_diff - g) / dx);
+  }
+  if (phi < 0 || phi > phim || (!fits && fabs(ds - fn(phi)) > tol))
+    phi = phi_interp(scan, fn, ds, phim, tol);
   if (phi < 0 || phi > phim)
     return -1;
   *phi_last = phi;
@@ -1437,14 +1509,23 @@ __device__ __forceinline__ long long clamp_bins(double d, int nb) {
   return d >= (double)nb ? nb : (long long)d;
 }
 
+/* marks in place of a solution's tolerance */
+#define PHI_KNOWN (-1.0)
+#define PHI_MAX (-2.0)
+#define PHI_END (-3.0)
+
 /* wake of one Stupakov kick, one CTA per bunch (csbend.c:3950-4054): the
- * histogram filters of the last dipole, phi solutions (serial, each starting
- * from the previous one), then per bin case C, case D's boundary term and its
+ * histogram filters of the last dipole, phi solutions (one warp, each starting
+ * from the previous one: the latency of that chain bounds the kernel, 64 us
+ * before and about 30 now for 300 bins, with the scan tabulated, the values of
+ * a Newton pass side by side and all that is no part of the chain formed by the
+ * whole block), then per bin case C, case D's boundary term and its
  * integral in the reference's order, times -4/rho GSConstant dz0.  Shared
  * memory: 4 nBins + 8 doubles for the filters, nBins for phi. */
 __global__ void __launch_bounds__(1024, 1) stupakov_wake_kernel(CsrBunches B, const unsigned int *counts_all, WakeArgs a, StupakovArgs sa) {
   extern __shared__ double sm[];
   __shared__ double stage[2][SG_STAGE];
+  __shared__ PhiScan scan;
   chain_release();
   stage_weights(a, stage);
   chain_wait();
@@ -1462,15 +1543,51 @@ __global__ void __launch_bounds__(1024, 1) stupakov_wake_kernel(CsrBunches B, co
       st->dGamma[ib] = 0;
     return;
   }
-  if (threadIdx.x == 0) {
+  /* what a solution does not need the previous one for; the tolerance is below
+   * zero where there is nothing to solve */
+  const StupakovFn fn = {sa.x, 4 * sa.x};
+  double *scaled = sm + 2 * nb, *tol = sm + 3 * nb;
+  phi_scan_fill(scan, fn, sa.theta);
+  const double at_phim = fn(sa.theta);
+  for (int ib = threadIdx.x; ib < nb; ib += blockDim.x) {
+    double ds = ib * dct / sa.rho, t = PHI_KNOWN, p = -1;
+    if (ib * dct > sa.dsMax)
+      t = PHI_END;
+    else if (ds == 0)
+      p = 0;
+    else if (!(ds < 0)) {
+      ds *= 24;
+      t = ds / 1e4;
+      if (fabs(ds - at_phim) < t) {
+        t = PHI_MAX;
+        p = sa.theta;
+      }
+    }
+    scaled[ib] = ds;
+    tol[ib] = t;
+    phi[ib] = p;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
     double last = st->phi_last;
     for (int ib = 0; ib < nb; ib++) {
-      phi[ib] = -1;
-      if (ib * dct > sa.dsMax)
+      const double t = tol[ib];
+      if (t == PHI_END)
         break;
-      phi[ib] = stupakov_phi(sa.x, ib * dct / sa.rho, sa.theta, &last);
+      if (t == PHI_KNOWN)
+        continue;
+      if (last == -1)
+        last = sa.theta / 2;
+      if (t == PHI_MAX) {
+        last = sa.theta;
+        continue;
+      }
+      const double p = stupakov_phi(scan, fn, scaled[ib], t, sa.theta, &last);
+      if (threadIdx.x == 0)
+        phi[ib] = p;
     }
-    st->phi_last = last;
+    if (threadIdx.x == 0)
+      st->phi_last = last;
   }
   __syncthreads();
   const long long diC = clamp_bins(sa.dsC / dct, nb), diD = clamp_bins(sa.dsMax / dct, nb);
