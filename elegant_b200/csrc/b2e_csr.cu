@@ -2588,8 +2588,8 @@ void csr_release(CsrState &st) {
  *
  * The array holds per-particle entrance velocities (up to
  * B2E_STATIC_MAX_PARTICLES), the CSR binning/wake state, the histogram, the
- * Savitzky-Golay weight tables (up to B2E_STATIC_MAX_BINS bins) and the
- * element record: about 10.2 MB.  Under lazy module loading (CUDA's default)
+ * Savitzky-Golay weight tables (of the widest windows) and the
+ * element record: about 8.5 MB.  Under lazy module loading (CUDA's default)
  * a device gives it memory when this module is first used there -- the
  * set-up in static_scratch() -- and keeps it until the process exits.  The
  * call only enqueues work: the alive count that decides whether CSR is

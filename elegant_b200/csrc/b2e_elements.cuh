@@ -579,39 +579,24 @@ __device__ __forceinline__ void bend_kick(double X, double Y, double &QX, double
   }
 }
 
-/* NSUB > 0: the substep count is a compile-time constant (4 for the default
- * INTEGRATION_ORDER=4) and the slice is unrolled (the CSR slice kernel: 5 %
- * less time per kick); NSUB = 0 takes nSub from the element.  The same
- * operations in the same order either way. */
-template <bool RAD, int NSUB = 0>
+/* nSlices slices of nSub substeps; rolled, as for kmult */
+template <bool RAD>
 __device__ __forceinline__ int csbend_integrate(double &X, double &QX, double &Y, double &QY, double &dist,
-                                                double &DPoP, const double *c, int nSlices, int nSub_rt,
-                                                bool isr_block, const DevAperture *ap, const DevElem &e,
-                                                const RadSite &rs) {
+                                                double &DPoP, const double *c, int nSlices, int nSub, bool isr_block,
+                                                const DevAperture *ap, const DevElem &e, const RadSite &rs) {
   const double rho0 = c[CB_RHO0];
-  const int nSub = NSUB > 0 ? NSUB : nSub_rt;
   int lost;
   dist = 0;
   for (int i = 0; i < nSlices; i++) {
     if (!mult_aperture_ok(X, Y, ap, e))
       return LOSS_APERTURE;
-    if constexpr (NSUB > 0) {
-#pragma unroll
-      for (int j = 0; j < NSUB; j++) {
-        if ((lost = bend_drift(X, QX, Y, QY, dist, DPoP, rho0, c[CB_DSH0 + j])))
-          return lost;
-        if (j < NSUB - 1) /* kickFrac[last] == 0 ends the slice */
-          bend_kick<RAD>(X, Y, QX, QY, DPoP, c, i, j, nSub, isr_block, e, rs);
-      }
-    } else {
 #pragma unroll 1
-      for (int j = 0; j < nSub; j++) {
-        if ((lost = bend_drift(X, QX, Y, QY, dist, DPoP, rho0, c[CB_DSH0 + j])))
-          return lost;
-        if (j == nSub - 1) /* kickFrac[last] == 0 ends the slice */
-          break;
-        bend_kick<RAD>(X, Y, QX, QY, DPoP, c, i, j, nSub, isr_block, e, rs);
-      }
+    for (int j = 0; j < nSub; j++) {
+      if ((lost = bend_drift(X, QX, Y, QY, dist, DPoP, rho0, c[CB_DSH0 + j])))
+        return lost;
+      if (j == nSub - 1) /* kickFrac[last] == 0 ends the slice */
+        break;
+      bend_kick<RAD>(X, Y, QX, QY, DPoP, c, i, j, nSub, isr_block, e, rs);
     }
   }
   if (!mult_aperture_ok(X, Y, ap, e))
@@ -708,8 +693,6 @@ __device__ __forceinline__ int csbend(Part &p, const DevElem &e, const DevApertu
   Q2 = y;
   Q3 = yp * f;
 
-  /* rolled here: in the fused ring kernel the unrolled slice measured
-   * slower (register pressure); the CSR slice kernel takes the unrolled one */
   lost = csbend_integrate<RAD>(Q0, Q1, Q2, Q3, Q4, dp, c, nSlices, nSub, (e.flags & EF_RADBLOCK) != 0, ap, e, rs);
 
   /* convertFromDipoleCanonicalCoordinates (csbend.c:1421-1429) */

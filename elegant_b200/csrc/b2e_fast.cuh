@@ -8,9 +8,9 @@
  * A form returns false, and leaves the particle untouched, when anything
  * leaves the range it was written for: an aperture (or a place too near its
  * edge to tell cheaply), a coordinate, slope or angle limit, a loss, a
- * non-finite or extremely small value.  The caller then runs the general map from the element's
- * entrance, which finds the loss or the value; a particle pays for that once
- * or twice in its life.  Range tests compare the high words of the doubles on
+ * non-finite or extremely small value.  The caller then runs the general map
+ * from the element's entrance, which finds the loss or the value; a particle
+ * pays for that once or twice in its life.  Range tests compare the high words of the doubles on
  * the integer pipe.
  *
  * Why: the general maps spend about 180 FP64-pipe operations per bend drift
@@ -328,13 +328,12 @@ __device__ __forceinline__ void bend_drift_fast(double &X, double &QX, double &Y
  * radiation's formulas take it in inv_rho) delta changes inside every trip, and
  * A, 1/A and f with it. */
 enum BendTrip { TRIP_NONE, TRIP, TRIP_SR };
-template <BendTrip MODE, int NSUB = 0>
+template <BendTrip MODE>
 __device__ __forceinline__ bool bend_slices_fast(double &X, double &QX, double &Y, double &QY, double &dist, double &A,
-                                                 double inv_A, const double *c, int nSlices, int nSub_rt,
+                                                 double inv_A, const double *c, int nSlices, int nSub,
                                                  const DevAperture *ap, const DevElem &e, double *delta = nullptr,
                                                  double rad = 0, double inv_rho = 0) {
   const double rho0 = c[CB_RHO0];
-  const int nSub = NSUB > 0 ? NSUB : nSub_rt;
   double f, inv_f, DP = MODE == TRIP_SR ? *delta : 0;
   unsigned sin_max = 0;
   bool ok = bend_root(A, QY, f, inv_f), moves = MODE == TRIP;
@@ -342,7 +341,7 @@ __device__ __forceinline__ bool bend_slices_fast(double &X, double &QX, double &
   for (int i = 0; i < nSlices && ok; i++) {
     if (ap)
       ok = ap_inside(X, Y, ap, e);
-#pragma unroll(NSUB > 0 ? NSUB : 1)
+#pragma unroll 1
     for (int j = 0;; j++) {
       bend_drift_fast(X, QX, Y, QY, dist, A, f, inv_f, rho0, c[CB_DSH0 + j], sin_max);
       if (j == nSub - 1)

@@ -576,7 +576,7 @@ int b2e_selftest_rounding(int64_t samples, uint64_t seed, int64_t mismatches[4])
  * -1 = alive) through one CSRCSBEND, exactly as b2e_track does for that
  * element (same kernels, same results), writing the per-kick wakes
  * (N_KICKS x BINS values) to dev_wakes when it is non-NULL.  It allocates
- * nothing: all working memory is one static device array of ~10.2 MB in the
+ * nothing: all working memory is one static device array of ~8.5 MB in the
  * library image, for up to B2E_STATIC_MAX_PARTICLES particles and
  * B2E_STATIC_MAX_BINS bins; larger requests are rejected with B2E_ERR_ARG and
  * a message in errbuf.  The first call on a device is its set-up: with that
