@@ -581,46 +581,62 @@ B2E_SG_FN void sg_row(int half, int order, int deriv, int nb, int row, double *w
       w[k] = t[k];
 }
 
-__device__ void sg_apply(const double *in, double *out, int nb, int half, const double *w) {
+template <bool CLIP = false>
+__device__ __forceinline__ void sg_apply(const double *in, double *out, int nb, int half, const double *w) {
   const int width = sg_width(half, nb);
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     const int start = half <= 0 ? b : min(max(b - half, 0), nb - width);
     const double *wb = w + (b - start) * width;
     double s = 0;
-    for (int k = 0; k < width; k++)
-      s += wb[k] * in[start + k];
-    out[b] = s;
+    for (int k0 = 0; k0 < width; k0 += 8) {
+      double term[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (k0 + k < width)
+          term[k] = wb[k0 + k] * in[start + k0 + k];
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (k0 + k < width)
+          s += term[k];
+    }
+    out[b] = CLIP && s < 0 ? 0 : s;
   }
 }
 
-/* ((v[0] + v[1]) + v[2]) + ... in index order, as a serial loop forms it;
- * the next eight values load while the current eight are added */
+/* ((v[0] + v[1]) + v[2]) + ... in index order, as a serial loop forms it: one
+ * addition's latency a value (8.4 cycles), eight values loading while eight are
+ * added */
 __device__ __forceinline__ double ordered_sum(const double *v, int n) {
-  double s = 0;
+  double s = 0, r[8], q[8];
+  auto load = [&](double(&to)[8], int from) {
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (from + k < n)
+        to[k] = v[from + k];
+  };
+  auto add = [&](const double(&of)[8]) {
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      s += of[k];
+  };
   int b = 0;
-  if (n >= 8) {
-    double r[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-      r[k] = v[k];
-    for (b = 8; b + 8 <= n; b += 8) {
-      double q[8];
-#pragma unroll
-      for (int k = 0; k < 8; k++)
-        q[k] = v[b + k];
-#pragma unroll
-      for (int k = 0; k < 8; k++)
-        s += r[k];
-#pragma unroll
-      for (int k = 0; k < 8; k++)
-        r[k] = q[k];
-    }
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-      s += r[k];
+  load(r, 0);
+  for (; b + 16 <= n; b += 16) {
+    load(q, b + 8);
+    add(r);
+    load(r, b + 16);
+    add(q);
   }
-  for (; b < n; b++)
-    s += v[b];
+  /* r holds what is left of the next eight values */
+  load(q, b + 8);
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    if (b + k < n)
+      s += r[k];
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    if (b + 8 + k < n)
+      s += q[k];
   return s;
 }
 
@@ -647,93 +663,86 @@ __device__ __forceinline__ void stage_weights(WakeArgs &a, double (&stage)[2][SG
  * derivative filter and the (dct*b)^(1/3) denominators.  Leaves hist = sm,
  * deriv = sm + nBins, denom = sm + 2 nBins (tmp = sm + 3 nBins is scratch) and,
  * with INVERSE, 1/denom at sm + 4 nBins + 8; returns whether the quotients
- * deriv/denom may be formed with them (fp_quot): every value plain. */
+ * deriv/denom may be formed with them (fp_quot): every value plain.  `first` is
+ * this thread's first count, loaded ahead. */
 template <typename CountT, typename SumT, bool INVERSE = false>
-__device__ bool wake_filters(const CountT *counts, const WakeArgs &a, const double dct, double *sm, SumT *nbinned_out) {
-  const int nb = a.nBins;
+__device__ bool wake_filters(const CountT *counts, CountT first, const WakeArgs &a, const double dct, double *sm,
+                             SumT *nbinned_out) {
+  constexpr bool EXACT = std::is_integral<SumT>::value;
+  const int nb = a.nBins, warps = blockDim.x >> 5;
   double *inv = sm + 4 * nb + 8;
   double *hist = sm, *deriv = sm + nb, *denom = sm + 2 * nb, *tmp = sm + 3 * nb;
-  __shared__ double nBinnedD;
-  __shared__ int skip;
+  __shared__ double nBinnedD, smoothed_sum;
   __shared__ SumT warp_sums[32];
-  if constexpr (std::is_integral<SumT>::value) {
-    /* integer counts: the total is exact in any order, so it is a block
-     * reduction (per thread, warp shuffles, then the warps' totals) */
-    SumT part = 0;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-      const CountT v = counts[b];
-      hist[b] = (double)v;
+  const bool plain_dct = fp_within(dct, FP_HI_2M250, FP_HI_2P100);
+  const double inv_dct = fp_recip(dct);
+  /* the total of the counts: integers in any order (per thread, warp shuffles,
+   * then the last warp), real values in bin order as the reference's loop; it is
+   * needed from the second barrier on, so it forms beside the work in between */
+  SumT part = 0;
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
+    const CountT v = b == threadIdx.x ? first : counts[b];
+    hist[b] = (double)v;
+    if (EXACT)
       part += v;
-    }
+  }
+  if (EXACT) {
     for (int o = 16; o > 0; o >>= 1)
       part += __shfl_down_sync(0xffffffffu, part, o);
     if ((threadIdx.x & 31) == 0)
       warp_sums[threadIdx.x >> 5] = part;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      SumT s = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); w++)
-        s += warp_sums[w];
-      nBinnedD = 1.0 * s;
-      if (nbinned_out)
-        *nbinned_out = s;
-      skip = 0;
-    }
-  } else {
-    /* real-valued counts: summed in bin order, as the reference's loop */
-    for (int b = threadIdx.x; b < nb; b += blockDim.x)
-      hist[b] = (double)counts[b];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      SumT s = ordered_sum(hist, nb);
-      nBinnedD = 1.0 * s;
-      if (nbinned_out)
-        *nbinned_out = s;
-      skip = 0;
-    }
   }
   __syncthreads();
+  if (EXACT) {
+    if ((int)(threadIdx.x >> 5) == warps - 1) {
+      const int lane = threadIdx.x & 31;
+      SumT total = lane < warps ? warp_sums[lane] : 0;
+      for (int o = 16; o > 0; o >>= 1)
+        total += __shfl_down_sync(0xffffffffu, total, o);
+      if (lane == 0) {
+        nBinnedD = 1.0 * total;
+        if (nbinned_out)
+          *nbinned_out = total;
+      }
+    }
+  } else if (a.lh) {
+    if (threadIdx.x == 0)
+      nBinnedD = ordered_sum(hist, nb);
+    __syncthreads();
+  }
   if (a.lh)
     lh_pass_filters(a, sm);
   if (a.sgHalf > 0) {
-    sg_apply(hist, tmp, nb, a.sgHalf, a.sg_w);
+    /* correctDistribution (csbend.c:4705-4721): negative bins clipped as the
+     * smoothing writes them, then the sum in bin order, as the reference forms
+     * it */
+    sg_apply<true>(hist, tmp, nb, a.sgHalf, a.sg_w);
     __syncthreads();
-    /* correctDistribution (csbend.c:4705-4721): negative bins clipped in
-     * parallel, then the sum in bin order, as the reference forms it */
-    for (int b = threadIdx.x; b < nb; b += blockDim.x)
-      if (tmp[b] < 0)
-        tmp[b] = 0;
-    __syncthreads();
-    /* thread 0 runs the serial sum while warps 1.. form the denominators */
-    if (threadIdx.x == 0) {
-      const double sum = ordered_sum(tmp, nb);
-      if (!sum)
-        skip = 1;
-      else
-        deriv[0] = nBinnedD / sum; /* factor, parked in deriv[0] */
-    } else if (threadIdx.x >= 32) {
-      for (int b = threadIdx.x - 32; b < nb; b += blockDim.x - 32) {
+    /* thread 0 runs the serial sum, for real counts thread 32 that of the
+     * counts, and the warps behind them form the denominators */
+    const int helpers = EXACT ? 32 : 64;
+    if (threadIdx.x == 0)
+      smoothed_sum = ordered_sum(tmp, nb);
+    else if (!EXACT && !a.lh && threadIdx.x == 32)
+      nBinnedD = ordered_sum(hist, nb);
+    else if (threadIdx.x >= helpers)
+      for (int b = threadIdx.x - helpers; b < nb; b += blockDim.x - helpers) {
         const double v = b2e_pow13(dct * b);
         denom[b] = v;
         if (INVERSE)
           inv[b] = fp_recip(v);
       }
-    }
     __syncthreads();
-    const double factor = deriv[0];
-    const int sk = skip;
-    __syncthreads();
-    for (int b = threadIdx.x; b < nb; b += blockDim.x)
-      hist[b] = sk ? tmp[b] : tmp[b] * factor;
   }
-  const bool denom_done = a.sgHalf > 0 && blockDim.x > 32;
+  const double sum = a.sgHalf > 0 ? smoothed_sum : 0, factor = a.sgHalf > 0 ? nBinnedD / sum : 0;
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    if (!denom_done) {
+    if (a.sgHalf <= 0) {
       denom[b] = b2e_pow13(dct * b);
       if (INVERSE)
         inv[b] = fp_recip(denom[b]);
     }
-    hist[b] = hist[b] / dct;
+    const double h = a.sgHalf > 0 ? (sum == 0 ? tmp[b] : tmp[b] * factor) : hist[b];
+    hist[b] = plain_dct && fp_plain(h, FP_HI_2P700) ? fp_quot(h, dct, inv_dct) : divide_ieee(h, dct);
   }
   __syncthreads();
   sg_apply(hist, deriv, nb, a.sgdHalf, a.sgd_w);
@@ -909,10 +918,10 @@ __device__ void igf_wake(const WakeArgs &a, const double dct, const double *hist
  * smoothed density (per unit ct) and its derivative when hist_out/deriv_out
  * are set. */
 template <typename CountT, typename SumT, int NI>
-__device__ void wake_body(const CountT *counts, const WakeArgs &a, const double dct, double *sm, double *dgamma,
+__device__ void wake_body(const CountT *counts, CountT first, const WakeArgs &a, const double dct, double *sm, double *dgamma,
                           SumT *nbinned_out, double *hist_out, double *deriv_out, double *page = nullptr) {
   const int nb = a.nBins;
-  const bool inverse = wake_filters<CountT, SumT, true>(counts, a, dct, sm, nbinned_out);
+  const bool inverse = wake_filters<CountT, SumT, true>(counts, first, a, dct, sm, nbinned_out);
   const double *hist = sm, *deriv = sm + nb, *denom = sm + 2 * nb, *inv = sm + 4 * nb + 8;
   double *page_t1 = page ? page + 2 * nb : nullptr, *page_t2 = page ? page + 3 * nb : nullptr;
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
@@ -986,8 +995,11 @@ __global__ void __launch_bounds__(1024, 1) csr_wake_kernel(CsrBunches B, unsigne
   stage_weights(a, stage);
   chain_wait();
   const int bunch = blockIdx.x;
-  /* the bunch's scalars load together with its active flag (all in bounds) */
+  /* the bunch's scalars and the first counts load together with its active
+   * flag (all in bounds) */
   const int active = B.active[bunch];
+  unsigned int *counts = counts_all + (size_t)bunch * a.nBins;
+  const unsigned int first = threadIdx.x < a.nBins ? counts[threadIdx.x] : 0;
   const double csr_constant = B.csr_const[bunch], igf_factor = B.csr_const[B.n + bunch];
   CsrDevState *st = B.st + bunch;
   const double dct = st->dct;
@@ -1027,8 +1039,7 @@ __global__ void __launch_bounds__(1024, 1) csr_wake_kernel(CsrBunches B, unsigne
   w.c2 = -csr_constant * a.length / a.nSlices / a.slippage13;
   w.igf_factor = igf_factor;
   w.wakelog = a.wakelog ? a.wakelog + (size_t)bunch * a.nBins : nullptr;
-  unsigned int *counts = counts_all + (size_t)bunch * a.nBins;
-  wake_body<unsigned int, long long, 1>(counts, w, dct, sm, st->dGamma, &st->nBinned, nullptr, nullptr, page);
+  wake_body<unsigned int, long long, 1>(counts, first, w, dct, sm, st->dGamma, &st->nBinned, nullptr, nullptr, page);
   if (recycle) /* the counts were copied to shared memory before the first barrier */
     for (int b = threadIdx.x; b < a.nBins; b += blockDim.x)
       counts[b] = 0;
@@ -1068,7 +1079,8 @@ __global__ void __launch_bounds__(1024, 1) csr_sur_filter_kernel(CsrBunches B, c
   }
   CsrDevState *st = B.st + b;
   const double dct = st->dct;
-  wake_filters<unsigned int, long long>(counts_all + (size_t)b * nb, a, dct, sm, &st->nBinned);
+  const unsigned int *counts = counts_all + (size_t)b * nb;
+  wake_filters<unsigned int, long long>(counts, threadIdx.x < nb ? counts[threadIdx.x] : 0, a, dct, sm, &st->nBinned);
   const double *hist = sm, *deriv = sm + nb, *denom = sm + 2 * nb;
   double *red = sm + 3 * nb;
   double *t = tab + (size_t)b * 3 * B2E_CSR_MAX_BINS;
@@ -1196,7 +1208,7 @@ constexpr int BATCH_THREADS = 256, BATCH_BINS = 4;
 struct SgTables {
   double w[2][SG_STAGE];
 };
-__global__ void __launch_bounds__(BATCH_THREADS)
+__global__ void __launch_bounds__(BATCH_THREADS, 3)
     wake_batch_kernel(const double *counts, const double *slippage_bins, WakeArgs a, const __grid_constant__ SgTables sg,
                       double *t1_out, double *hist_out, double *deriv_out) {
   extern __shared__ double sm[];
@@ -1214,7 +1226,7 @@ __global__ void __launch_bounds__(BATCH_THREADS)
   w.c2 = 0;
   w.csr_constant = 1;
   w.wakelog = nullptr;
-  wake_body<double, double, BATCH_BINS>(counts + off, w, 1.0, sm, t1_out + off, (double *)nullptr, hist_out + off,
+  wake_body<double, double, BATCH_BINS>(counts + off, threadIdx.x < a.nBins ? counts[off + threadIdx.x] : 0, w, 1.0, sm, t1_out + off, (double *)nullptr, hist_out + off,
                                         deriv_out + off);
 }
 
@@ -1535,7 +1547,8 @@ __global__ void __launch_bounds__(1024, 1) stupakov_wake_kernel(CsrBunches B, co
   CsrDevState *st = B.st + bunch;
   const int nb = a.nBins;
   const double dct = st->dct;
-  wake_filters<unsigned int, unsigned long long>(counts_all + (size_t)bunch * nb, a, dct, sm, nullptr);
+  const unsigned int *counts = counts_all + (size_t)bunch * nb;
+  wake_filters<unsigned int, unsigned long long>(counts, threadIdx.x < nb ? counts[threadIdx.x] : 0, a, dct, sm, nullptr);
   const double *hist = sm, *deriv = sm + nb;
   double *phi = sm + 4 * nb + 8;
   if (!(dct > 0)) {
