@@ -784,16 +784,9 @@ static int track_impl(b2e_ctx *ctx, double *effort) {
       if (rc)
         return rc;
     } else {
-      /* the collective step needs the number of particles alive at its entrance
-       * (n_part > 1 decides whether CSR is computed at all, csbend.c:1987) */
-      std::vector<int64_t> alive;
       ctx->csr.d_offsets = ctx->d_inst_offsets.ptr;
-      int rc = csr_count_alive(ctx->csr, particle_view(ctx).lost_pass, ctx->n, alive, ctx->stream, ctx->err);
-      if (rc)
-        return rc;
-      ctx->launches++;
-      rc = csr_track_element(ctx->csr, ctx->d_elems.ptr, ctx->lat.elems[stop_e], particle_view(ctx), ctx->n, alive,
-                             stop_e, p, ctx->stream, ctx->err, &ctx->launches);
+      int rc = csr_track_element(ctx->csr, ctx->d_elems.ptr, ctx->lat.elems[stop_e], particle_view(ctx), ctx->n, stop_e,
+                                 p, ctx->stream, ctx->err, &ctx->launches);
       if (rc)
         return rc;
       const int iap = p == 0 ? ctx->lat.elems[stop_e].ap_pass0 : ctx->lat.elems[stop_e].ap_later;

@@ -1877,6 +1877,9 @@ int csr_set_bunches(CsrState &st, int n_bunches, const int64_t *d_offsets, std::
     cudaFree(st.d_flags);
   if (st.d_alive)
     cudaFree(st.d_alive);
+  if (st.h_alive)
+    cudaFreeHost(st.h_alive);
+  st.h_alive = nullptr;
   if (st.d_keys)
     cudaFree(st.d_keys);
   st.d_keys = nullptr;
@@ -1894,7 +1897,9 @@ int csr_set_bunches(CsrState &st, int n_bunches, const int64_t *d_offsets, std::
       cudaMalloc(&st.d_csr_const, 4 * sizeof(double) * n_bunches) != cudaSuccess ||
       cudaMalloc(&st.d_flags, 2 * n_bunches) != cudaSuccess ||
       cudaMalloc(&st.d_alive, sizeof(unsigned long long) * n_bunches) != cudaSuccess ||
-      cudaMalloc(&st.d_keys, 2 * sizeof(unsigned long long) * n_bunches) != cudaSuccess) {
+      cudaMalloc(&st.d_keys, 2 * sizeof(unsigned long long) * n_bunches) != cudaSuccess ||
+      cudaMallocHost(&st.h_alive, sizeof(unsigned long long) * n_bunches) != cudaSuccess ||
+      (!st.alive_known && cudaEventCreateWithFlags(&st.alive_known, cudaEventDisableTiming) != cudaSuccess)) {
     err = "CSR state allocation failed";
     return B2E_ERR_NOMEM;
   }
@@ -1924,10 +1929,35 @@ __global__ void alive_per_bunch_kernel(const int32_t *lost_pass, int64_t n, cons
     atomicAdd(&alive[b], c);
 }
 
-int csr_count_alive(CsrState &st, const int32_t *lost_pass, int64_t n, std::vector<int64_t> &alive, cudaStream_t stream,
-                    std::string &err) {
+/* What an element's kernels do per bunch, from the particles alive at its
+ * entrance (n_part > 1 decides whether CSR is computed, csbend.c:1987,
+ * :3196-3212): a bend's active flags with the constants of the others at zero
+ * and empty range keys and counts (one block per bunch), or a drift's mode
+ * flags out of the candidates that the host has copied there.  The counts go
+ * to the host's memory as well. */
+__global__ void csr_begin_kernel(CsrBunches B, const unsigned long long *alive, int drift, double *csr_const,
+                                 unsigned int *counts, int nBins, unsigned long long *host_alive) {
+  const int b = blockIdx.x;
+  const bool some = alive[b] > 1;
+  if (threadIdx.x == 0) {
+    unsigned char *active = const_cast<unsigned char *>(B.active), *mode = const_cast<unsigned char *>(B.mode);
+    host_alive[b] = alive[b];
+    active[b] = !drift && some;
+    mode[b] = drift && some && mode[b];
+    if (!drift) {
+      if (!some)
+        csr_const[b] = csr_const[2 * B.n + b] = 0;
+      B.st[b].ct_min_key = ~0ull;
+      B.st[b].ct_max_key = 0ull;
+    }
+  }
+  if (!drift)
+    for (int k = threadIdx.x; k < nBins; k += blockDim.x)
+      counts[(size_t)b * nBins + k] = 0;
+}
+
+static int count_alive(CsrState &st, const int32_t *lost_pass, int64_t n, cudaStream_t stream, std::string &err) {
   const int nb = st.n_bunches;
-  std::vector<unsigned long long> h(nb);
   if (cudaMemsetAsync(st.d_alive, 0, sizeof(unsigned long long) * nb, stream) != cudaSuccess) {
     err = "CSR: alive count failed";
     return B2E_ERR_CUDA;
@@ -1938,14 +1968,31 @@ int csr_count_alive(CsrState &st, const int32_t *lost_pass, int64_t n, std::vect
     err = "CSR: the all-rank reduction of alive counts failed";
     return B2E_ERR_CUDA;
   }
-  if (cudaGetLastError() != cudaSuccess ||
-      cudaMemcpyAsync(h.data(), st.d_alive, sizeof(unsigned long long) * nb, cudaMemcpyDeviceToHost, stream) !=
-          cudaSuccess ||
-      cudaStreamSynchronize(stream) != cudaSuccess) {
+  if (cudaGetLastError() != cudaSuccess) {
     err = "CSR: alive count failed";
     return B2E_ERR_CUDA;
   }
-  alive.assign(h.begin(), h.end());
+  return B2E_OK;
+}
+
+/* launches csr_begin_kernel and marks the place from which h_alive holds the
+ * counts (await_alive) */
+static int begin_element(CsrState &st, const CsrBunches &B, int drift, int bins, cudaStream_t stream,
+                         std::string &err, int64_t *launches) {
+  csr_begin_kernel<<<B.n, 256, 0, stream>>>(B, st.d_alive, drift, st.d_csr_const, st.d_counts, bins, st.h_alive);
+  (*launches)++;
+  if (cudaGetLastError() != cudaSuccess || cudaEventRecord(st.alive_known, stream) != cudaSuccess) {
+    err = "CSR: alive count failed";
+    return B2E_ERR_CUDA;
+  }
+  return B2E_OK;
+}
+
+static int await_alive(CsrState &st, std::string &err) {
+  if (cudaEventSynchronize(st.alive_known) != cudaSuccess) {
+    err = "CSR: alive count failed";
+    return B2E_ERR_CUDA;
+  }
   return B2E_OK;
 }
 
@@ -1995,15 +2042,20 @@ void csr_reset(CsrState &st) {
   st.last_bend = -1;
 }
 
-static int ensure_pagelog(CsrState &st, int64_t values) {
+static int ensure_pagelog(CsrState &st, int64_t values, cudaStream_t stream) {
   if (values <= st.pagelog_cap)
     return B2E_OK;
   double *p = nullptr;
   if (cudaMalloc(&p, sizeof(double) * values) != cudaSuccess)
     return B2E_ERR_NOMEM;
   if (st.d_pagelog) {
-    if (st.page_values)
-      cudaMemcpy(p, st.d_pagelog, sizeof(double) * st.page_values, cudaMemcpyDeviceToDevice);
+    /* behind the kernels that still write the old log */
+    if ((st.page_values && cudaMemcpyAsync(p, st.d_pagelog, sizeof(double) * st.page_values, cudaMemcpyDeviceToDevice,
+                                           stream) != cudaSuccess) ||
+        cudaStreamSynchronize(stream) != cudaSuccess) {
+      cudaFree(p);
+      return B2E_ERR_NOMEM;
+    }
     cudaFree(st.d_pagelog);
   }
   st.d_pagelog = p;
@@ -2011,15 +2063,20 @@ static int ensure_pagelog(CsrState &st, int64_t values) {
   return B2E_OK;
 }
 
-static int ensure_wakelog(CsrState &st, int64_t values) {
+static int ensure_wakelog(CsrState &st, int64_t values, cudaStream_t stream) {
   if (values <= st.wakelog_cap)
     return B2E_OK;
   double *p = nullptr;
   if (cudaMalloc(&p, sizeof(double) * values) != cudaSuccess)
     return B2E_ERR_NOMEM;
   if (st.d_wakelog) {
-    if (st.wake_values)
-      cudaMemcpy(p, st.d_wakelog, sizeof(double) * st.wake_values, cudaMemcpyDeviceToDevice);
+    /* behind the kernels that still write the old log */
+    if ((st.wake_values && cudaMemcpyAsync(p, st.d_wakelog, sizeof(double) * st.wake_values, cudaMemcpyDeviceToDevice,
+                                           stream) != cudaSuccess) ||
+        cudaStreamSynchronize(stream) != cudaSuccess) {
+      cudaFree(p);
+      return B2E_ERR_NOMEM;
+    }
     cudaFree(st.d_wakelog);
   }
   st.d_wakelog = p;
@@ -2184,17 +2241,16 @@ static int stupakov_drift(CsrState &st, const CsrElem &ce, const CsrBunches &B, 
 }
 
 int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_elem, const DevParticles &P, int64_t n,
-                      const std::vector<int64_t> &alive, int elem, int pass, cudaStream_t stream, std::string &err,
-                      int64_t *launches) {
+                      int elem, int pass, cudaStream_t stream, std::string &err, int64_t *launches) {
+  const int count_rc = count_alive(st, P.lost_pass, n, stream, err);
+  if (count_rc)
+    return count_rc;
+  (*launches)++;
   size_t k = 0;
   while (k < st.elems.size() && st.elems[k].index != elem)
     k++;
   if (k == st.elems.size()) {
     err = "CSR element not configured";
-    return B2E_ERR_STATE;
-  }
-  if ((int)alive.size() != st.n_bunches) {
-    err = "CSR: per-bunch alive counts do not match the bunch layout";
     return B2E_ERR_STATE;
   }
   const CsrElem &ce = st.elems[k];
@@ -2215,8 +2271,23 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
      * an exact drift (csbend.c:3196-3212) */
     bool any = false;
     for (int b = 0; b < nbunch; b++) {
-      flags[nbunch + b] = alive[b] > 1 && st.wake_valid[b] && ce.drift_csr;
+      flags[nbunch + b] = st.wake_valid[b] && ce.drift_csr;
       any = any || flags[nbunch + b];
+    }
+    /* the flags are settled on the device; what the host needs of them is
+     * whether an invalid number of kicks is an error */
+    if (any) {
+      CSR_CUDA(cudaMemcpyAsync(st.d_flags, flags.data(), flags.size(), cudaMemcpyHostToDevice, stream));
+      const int rc = begin_element(st, B, 1, 0, stream, err, launches);
+      if (rc)
+        return rc;
+      if (!(ce.drift_dz > 0) && ce.drift_kicks <= 0) {
+        if (await_alive(st, err))
+          return B2E_ERR_CUDA;
+        any = false;
+        for (int b = 0; b < nbunch; b++)
+          any = any || (flags[nbunch + b] && st.h_alive[b] > 1);
+      }
     }
     if (!any) {
       CsrBunches all = B;
@@ -2226,15 +2297,9 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
       CSR_CUDA(cudaGetLastError());
       return B2E_OK;
     }
-    CSR_CUDA(cudaMemcpyAsync(st.d_flags, flags.data(), flags.size(), cudaMemcpyHostToDevice, stream));
-    bool some_plain = false;
-    for (int b = 0; b < nbunch; b++)
-      some_plain = some_plain || !flags[nbunch + b];
-    if (some_plain) {
-      edrift_kernel<<<g, 256, 0, stream>>>(P, n, ce.drift_length, B, 0);
-      (*launches)++;
-      CSR_CUDA(cudaGetLastError());
-    }
+    CSR_CUDA(launch_chained(edrift_kernel, dim3(g), dim3(256), 0, stream, P, n, ce.drift_length, B, 0));
+    (*launches)++;
+    CSR_CUDA(cudaGetLastError());
     double zStart = ce.z_start;
     /* a drift behind the previous pass's dipole (csbend.c:3251-3255) */
     for (int guard = 0; zStart + 1e-12 < st.zLast && st.revolution_length > 0 && guard < (1 << 20); guard++)
@@ -2279,11 +2344,6 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
 
   /* ---- CSRCSBEND ---- */
   const DevElem *d_e = d_elems + elem;
-  bool any_active = false;
-  for (int b = 0; b < nbunch; b++) {
-    flags[b] = alive[b] > 1; /* csbend.c:1987 */
-    any_active = any_active || flags[b];
-  }
   if (!ce.same_bend_precedes)
     st.accumulated_angle = 0;
   st.wake_valid.assign(nbunch, 0);
@@ -2296,12 +2356,12 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
     }
     st.beta0_cap = n;
   }
-  if (ensure_wakelog(st, st.wake_values + (int64_t)ce.nSlices * ce.bins * nbunch)) {
+  if (ensure_wakelog(st, st.wake_values + (int64_t)ce.nSlices * ce.bins * nbunch, stream)) {
     err = "CSR wake log allocation failed";
     return B2E_ERR_NOMEM;
   }
   const int64_t page_stride = B2E_CSR_PAGE_HEADER + 4 * (int64_t)ce.bins;
-  if (st.record_pages && ensure_pagelog(st, st.page_values + (int64_t)ce.nSlices * nbunch * page_stride)) {
+  if (st.record_pages && ensure_pagelog(st, st.page_values + (int64_t)ce.nSlices * nbunch * page_stride, stream)) {
     err = "CSR page record allocation failed";
     return B2E_ERR_NOMEM;
   }
@@ -2311,7 +2371,7 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
   const double eps0 = 1 / ((4 * kPI * 1e-7) * kC * kC);
   std::vector<double> csr_constant(4 * nbunch, 0.0);
   for (int b = 0; b < nbunch; b++) {
-    if (ce.csr && flags[b])
+    if (ce.csr) /* zeroed by csr_begin_kernel where one particle or none is alive */
       csr_constant[b] = 2 * st.macro_charge[b] * kE / b2e_pow(3 * ce.rho0 * ce.rho0, 1. / 3.) /
                         (4 * kPI * eps0 * kME * (kC * kC));
     /* the IGF wake's factor (csbend.c:2678-2679) */
@@ -2323,37 +2383,47 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
   }
   CSR_CUDA(cudaMemcpyAsync(st.d_csr_const, csr_constant.data(), 4 * sizeof(double) * nbunch, cudaMemcpyHostToDevice,
                            stream));
-  CSR_CUDA(cudaMemcpyAsync(st.d_flags, flags.data(), flags.size(), cudaMemcpyHostToDevice, stream));
+  if (int rc = begin_element(st, B, 0, ce.bins, stream, err, launches))
+    return rc;
   const double *sgw = st.d_sg + st.sg_offset[k];
   const size_t wake_smem = sizeof(double) * (5 * ce.bins + 8);
   CSR_CUDA(cudaFuncSetAttribute(csr_wake_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wake_smem));
-  /* learned wake: trained on the transient integral with trapezoid rule (the
-   * CSRCSBEND defaults); other settings, or a bunch train larger than the
-   * network's batch, use the plain integral */
-  const bool use_net = st.net && any_active && !ce.steady && ce.trapz && !ce.lh && ce.bins <= wakenet_bins(st.net) &&
-                       nbunch <= wakenet_max_batch(st.net);
+  /* the host learns which bunches are active once the entry and the first
+   * slice are on their way: the device works on while it waits */
+  bool any_active = false, use_net = false, recycle = false;
   const size_t sur_smem = sizeof(double) * (3 * ce.bins + 1024);
-  if (use_net) {
-    int rc = ensure_surrogate_buffers(st, (int64_t)ce.nSlices * nbunch, err);
-    if (rc)
-      return rc;
-    CSR_CUDA(cudaFuncSetAttribute(csr_sur_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)std::max(sur_smem, sizeof(double) * (4 * ce.bins + 1024))));
-    CSR_CUDA(cudaFuncSetAttribute(csr_sur_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sur_smem));
-  }
-
+  auto settle = [&]() -> int {
+    if (await_alive(st, err))
+      return B2E_ERR_CUDA;
+    for (int b = 0; b < nbunch; b++) {
+      flags[b] = st.h_alive[b] > 1; /* csbend.c:1987 */
+      any_active = any_active || flags[b];
+    }
+    /* learned wake: trained on the transient integral with trapezoid rule (the
+     * CSRCSBEND defaults); other settings, or a bunch train larger than the
+     * network's batch, use the plain integral */
+    use_net = st.net && any_active && !ce.steady && ce.trapz && !ce.lh && ce.bins <= wakenet_bins(st.net) &&
+              nbunch <= wakenet_max_batch(st.net);
+    if (use_net) {
+      int rc = ensure_surrogate_buffers(st, (int64_t)ce.nSlices * nbunch, err);
+      if (rc)
+        return rc;
+      CSR_CUDA(cudaFuncSetAttribute(csr_sur_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)std::max(sur_smem, sizeof(double) * (4 * ce.bins + 1024))));
+      CSR_CUDA(cudaFuncSetAttribute(csr_sur_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sur_smem));
+    }
+    /* on the plain-integral path the wake kernel empties the range keys and the
+     * counts for the next kick; otherwise both are reset before every kick */
+    recycle = any_active && !use_net;
+    return B2E_OK;
+  };
   CSR_CUDA(launch_chained(csr_entry_kernel, dim3(g), dim3(256), 0, stream, P, n, st.d_beta0, d_e, ce.bx, Po));
   (*launches)++;
   CSR_CUDA(cudaGetLastError());
   double phiBend = st.accumulated_angle;
-  /* on the plain-integral path the wake kernel empties the range keys and the
-   * counts for the next kick; otherwise both are reset before every kick */
-  const bool recycle = any_active && !use_net;
-  if (recycle)
-    CSR_CUDA(cudaMemsetAsync(st.d_counts, 0, sizeof(unsigned int) * ce.bins * nbunch, stream));
   for (int kick = 0; kick < ce.nSlices; kick++) {
-    if (!recycle || kick == 0) {
+    if (!recycle && kick > 0) {
       csr_reset_keys_kernel<<<1, 32, 0, stream>>>(B);
       (*launches)++;
     }
@@ -2363,12 +2433,15 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
                             (const double *)st.d_beta0, h_elem, B, (int)(kick > 0), ce.bins, Po, 1 / Po, pass, elem));
     (*launches)++;
     CSR_CUDA(cudaGetLastError());
+    if (kick == 0)
+      if (int rc = settle())
+        return rc;
     if (!any_active)
       continue;
     int rrc = reduce_keys(st, B, stream, err, launches);
     if (rrc)
       return rrc;
-    if (!recycle)
+    if (!recycle && kick > 0)
       CSR_CUDA(cudaMemsetAsync(st.d_counts, 0, sizeof(unsigned int) * ce.bins * nbunch, stream));
     int64_t per = (n + nbunch - 1) / nbunch;
     int hb = hist_blocks(per, nbunch);
@@ -2460,6 +2533,9 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
     if (a.pagelog)
       st.page_values += nbunch * page_stride;
   }
+  if (ce.nSlices <= 0)
+    if (int rc = settle())
+      return rc;
   if (!recycle || ce.nSlices <= 0) {
     csr_reset_keys_kernel<<<1, 32, 0, stream>>>(B);
     (*launches)++;
@@ -2549,6 +2625,12 @@ void csr_release(CsrState &st) {
     cudaFree(st.d_flags);
   if (st.d_alive)
     cudaFree(st.d_alive);
+  if (st.h_alive)
+    cudaFreeHost(st.h_alive);
+  st.h_alive = nullptr;
+  if (st.alive_known)
+    cudaEventDestroy(st.alive_known);
+  st.alive_known = nullptr;
   if (st.d_keys)
     cudaFree(st.d_keys);
   st.d_keys = nullptr;

@@ -63,6 +63,8 @@ struct CsrState {
   double *d_csr_const = nullptr;  /* [4][n_bunches]: CSRConstant, IGF wake factor, GSConstant, macro charge */
   unsigned char *d_flags = nullptr; /* [2][n_bunches]: active, CSRDRIFT mode */
   unsigned long long *d_alive = nullptr; /* [n_bunches] */
+  unsigned long long *h_alive = nullptr; /* the same in host memory once alive_known has passed */
+  cudaEvent_t alive_known = nullptr;
   /* optional all-rank reduction (a bunch spread over several GPUs) */
   b2e_reduce_fn reducer = nullptr;
   void *reducer_user = nullptr;
@@ -116,13 +118,9 @@ void csr_reset(CsrState &st);
 int csr_set_bunches(CsrState &st, int n_bunches, const int64_t *d_offsets, std::string &err);
 /* all-rank sums of per-bunch counts (identity without a reducer) */
 int csr_reduce_counts(CsrState &st, std::vector<int64_t> &counts, cudaStream_t stream, std::string &err);
-/* particles alive (lost_pass < 0), per bunch */
-int csr_count_alive(CsrState &st, const int32_t *lost_pass, int64_t n, std::vector<int64_t> &alive, cudaStream_t stream,
-                    std::string &err);
-/* alive: particles alive at the element entrance, per bunch */
+/* one CSRCSBEND or CSRDRIFT; counts the particles alive at its entrance */
 int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_elem, const DevParticles &P, int64_t n,
-                      const std::vector<int64_t> &alive, int elem, int pass, cudaStream_t stream, std::string &err,
-                      int64_t *launches);
+                      int elem, int pass, cudaStream_t stream, std::string &err, int64_t *launches);
 int csr_copy_wakes(CsrState &st, double *wakes, int64_t capacity, int64_t *written, std::string &err);
 int csr_copy_pages(CsrState &st, double *pages, int64_t capacity, int64_t *written, std::string &err);
 /* total device time of the timed wake stages of the last run, and the kicks
