@@ -127,19 +127,20 @@ __global__ void __launch_bounds__(128, 1)
  * Persistent, warp-specialised implicit-GEMM convolution, one 128-bin tile
  * of one profile per accumulator:
  *   warp 0   TMA producer: the 5 weight taps once, then per tile the 5
- *            shifted 128x64 activation boxes through a WN_STAGES-deep ring;
+ *            shifted 128x64 activation boxes through a ring of conv_stages;
  *   warp 1   one thread issues UMMA 128x64x16 (4 per tap, 20 per tile) into
  *            one of two TMEM accumulators and commits to free the stage;
  *   warps 2-17 epilogue: TMEM -> registers (warp w reads lanes 32*(w%4)..;
  *            four warps per lane quadrant, 16 of the 64 channels each),
  *            bias + GELU (hidden), output channel 0 (output), or times
  *            GELU'(z) of the previous layer (backward data), BF16.
- *            The erf/exp of GELU and GELU' bound the epilogue: with 32
- *            channels per warp, 16 epilogue warps per SM, the issue slots were
- *            48 % busy; 16 channels need few enough registers (56) for 32
- *            warps.  A thread's 16 channels are one 32-byte sector, moved by
- *            one 256-bit access; in 16-byte pieces each sector was written
- *            twice.
+ *            The erf/exp of GELU bound the forward epilogue: with 32 channels
+ *            per warp, 16 epilogue warps per SM, the issue slots were 48 %
+ *            busy; 16 channels need few enough registers (56) for 32 warps.
+ *            Backward, GELU' of the BF16 z comes from a table: 39 -> 33 us for
+ *            256 profiles, now bound by the latency of z and of the boxes.  A
+ *            thread's 16 channels are one 32-byte sector, moved by one 256-bit
+ *            access; in 16-byte pieces each sector was written twice.
  * Bounded waits everywhere; a timeout sets the status word and every role
  * leaves its loop. */
 constexpr int CONV_EPI_WARPS = 16;
@@ -147,11 +148,42 @@ constexpr int CONV_THREADS = 64 + 32 * CONV_EPI_WARPS;
 constexpr int WG_THREADS = 192;
 constexpr size_t CONV_W_BYTES = (size_t)WN_TAPS * 64 * 128;  /* 40 KB */
 constexpr size_t CONV_STAGE_BYTES = 128 * 128;               /* 16 KB */
-constexpr size_t CONV_SMEM = 1024 + CONV_W_BYTES + WN_STAGES * CONV_STAGE_BYTES;
+/* GELU' at every BF16 value with 2^-25 <= |z| < 8, per sign, behind one entry
+ * for the smaller ones, where both terms round to 1/2: the backward epilogue's z
+ * is BF16, so this table in shared memory holds the floats that the formula
+ * gives.  It takes the place of two stages; four boxes in flight per SM are
+ * enough.  Most z of an untrained network are tiny (profile tails), and a warp
+ * takes the formula if one of its 512 values needs it, so the range matters:
+ * from 2^-14 on, half of the gain was gone. */
+constexpr int GG_LOW = (127 - 25) << 7, GG_N = 28 * 128;
+constexpr int GG_FLOATS = (2 * (GG_N + 1) + 3) / 4 * 4;
+constexpr size_t GG_BYTES = sizeof(float) * GG_FLOATS;
+__host__ __device__ constexpr int conv_stages(int epi) { return epi == EPI_BWD ? 2 : WN_STAGES; }
+__host__ __device__ constexpr size_t conv_smem(int epi) {
+  return 1024 + CONV_W_BYTES + conv_stages(epi) * CONV_STAGE_BYTES + (epi == EPI_BWD ? GG_BYTES : 0);
+}
 
 __device__ __forceinline__ float gelu_f(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_grad_f(float z) {
   return 0.5f * (1.f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
+}
+
+__device__ __forceinline__ float bf16_value(unsigned h) { return __uint_as_float(h << 16); }
+__global__ void gelu_grad_table_kernel(float *table) {
+  for (int i = threadIdx.x; i < GG_FLOATS; i += blockDim.x) {
+    const int sign = i > GG_N, k = i - sign * (GG_N + 1);
+    table[i] = k <= GG_N ? gelu_grad_f(bf16_value(sign << 15 | (k > 0 ? GG_LOW + k - 1 : 0))) : 0.f;
+  }
+}
+cudaError_t launch_gelu_grad_table(float *table, cudaStream_t s) {
+  gelu_grad_table_kernel<<<1, 1024, 0, s>>>(table);
+  return cudaGetLastError();
+}
+/* GELU' at the BF16 value h; sets beyond from |z| = 8 on */
+__device__ __forceinline__ float gelu_grad_at(const float *table, unsigned h, bool &beyond) {
+  const int k = (int)(h & 0x7fff) - (GG_LOW - 1);
+  beyond = beyond || k > GG_N;
+  return table[(h >> 15) * (GG_N + 1) + min(max(k, 0), GG_N)];
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
@@ -208,7 +240,9 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
   unsigned char *sm = (unsigned char *)(((uintptr_t)dsm + 1023) & ~(uintptr_t)1023);
   unsigned char *sw = sm;
   unsigned char *sa = sm + CONV_W_BYTES;
-  __shared__ __align__(8) uint64_t full[WN_STAGES], empty[WN_STAGES], tfull[2], tempty[2], wbar;
+  constexpr int STAGES = conv_stages(EPI);
+  float *gelu_grad = (float *)(sa + STAGES * CONV_STAGE_BYTES);
+  __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], tfull[2], tempty[2], wbar;
   __shared__ uint32_t tmem_base;
   __shared__ float sbias[64];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -218,7 +252,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
   constexpr uint32_t IDESC = umma::idesc_bf16(128, N, false, false);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < WN_STAGES; i++) {
+    for (int i = 0; i < STAGES; i++) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
@@ -238,9 +272,11 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
       /* the weights are older than any kernel of the pass */
       prefetch_tmap(&t_in);
       prefetch_tmap(&t_w);
-      mbar_expect_tx(&wbar, (uint32_t)CONV_W_BYTES);
+      mbar_expect_tx(&wbar, (uint32_t)(CONV_W_BYTES + (EPI == EPI_BWD ? GG_BYTES : 0)));
       for (int t = 0; t < WN_TAPS; t++)
         tma_load_3d(sw + t * 8192, &t_w, &wbar, 0, t * 64, 0);
+      if (EPI == EPI_BWD)
+        bulk_load(gelu_grad, a.gelu_grad, (uint32_t)GG_BYTES, &wbar);
     }
     __syncwarp();
   }
@@ -257,8 +293,8 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
         const int b = tile / tpp, l0 = (tile - b * tpp) << 7;
         for (int t = 0; t < WN_TAPS; t++, it++) {
-          const int s = it % WN_STAGES;
-          if (!mbar_wait(&empty[s], ((it / WN_STAGES) & 1) ^ 1, a.status, ST_TIMEOUT_TMA)) {
+          const int s = it % STAGES;
+          if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, a.status, ST_TIMEOUT_TMA)) {
             ok = false;
             break;
           }
@@ -267,8 +303,8 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
         }
       }
       /* let the copies still in flight land before the block can exit */
-      for (uint32_t k = it > WN_STAGES ? it - WN_STAGES : 0; k < it; k++)
-        mbar_wait(&full[k % WN_STAGES], (k / WN_STAGES) & 1, nullptr, 0);
+      for (uint32_t k = it > STAGES ? it - STAGES : 0; k < it; k++)
+        mbar_wait(&full[k % STAGES], (k / STAGES) & 1, nullptr, 0);
       mbar_wait(&wbar, 0, nullptr, 0);
     }
   } else if (warp == 1) {
@@ -285,8 +321,8 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
         tc_fence_after();
         const uint32_t d = tmem + acc * 64;
         for (int t = 0; t < WN_TAPS; t++, it++) {
-          const int s = it % WN_STAGES;
-          if (!mbar_wait(&full[s], (it / WN_STAGES) & 1, a.status, ST_TIMEOUT_MMA)) {
+          const int s = it % STAGES;
+          if (!mbar_wait(&full[s], (it / STAGES) & 1, a.status, ST_TIMEOUT_MMA)) {
             ok = false;
             break;
           }
@@ -309,7 +345,8 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
     const bool works = N == 64 || part == 0; /* the output layer's channel 0: one warp per quadrant */
     const int r = q * 32 + lane;           /* row of the tile this thread owns */
     uint32_t j = 0;
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, j++) {
+    const bool table_ok = EPI != EPI_BWD || mbar_wait(&wbar, 0, a.status, ST_TIMEOUT_WEIGHTS);
+    for (int tile = blockIdx.x; tile < n_tiles && table_ok; tile += gridDim.x, j++) {
       const uint32_t acc = j & 1;
       const int b = tile / tpp, l0 = (tile - b * tpp) << 7;
       const size_t row = (size_t)b * a.L + l0 + r;
@@ -345,10 +382,16 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
         store_row16(a.a_out + row * 64 + c0, ao);
       } else {
         Row16 go;
+        bool beyond = false;
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&zz.w[i]));
-          go.w[i] = pack_bf16(v[2 * i] * gelu_grad_f(f.x), v[2 * i + 1] * gelu_grad_f(f.y));
+        for (int i = 0; i < 8; i++)
+          go.w[i] = pack_bf16(v[2 * i] * gelu_grad_at(gelu_grad, zz.w[i] & 0xffff, beyond),
+                              v[2 * i + 1] * gelu_grad_at(gelu_grad, zz.w[i] >> 16, beyond));
+        if (beyond) {
+#pragma unroll
+          for (int i = 0; i < 8; i++)
+            go.w[i] = pack_bf16(v[2 * i] * gelu_grad_f(bf16_value(zz.w[i] & 0xffff)),
+                                v[2 * i + 1] * gelu_grad_f(bf16_value(zz.w[i] >> 16)));
         }
         store_row16(a.a_out + row * 64 + c0, go);
       }
@@ -512,19 +555,19 @@ cudaError_t launch_conv(int epi, const CUtensorMap &t_in, const CUtensorMap &t_w
   cudaError_t e;
   switch (epi) {
   case EPI_HIDDEN:
-    e = cudaFuncSetAttribute(conv_kernel<EPI_HIDDEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
+    e = cudaFuncSetAttribute(conv_kernel<EPI_HIDDEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)conv_smem(EPI_HIDDEN));
     if (e == cudaSuccess)
-      e = launch_chained(conv_kernel<EPI_HIDDEN>, grid, CONV_THREADS, CONV_SMEM, s, t_in, t_w, a);
+      e = launch_chained(conv_kernel<EPI_HIDDEN>, grid, CONV_THREADS, conv_smem(EPI_HIDDEN), s, t_in, t_w, a);
     break;
   case EPI_OUTPUT:
-    e = cudaFuncSetAttribute(conv_kernel<EPI_OUTPUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
+    e = cudaFuncSetAttribute(conv_kernel<EPI_OUTPUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)conv_smem(EPI_OUTPUT));
     if (e == cudaSuccess)
-      e = launch_chained(conv_kernel<EPI_OUTPUT>, grid, CONV_THREADS, CONV_SMEM, s, t_in, t_w, a);
+      e = launch_chained(conv_kernel<EPI_OUTPUT>, grid, CONV_THREADS, conv_smem(EPI_OUTPUT), s, t_in, t_w, a);
     break;
   default:
-    e = cudaFuncSetAttribute(conv_kernel<EPI_BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONV_SMEM);
+    e = cudaFuncSetAttribute(conv_kernel<EPI_BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)conv_smem(EPI_BWD));
     if (e == cudaSuccess)
-      e = launch_chained(conv_kernel<EPI_BWD>, grid, CONV_THREADS, CONV_SMEM, s, t_in, t_w, a);
+      e = launch_chained(conv_kernel<EPI_BWD>, grid, CONV_THREADS, conv_smem(EPI_BWD), s, t_in, t_w, a);
     break;
   }
   return e == cudaSuccess ? cudaGetLastError() : e;
@@ -682,6 +725,7 @@ struct b2e_wakenet {
   int device = 0, L = 0, max_batch = 0;
   int dil[WN_LAYERS];
   int64_t step = 0;
+  float *gelu_grad = nullptr; /* GELU' table of the backward convolutions */
   float *params = nullptr, *grads = nullptr, *adam_m = nullptr, *adam_v = nullptr;
   __nv_bfloat16 *wk = nullptr, *wt = nullptr;
   __nv_bfloat16 *x0 = nullptr, *z[WN_LAYERS] = {}, *act[WN_LAYERS] = {}, *dz[WN_LAYERS] = {};
@@ -775,6 +819,7 @@ int backward(b2e_wakenet *n, const float *targets, int n_prof, double *loss, cud
       a.sign = -1;
       a.z_prev = n->z[l - 1];
       a.a_out = n->dz[l - 1];
+      a.gelu_grad = n->gelu_grad;
       a.status = n->status;
       WN_TRY(n, launch_conv(EPI_BWD, n->t_dz[l], n->t_wt[l], a, cgrid, s));
     }
@@ -864,6 +909,7 @@ extern "C" int b2e_wakenet_create(b2e_wakenet **out, int32_t bins, int32_t max_b
   ok(dalloc(&n->bpart, (size_t)n->wgrad_grid_max * 64));
   ok(dalloc(&n->lpart, (size_t)((int64_t)max_batch * bins + 255) / 256));
   ok(dalloc(&n->status, 1));
+  ok(dalloc(&n->gelu_grad, GG_FLOATS));
   if (e == cudaSuccess) {
     ok(cudaMemset(n->params, 0, sizeof(float) * WN_NPARAM));
     ok(cudaMemset(n->grads, 0, sizeof(float) * WN_NPARAM));
@@ -885,6 +931,8 @@ extern "C" int b2e_wakenet_create(b2e_wakenet **out, int32_t bins, int32_t max_b
     }
   }
   if (e == cudaSuccess)
+    ok(launch_gelu_grad_table(n->gelu_grad, 0));
+  if (e == cudaSuccess)
     ok(refresh_weights(n, 0));
   if (e == cudaSuccess)
     ok(cudaDeviceSynchronize());
@@ -902,7 +950,7 @@ extern "C" int b2e_wakenet_destroy(b2e_wakenet *n) {
   cudaSetDevice(n->device);
   cudaDeviceSynchronize();
   void *ptrs[] = {n->params, n->grads, n->adam_m, n->adam_v, n->wk, n->wt, n->x0, n->y, n->wpart, n->bpart,
-                  n->lpart, n->status};
+                  n->lpart, n->status, n->gelu_grad};
   for (void *p : ptrs)
     if (p)
       cudaFree(p);

@@ -31,6 +31,7 @@ struct ConvArgs {
   __nv_bfloat16 *z_out;          /* EPI_HIDDEN: pre-activation (may be null) */
   __nv_bfloat16 *a_out;          /* EPI_HIDDEN: GELU(z); EPI_BWD: gradient of the previous pre-activation */
   const __nv_bfloat16 *z_prev;   /* EPI_BWD: pre-activation of the previous layer */
+  const float *gelu_grad;        /* EPI_BWD: the table of GELU' */
   float *y_out;                  /* EPI_OUTPUT: channel 0, [n_prof * L] */
   unsigned int *status;
 };
