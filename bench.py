@@ -205,6 +205,10 @@ class ClockSampler:
 
 
 # ------------------------------------------------------------ CPU oracle ----
+REF_LIB = os.path.join(os.path.dirname(os.path.abspath(__file__)), "oracle", "_ref", "libb2e_ref.so")
+REF_MISSING = "elegant's own code is not compiled here (oracle/_ref; its sources are not on this machine)"
+
+
 def _ref_worker(args):
     """Track a slice of ensemble instances with the reference's C code (libm)."""
     sys.path.insert(0, os.path.join(ROOT, "tests"))
@@ -393,7 +397,9 @@ def main():
     train = None if (args.no_bunch_train or world > 1) else bunch_train_section(args)
 
     cpu = None
-    if rank == 0 and world == 1 and not args.no_cpu_baseline:
+    if rank == 0 and world == 1 and not args.no_cpu_baseline and not os.path.exists(REF_LIB):
+        cpu = {"unavailable": REF_MISSING}
+    elif rank == 0 and world == 1 and not args.no_cpu_baseline:
         cores = os.cpu_count() or 1
         rate, info = cpu_reference_rate(args.instances, 2024, args.cpu_seconds, cores)
         cpu = {"value": rate, "unit": UNIT, "cores": cores, "kind": "reference",
@@ -437,6 +443,9 @@ def main():
 
 def run_reference(args, world, rank):
     if rank != 0:
+        return
+    if not os.path.exists(REF_LIB):
+        print(json.dumps({"impl": "reference", "unavailable": REF_MISSING}))
         return
     cores = os.cpu_count() or 1
     steps = []
