@@ -621,22 +621,27 @@ __device__ __forceinline__ double ordered_sum(const double *v, int n) {
   };
   int b = 0;
   load(r, 0);
-  for (; b + 16 <= n; b += 16) {
-    load(q, b + 8);
+  for (; b + 24 <= n; b += 16) {
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      q[k] = v[b + 8 + k];
     add(r);
-    load(r, b + 16);
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      r[k] = v[b + 16 + k];
     add(q);
   }
-  /* r holds what is left of the next eight values */
-  load(q, b + 8);
+  /* r holds v[b...b + 7] as far as they go; at most 23 are left */
+  for (; b < n; b += 8) {
+    load(q, b + 8);
 #pragma unroll
-  for (int k = 0; k < 8; k++)
-    if (b + k < n)
-      s += r[k];
+    for (int k = 0; k < 8; k++)
+      if (b + k < n)
+        s += r[k];
 #pragma unroll
-  for (int k = 0; k < 8; k++)
-    if (b + 8 + k < n)
-      s += q[k];
+    for (int k = 0; k < 8; k++)
+      r[k] = q[k];
+  }
   return s;
 }
 
@@ -719,14 +724,18 @@ __device__ bool wake_filters(const CountT *counts, CountT first, const WakeArgs 
     sg_apply<true>(hist, tmp, nb, a.sgHalf, a.sg_w);
     __syncthreads();
     /* thread 0 runs the serial sum, for real counts thread 32 that of the
-     * counts, and the warps behind them form the denominators */
-    const int helpers = EXACT ? 32 : 64;
+     * counts, and other warps form the denominators: not those of the first
+     * sub-partition (every fourth), whose FP64 pipe the sum waits for, 11.7
+     * cycles an addition with them there */
+    const int warp = threadIdx.x >> 5;
+    const bool helps = EXACT ? (warp & 3) != 0 : warp >= 2;
+    const int rank = EXACT ? warp - (warp >> 2) - 1 : warp - 2, helpers = EXACT ? warps - (warps + 3) / 4 : warps - 2;
     if (threadIdx.x == 0)
       smoothed_sum = ordered_sum(tmp, nb);
     else if (!EXACT && !a.lh && threadIdx.x == 32)
       nBinnedD = ordered_sum(hist, nb);
-    else if (threadIdx.x >= helpers)
-      for (int b = threadIdx.x - helpers; b < nb; b += blockDim.x - helpers) {
+    else if (helps)
+      for (int b = rank * 32 + (threadIdx.x & 31); b < nb; b += helpers * 32) {
         const double v = b2e_pow13(dct * b);
         denom[b] = v;
         if (INVERSE)
@@ -979,8 +988,12 @@ __device__ void wake_body(const CountT *counts, CountT first, const WakeArgs &a,
   }
 }
 
-/* threads of a wake CTA: a warp for the serial sum beside one thread per bin */
-static inline int wake_threads(int bins) { return std::min(1024, (bins + 31) / 32 * 32 + 32); }
+/* threads of a wake CTA: one per bin in the warps that form the denominators
+ * beside the serial sum, three of four */
+static inline int wake_threads(int bins) {
+  const int need = std::max(1, (bins + 31) / 32);
+  return std::min(1024, 32 * (need + (need + 2) / 3));
+}
 
 /* wake of one kick, one CTA per bunch; c1 and c2 from the bunch's CSRConstant
  * in the host expression's order (csbend.c:2664-2667).  With recycle set the
