@@ -98,7 +98,7 @@ def csr_section(args, device, flush):
     return {"workload": "bunch-compressor chicane with CSR, 1 GeV, 1 nC", "particles": beam.n, "dipole_kicks": kicks,
             "run_ms": ms, "csr_pass_ms_per_kick": ms / kicks,
             "particle_kicks_per_s": beam.n * kicks / (ms / 1e3),
-            "timing": "CUDA events on the engine stream; includes CSRDRIFT kicks and the one host sync per CSR element"}
+            "timing": "CUDA events on the engine stream; includes CSRDRIFT kicks and one host wait per CSR dipole"}
 
 
 def single_ring_section(args, flush):

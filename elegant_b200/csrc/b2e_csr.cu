@@ -1542,11 +1542,12 @@ __device__ __forceinline__ long long clamp_bins(double d, int nb) {
 /* wake of one Stupakov kick, one CTA per bunch (csbend.c:3950-4054): the
  * histogram filters of the last dipole, phi solutions (one warp, each starting
  * from the previous one: the latency of that chain bounds the kernel, 64 us
- * before and about 30 now for 300 bins, with the scan tabulated, the values of
- * a Newton pass side by side and all that is no part of the chain formed by the
- * whole block), then per bin case C, case D's boundary term and its
- * integral in the reference's order, times -4/rho GSConstant dz0.  Shared
- * memory: 4 nBins + 8 doubles for the filters, nBins for phi. */
+ * before and about 16 (30,000 cycles) now for 300 bins, with the scan
+ * tabulated, the values of a Newton pass side by side and all that is no part
+ * of the chain formed by the whole block), then per bin case C, case D's
+ * boundary term and its integral in the reference's order, times -4/rho
+ * GSConstant dz0.  Shared memory: 4 nBins + 8 doubles for the filters, nBins
+ * for phi. */
 __global__ void __launch_bounds__(1024, 1) stupakov_wake_kernel(CsrBunches B, const unsigned int *counts_all, WakeArgs a, StupakovArgs sa) {
   extern __shared__ double sm[];
   __shared__ double stage[2][SG_STAGE];
