@@ -927,8 +927,9 @@ __device__ void igf_wake(const WakeArgs &a, const double dct, const double *hist
  * smoothed density (per unit ct) and its derivative when hist_out/deriv_out
  * are set. */
 template <typename CountT, typename SumT, int NI>
-__device__ void wake_body(const CountT *counts, CountT first, const WakeArgs &a, const double dct, double *sm, double *dgamma,
-                          SumT *nbinned_out, double *hist_out, double *deriv_out, double *page = nullptr) {
+__device__ void wake_body(const CountT *counts, CountT first, const WakeArgs &a, const double dct, double *sm,
+                          double *dgamma, SumT *nbinned_out, double *hist_out, double *deriv_out,
+                          double *page = nullptr) {
   const int nb = a.nBins;
   const bool inverse = wake_filters<CountT, SumT, true>(counts, first, a, dct, sm, nbinned_out);
   const double *hist = sm, *deriv = sm + nb, *denom = sm + 2 * nb, *inv = sm + 4 * nb + 8;
@@ -1239,8 +1240,8 @@ __global__ void __launch_bounds__(BATCH_THREADS, 3)
   w.c2 = 0;
   w.csr_constant = 1;
   w.wakelog = nullptr;
-  wake_body<double, double, BATCH_BINS>(counts + off, threadIdx.x < a.nBins ? counts[off + threadIdx.x] : 0, w, 1.0, sm, t1_out + off, (double *)nullptr, hist_out + off,
-                                        deriv_out + off);
+  wake_body<double, double, BATCH_BINS>(counts + off, threadIdx.x < a.nBins ? counts[off + threadIdx.x] : 0, w, 1.0, sm,
+                                        t1_out + off, (double *)nullptr, hist_out + off, deriv_out + off);
 }
 
 /* Blocks of the kernels that collect ranges, and the run of particles each
@@ -1263,7 +1264,8 @@ static Sweep sweep_of(int64_t n) {
 }
 
 /* after the last kick: its wake kick and the min/max for the exit binning */
-__global__ void csr_last_kick_kernel(DevParticles P, int64_t n, int64_t share, CsrBunches B, int nBins, double Po, double rho0) {
+__global__ void csr_last_kick_kernel(DevParticles P, int64_t n, int64_t share, CsrBunches B, int nBins, double Po,
+                                     double rho0) {
   chain_enter();
   const int64_t first = blockIdx.x * share, end = min(n, first + share);
   BunchRange range(first < n ? bunch_of(first, B) : 0);
@@ -1385,7 +1387,8 @@ __global__ void csr_init_state_kernel(CsrDevState *st, int n) {
  * first kick when the drift does not start where the last CSR element ended,
  * csbend.c:3835-3848), then forward by dz; c*t = s/beta; min/max of c*t per
  * bunch (csbend.c:3876-3893) */
-__global__ void stupakov_drift_kernel(DevParticles P, int64_t n, int64_t share, CsrBunches B, double dz_back, double dz, double Po) {
+__global__ void stupakov_drift_kernel(DevParticles P, int64_t n, int64_t share, CsrBunches B, double dz_back,
+                                      double dz, double Po) {
   chain_enter();
   const int64_t first = blockIdx.x * share, end = min(n, first + share);
   BunchRange range(first < n ? bunch_of(first, B) : 0);
@@ -1548,7 +1551,8 @@ __device__ __forceinline__ long long clamp_bins(double d, int nb) {
  * boundary term and its integral in the reference's order, times -4/rho
  * GSConstant dz0.  Shared memory: 4 nBins + 8 doubles for the filters, nBins
  * for phi. */
-__global__ void __launch_bounds__(1024, 1) stupakov_wake_kernel(CsrBunches B, const unsigned int *counts_all, WakeArgs a, StupakovArgs sa) {
+__global__ void __launch_bounds__(1024, 1)
+    stupakov_wake_kernel(CsrBunches B, const unsigned int *counts_all, WakeArgs a, StupakovArgs sa) {
   extern __shared__ double sm[];
   __shared__ double stage[2][SG_STAGE];
   __shared__ PhiScan scan;
@@ -1562,7 +1566,8 @@ __global__ void __launch_bounds__(1024, 1) stupakov_wake_kernel(CsrBunches B, co
   const int nb = a.nBins;
   const double dct = st->dct;
   const unsigned int *counts = counts_all + (size_t)bunch * nb;
-  wake_filters<unsigned int, unsigned long long>(counts, threadIdx.x < nb ? counts[threadIdx.x] : 0, a, dct, sm, nullptr);
+  wake_filters<unsigned int, unsigned long long>(counts, threadIdx.x < nb ? counts[threadIdx.x] : 0, a, dct, sm,
+                                                 nullptr);
   const double *hist = sm, *deriv = sm + nb;
   double *phi = sm + 4 * nb + 8;
   if (!(dct > 0)) {
