@@ -415,13 +415,35 @@ __global__ void __launch_bounds__(CONV_THREADS, 2)
  * of the block.  The epilogue writes the block's partial sums
  * [5][64 ci][64 co].
  *
- * The fifth tap's partner in the third pair is a constant block whose channel
- * 0 is one in every bin: its accumulator row is the sum of dZ over the bins, the
- * bias gradient.  The tensor cores form it beside products they do anyway; a
- * kernel of its own read dZ again, 19 us per layer at 256 profiles. */
+ * The bias gradient, the sum of dZ over the bins, is taken from the dZ boxes
+ * while the tensor cores work on them, by the four warps that otherwise wait
+ * for the epilogue (a kernel of its own read dZ again, 19 us per layer at 256
+ * profiles): FP32 sums of 32 bins, FP64 from there on.  As one more accumulator
+ * row of the MMA the sums came out low, -4.1e-6 of the sum of magnitudes in the
+ * mean over residuals of one sign and many binades at 512 profiles (-1.6e-6 at
+ * 256): the accumulator does not round to nearest, and the loss grows with the
+ * bins of a block.  Now at most 4e-8, and the gradients call of 256 profiles
+ * takes 544 us instead of 552. */
 constexpr int WG_STAGES = 2;
 constexpr size_t WG_STAGE_BYTES = 6 * CONV_STAGE_BYTES; /* 96 KB */
-constexpr size_t WG_SMEM = 1024 + WG_STAGES * WG_STAGE_BYTES + CONV_STAGE_BYTES;
+constexpr size_t WG_SMEM = 1024 + WG_STAGES * WG_STAGE_BYTES;
+constexpr int WG_BIAS_WARPS = 4; /* warps 2 to 5 */
+
+/* sums over bins [32 part, 32 part + 32) of channels 2 lane and 2 lane + 1 of a
+ * 128-bin box; the 128-byte swizzle puts the 16-byte chunk c of a bin at
+ * c ^ (bin & 7), so a warp reads one bin without bank conflicts */
+__device__ __forceinline__ float2 column_sums(const unsigned char *box, int part, int lane) {
+  float2 s[4] = {};
+#pragma unroll
+  for (int k = 0; k < 32; k++) {
+    const int bin = part * 32 + k;
+    const uint32_t w =
+      *reinterpret_cast<const uint32_t *>(box + bin * 128 + (((lane >> 2) ^ (bin & 7)) << 4) + (lane & 3) * 4);
+    s[k & 3].x += bf16_value(w & 0xffff);
+    s[k & 3].y += __uint_as_float(w & 0xffff0000u);
+  }
+  return make_float2((s[0].x + s[1].x) + (s[2].x + s[3].x), (s[0].y + s[1].y) + (s[2].y + s[3].y));
+}
 
 __global__ void __launch_bounds__(WG_THREADS, 1)
     wgrad_kernel(const __grid_constant__ CUtensorMap t_in, const __grid_constant__ CUtensorMap t_dz, WgradArgs a) {
@@ -429,6 +451,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   unsigned char *sm = (unsigned char *)(((uintptr_t)dsm + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t full[WG_STAGES], empty[WG_STAGES], done;
   __shared__ uint32_t tmem_base;
+  __shared__ double2 bias[WG_BIAS_WARPS][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   chain_release();
   const int tpp = a.L >> 7, n_tiles = a.n_prof * tpp;
@@ -437,19 +460,11 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   if (threadIdx.x == 0) {
     for (int i = 0; i < WG_STAGES; i++) {
       mbar_init(&full[i], 1);
-      mbar_init(&empty[i], 1);
+      mbar_init(&empty[i], 1 + WG_BIAS_WARPS);
     }
     mbar_init(&done, 1);
     fence_barrier_init();
   }
-  unsigned char *ones = sm + WG_STAGES * WG_STAGE_BYTES;
-  for (int k = threadIdx.x; k < (int)(CONV_STAGE_BYTES / 16); k += WG_THREADS) {
-    /* 16-byte chunk k & 7 of bin k >> 3; the 128-byte swizzle puts channels 0-7
-     * of a bin in chunk (bin & 7) */
-    const int bin = k >> 3;
-    reinterpret_cast<uint4 *>(ones)[k] = make_uint4((k & 7) == (bin & 7) ? 0x3f80u : 0u, 0u, 0u, 0u);
-  }
-  fence_proxy_async(); /* the MMA reads it through the async proxy */
   if (warp == 0) {
     tmem_alloc(&tmem_base, 256);
     tmem_relinquish();
@@ -494,12 +509,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
         const uint32_t st = smem_u32(sm + s * WG_STAGE_BYTES);
         const uint32_t bz = st + 5 * (uint32_t)CONV_STAGE_BYTES;
         for (int p = 0; p < 3; p++) {
-          /* the two 64-channel blocks of A: taps 2p and 2p + 1, the last tap and
-           * the ones */
           const uint32_t ax = st + 2 * p * (uint32_t)CONV_STAGE_BYTES;
-          const uint32_t step = p < 2 ? (uint32_t)CONV_STAGE_BYTES : smem_u32(ones) - ax;
           for (int k = 0; k < 8; k++)
-            mma_bf16(tmem + 64 * p, sw128_desc(ax + 2048 * k, step, 1024),
+            mma_bf16(tmem + 64 * p, sw128_desc(ax + 2048 * k, (uint32_t)CONV_STAGE_BYTES, 1024),
                      sw128_desc(bz + 2048 * k, (uint32_t)CONV_STAGE_BYTES, 1024), IDESC, it > 0 || k > 0);
         }
         mma_commit(&empty[s]);
@@ -514,6 +526,28 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   if (warp >= 2) {
     const int q = warp & 3;
     const int m = q * 32 + lane; /* accumulator row */
+    double2 sum = make_double2(0, 0);
+    uint32_t it = 0;
+    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, it++) {
+      const int s = it % WG_STAGES;
+      if (!mbar_wait(&full[s], (it / WG_STAGES) & 1, a.status, ST_TIMEOUT_EPI))
+        break;
+      const float2 v = column_sums(sm + s * WG_STAGE_BYTES + 5 * CONV_STAGE_BYTES, warp - 2, lane);
+      __syncwarp();
+      if (lane == 0)
+        mbar_arrive(&empty[s]);
+      sum.x += v.x;
+      sum.y += v.y;
+    }
+    bias[warp - 2][lane] = sum;
+    asm volatile("bar.sync 1, 128;" ::: "memory"); /* the four warps */
+    if (warp == 2) {
+      for (int w = 1; w < WG_BIAS_WARPS; w++) {
+        sum.x += bias[w][lane].x;
+        sum.y += bias[w][lane].y;
+      }
+      reinterpret_cast<double2 *>(a.bias_partial + (size_t)blockIdx.x * 64)[lane] = sum;
+    }
     const bool ok = mbar_wait(&done, 0, a.status, ST_TIMEOUT_EPI);
     tc_fence_after();
     for (int p = 0; p < 3; p++) {
@@ -531,11 +565,6 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
       }
       if (t < WN_TAPS) {
         float4 *o = reinterpret_cast<float4 *>(a.partial + (((size_t)blockIdx.x * WN_TAPS + t) * 64 + ci) * 64);
-#pragma unroll
-        for (int c = 0; c < 64; c += 4)
-          o[c / 4] = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
-      } else if (ci == 0) {
-        float4 *o = reinterpret_cast<float4 *>(a.bias_partial + (size_t)blockIdx.x * 64);
 #pragma unroll
         for (int c = 0; c < 64; c += 4)
           o[c / 4] = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
@@ -663,36 +692,44 @@ __global__ void wn_loss_kernel(const float *y, const float *target, int64_t rows
     partial[blockIdx.x] = red[0];
 }
 
-/* grad[t][co][ci] = scale * sum_block wpart[block][t][ci][co]; grad_b[co]
- * likewise from bpart.  A block takes 64 consecutive sums, four threads each
- * (blocks b, b + 4, ... of the partials, then the four in order): four times the
- * loads in flight of one thread per sum. */
+/* sum of part(block, i) over the blocks of the partials: four threads (blocks b,
+ * b + 4, ...) and then the four in order; the total in the threads of the first
+ * 64 */
 constexpr int REDUCE_SPLIT = 4;
-__global__ void __launch_bounds__(64 * REDUCE_SPLIT)
-    wn_reduce_kernel(const float *wpart, int n_wblocks, const float *bpart, float scale, float *grad_w,
-                     float *grad_b) {
-  __shared__ float part[REDUCE_SPLIT][64];
-  chain_release();
-  chain_wait();
+template <typename T>
+__device__ __forceinline__ T reduce_blocks(const T *src, size_t stride, int n_blocks, T (*part)[64]) {
   const int c = threadIdx.x & 63, g = threadIdx.x >> 6;
-  const int idx = blockIdx.x * 64 + c; /* (t, ci, co), then the 64 biases */
-  const bool weights = idx < WN_WSIZE;
-  const float *src = weights ? wpart + idx : bpart + c;
-  const size_t stride = weights ? WN_WSIZE : 64;
-  float s = 0;
+  T s = 0;
 #pragma unroll 8
-  for (int b = g; b < n_wblocks; b += REDUCE_SPLIT)
+  for (int b = g; b < n_blocks; b += REDUCE_SPLIT)
     s += src[b * stride];
   part[g][c] = s;
   __syncthreads();
-  if (g)
-    return;
-  s = ((part[0][c] + part[1][c]) + part[2][c]) + part[3][c];
-  if (weights) {
-    const int co = idx & 63, ci = (idx >> 6) & 63, t = idx >> 12;
-    grad_w[(t * 64 + co) * 64 + ci] = s * scale;
-  } else
-    grad_b[c] = s * scale;
+  return ((part[0][c] + part[1][c]) + part[2][c]) + part[3][c];
+}
+
+/* grad[t][co][ci] = scale * sum_block wpart[block][t][ci][co], grad_b[co]
+ * likewise from bpart, in FP64.  A block takes 64 consecutive sums, four threads
+ * each: four times the loads in flight of one thread per sum.  The last block
+ * takes the biases. */
+__global__ void __launch_bounds__(64 * REDUCE_SPLIT)
+    wn_reduce_kernel(const float *wpart, int n_blocks, const double *bpart, float scale, float *grad_w,
+                     float *grad_b) {
+  __shared__ double part[REDUCE_SPLIT][64];
+  chain_release();
+  chain_wait();
+  const int idx = blockIdx.x * 64 + (threadIdx.x & 63); /* (t, ci, co), then the 64 biases */
+  if (idx < WN_WSIZE) {
+    const float s = reduce_blocks(wpart + idx, WN_WSIZE, n_blocks, reinterpret_cast<float(*)[64]>(part));
+    if (threadIdx.x < 64) {
+      const int co = idx & 63, ci = (idx >> 6) & 63, t = idx >> 12;
+      grad_w[(t * 64 + co) * 64 + ci] = s * scale;
+    }
+  } else {
+    const double s = reduce_blocks(bpart + (idx - WN_WSIZE), 64, n_blocks, part);
+    if (threadIdx.x < 64)
+      grad_b[threadIdx.x] = (float)(s * scale);
+  }
 }
 
 /* Adam (Kingma & Ba 2015) on the flat FP32 parameters, then the BF16 weight
@@ -726,10 +763,11 @@ struct b2e_wakenet {
   int dil[WN_LAYERS];
   int64_t step = 0;
   float *gelu_grad = nullptr; /* GELU' table of the backward convolutions */
+  double *bpart = nullptr; /* bias partials [wgrad_grid_max][64] */
   float *params = nullptr, *grads = nullptr, *adam_m = nullptr, *adam_v = nullptr;
   __nv_bfloat16 *wk = nullptr, *wt = nullptr;
   __nv_bfloat16 *x0 = nullptr, *z[WN_LAYERS] = {}, *act[WN_LAYERS] = {}, *dz[WN_LAYERS] = {};
-  float *y = nullptr, *wpart = nullptr, *bpart = nullptr;
+  float *y = nullptr, *wpart = nullptr;
   double *lpart = nullptr;
   unsigned int *status = nullptr;
   CUtensorMap t_x0, t_act[WN_LAYERS], t_dz[WN_LAYERS], t_wk[WN_LAYERS], t_wt[WN_LAYERS];
@@ -809,7 +847,7 @@ int backward(b2e_wakenet *n, const float *targets, int n_prof, double *loss, cud
     w.status = n->status;
     WN_TRY(n, launch_wgrad(l == 0 ? n->t_x0 : n->t_act[l - 1], n->t_dz[l], w, wgrid, s));
     WN_TRY(n, launch_chained(wn_reduce_kernel, WN_WSIZE / 64 + 1, 64 * REDUCE_SPLIT, 0, s, (const float *)n->wpart, wgrid,
-                             (const float *)n->bpart, scale, n->grads + l * WN_WSIZE,
+                             (const double *)n->bpart, scale, n->grads + l * WN_WSIZE,
                              n->grads + WN_LAYERS * WN_WSIZE + l * WN_CH));
     if (l > 0) {
       ConvArgs a{};

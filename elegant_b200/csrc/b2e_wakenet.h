@@ -39,7 +39,7 @@ struct ConvArgs {
 struct WgradArgs {
   int L, n_prof, dilation;
   float *partial;      /* [gridDim.x][5][64 ci][64 co] */
-  float *bias_partial; /* [gridDim.x][64 co] */
+  double *bias_partial; /* [gridDim.x][64 co] */
   unsigned int *status;
 };
 
