@@ -89,6 +89,7 @@ struct b2e_ctx {
   DevParticles ext{};
   bool use_ext = false;
   bool radiates = false; /* some element of some instance reads the DevRad table (any_radiation) */
+  bool fast = false;     /* some magnet of some instance takes the straight-line maps (any_fast) */
   CsrState csr;
   int pass_counter = 0; /* next pass to track in the current run */
   int64_t launches = 0; /* kernels launched by this context */
@@ -280,6 +281,13 @@ static bool any_radiation(const std::vector<DevElem> &elems) {
   return false;
 }
 
+static bool any_fast(const std::vector<DevElem> &elems) {
+  for (const DevElem &d : elems)
+    if ((d.kind == K_KMULT || d.kind == K_CSBEND) && (d.flags & EF_FAST))
+      return true;
+  return false;
+}
+
 extern "C" int b2e_element_defaults(int32_t type, b2e_element *element) {
   if (!element || type < B2E_DRIF || type > B2E_WATCH)
     return B2E_ERR_ARG;
@@ -315,6 +323,7 @@ extern "C" int b2e_load_lattice(b2e_ctx *ctx, const b2e_element *elements, int32
   ctx->rads_all = ctx->lat.rads;
   ctx->aps_all = ctx->lat.aps;
   ctx->radiates = any_radiation(ctx->elems_all);
+  ctx->fast = any_fast(ctx->elems_all);
   build_tiles(ctx);
   ctx->lattice_loaded = true;
   int rc = csr_configure(ctx->csr, ctx->base.data(), n_elements, ctx->lat, ctx->opt, ctx->err);
@@ -365,6 +374,7 @@ extern "C" int b2e_load_ensemble(b2e_ctx *ctx, int32_t n_instances, const int64_
     ctx->aps_all.insert(ctx->aps_all.end(), cl.aps.begin(), cl.aps.end());
   }
   ctx->radiates = any_radiation(ctx->elems_all);
+  ctx->fast = any_fast(ctx->elems_all);
   build_tiles(ctx);
   int rc = upload_lattice_tables(ctx);
   if (rc)
@@ -548,6 +558,7 @@ static int run_ring_range(b2e_ctx *ctx, int pb, int eb, int pe, int ee) {
   L.hist_pass0 = ctx->hist_pass0;
   L.hist_passes = ctx->hist_passes;
   L.rad = ctx->radiates;
+  L.fast = ctx->fast;
   L.rads = ctx->d_rads.ptr;
   L.tbt = ctx->opt.record_tbt && !ctx->use_ext && ctx->tbt_records > 0 ? ctx->d_tbt.ptr : nullptr;
   L.tbt_pass0 = ctx->pass_counter;

@@ -81,8 +81,10 @@ __device__ __forceinline__ void tile_moments(const Part &p, bool alive, double *
  * stay on the same element share its instruction stream and its shared-
  * memory record.  The arithmetic is identical in every variant.  HIST records
  * the per-pass tile moments (it needs SYNC >= 1); when SYNC >= 1 every thread
- * stays in the pass loop until the whole tile is lost. */
-template <bool STAGED, int MINB, int SYNC, bool HIST, int TPB, bool RAD = false>
+ * stays in the pass loop until the whole tile is lost.  FAST: magnets of EF_FAST
+ * take the straight-line maps and the general ones are called out of line;
+ * without it the general maps are in line. */
+template <bool STAGED, int MINB, int SYNC, bool HIST, int TPB, bool RAD = false, bool FAST = true>
 __global__ void __launch_bounds__(128 * TPB, MINB) ring_kernel(RingLaunch L) {
   static_assert(!HIST || SYNC >= 1, "history needs the per-pass barrier");
   static_assert(TPB == 1 || ((TPB == 2 || TPB == 4 || TPB == 8) && SYNC >= 1), "tiles of a block run in step");
@@ -177,8 +179,10 @@ __global__ void __launch_bounds__(128 * TPB, MINB) ring_kernel(RingLaunch L) {
           rs.elem = ie;
           rs.rc = rads[ie].c;
         }
-        if (!((e.flags & EF_FAST) && (RAD && (e.flags & EF_SR) ? kmult_fast<true>(p, e, ap, L.g, rs.rc)
-                                                               : kmult_fast<false>(p, e, ap, L.g, nullptr))))
+        if constexpr (!FAST)
+          lost = kmult<RAD>(p, e, ap, L.g, rs);
+        else if (!((e.flags & EF_FAST) && (RAD && (e.flags & EF_SR) ? kmult_fast<true>(p, e, ap, L.g, rs.rc)
+                                                                    : kmult_fast<false>(p, e, ap, L.g, nullptr))))
           lost = kmult_general<RAD>(p, e, ap, L.g, rs);
         break;
       case K_CSBEND:
@@ -187,8 +191,10 @@ __global__ void __launch_bounds__(128 * TPB, MINB) ring_kernel(RingLaunch L) {
           rs.elem = ie;
           rs.rc = rads[ie].c;
         }
-        if (!((e.flags & EF_FAST) && (RAD && (e.flags & EF_SR) ? csbend_fast<true>(p, e, ap, L.g, rs.rc)
-                                                               : csbend_fast<false>(p, e, ap, L.g, nullptr))))
+        if constexpr (!FAST)
+          lost = csbend<RAD>(p, e, ap, L.g, rs);
+        else if (!((e.flags & EF_FAST) && (RAD && (e.flags & EF_SR) ? csbend_fast<true>(p, e, ap, L.g, rs.rc)
+                                                                    : csbend_fast<false>(p, e, ap, L.g, nullptr))))
           lost = csbend_general<RAD>(p, e, ap, L.g, rs);
         break;
       case K_MALIGN: {
@@ -541,7 +547,7 @@ __global__ void effort_kernel(const int32_t *lost_pass, int64_t n, int pass_begi
   }
 }
 
-template <int MINB, int SYNC, bool HIST, int TPB, bool RAD = false>
+template <int MINB, int SYNC, bool HIST, int TPB, bool RAD = false, bool FAST = true>
 static cudaError_t launch_ring_v(const RingLaunch &L, int n_tiles, bool staged, size_t smem_bytes,
                                  cudaStream_t stream) {
   const int grid = (n_tiles + TPB - 1) / TPB;
@@ -549,13 +555,13 @@ static cudaError_t launch_ring_v(const RingLaunch &L, int n_tiles, bool staged, 
     staged = false; /* two instances' records do not fit: read them from global memory */
   if (staged) {
     const size_t bytes = smem_bytes * TPB;
-    cudaError_t err = cudaFuncSetAttribute(ring_kernel<true, MINB, SYNC, HIST, TPB, RAD>,
+    cudaError_t err = cudaFuncSetAttribute(ring_kernel<true, MINB, SYNC, HIST, TPB, RAD, FAST>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (err != cudaSuccess)
       return err;
-    ring_kernel<true, MINB, SYNC, HIST, TPB, RAD><<<grid, 128 * TPB, bytes, stream>>>(L);
+    ring_kernel<true, MINB, SYNC, HIST, TPB, RAD, FAST><<<grid, 128 * TPB, bytes, stream>>>(L);
   } else {
-    ring_kernel<false, MINB, SYNC, HIST, TPB, RAD><<<grid, 128 * TPB, 0, stream>>>(L);
+    ring_kernel<false, MINB, SYNC, HIST, TPB, RAD, FAST><<<grid, 128 * TPB, 0, stream>>>(L);
   }
   return cudaGetLastError();
 }
@@ -602,9 +608,20 @@ cudaError_t launch_ring(const RingLaunch &L, int n_tiles, bool staged, size_t sm
                         int variant) {
   if (n_tiles <= 0)
     return cudaSuccess;
-  if (L.rad) /* radiating lattices: one configuration (two tiles per block, a barrier per element) */
+  if (L.rad) { /* radiating lattices: one configuration (two tiles per block, a barrier per element) */
+    /* Without a single straight-line magnet the general maps are in line: out
+     * of line they keep the particle and the constants' addresses in memory,
+     * 4 to 6 % of a turn.  Quantum excitation everywhere, 10 turns of 200
+     * particles 16.1 -> 15.2 ms, an ensemble of 256 instances 56.2 -> 51.0 ms for
+     * 3 turns; field terms and steering 3.54 -> 3.26 ms.  One magnet in twenty of
+     * the other kind makes up for it: a straight-line map takes less than half of
+     * the time. */
+    if (!L.fast)
+      return L.hist ? launch_ring_v<2, 2, true, 2, true, false>(L, n_tiles, staged, smem_bytes, stream)
+                    : launch_ring_v<2, 2, false, 2, true, false>(L, n_tiles, staged, smem_bytes, stream);
     return L.hist ? launch_ring_v<2, 2, true, 2, true>(L, n_tiles, staged, smem_bytes, stream)
                   : launch_ring_v<2, 2, false, 2, true>(L, n_tiles, staged, smem_bytes, stream);
+  }
   if (variant < 1 || variant > B2E_RING_VARIANTS)
     variant = 1;
   if (variant > 12)
