@@ -1341,16 +1341,35 @@ __global__ void csr_exit_kernel(DevParticles P, int64_t n, const DevElem *ep, Be
   P.s[i] = s;
 }
 
+/* exact drift of particle i */
+__device__ __forceinline__ void exact_drift(const DevParticles &P, int64_t i, double L) {
+  const double xp = P.xp[i], yp = P.yp[i];
+  P.x[i] = P.x[i] + xp * L;
+  P.y[i] = P.y[i] + yp * L;
+  P.s[i] = P.s[i] + L * sqrt((1 + xp * xp) + yp * yp);
+}
+
+/* The particles of a CSRDRIFT's bunches without a wake (csbend.c:3196-3212):
+ * its first kick kernel takes them through the whole length, so that no pass of
+ * its own asks every particle for its bunch's mode */
+struct PlainDrift {
+  double length;
+  int now; /* the first kick */
+};
+
 /* CSRDRIFT mode 0, one kick (csbend.c:3415-3502) */
-__global__ void csr_drift_kick_kernel(DevParticles P, int64_t n, CsrBunches B, double dz, double s0_incr,
-                                      double factor, int apply, int nBins, double Po) {
+__global__ void csr_drift_kick_kernel(DevParticles P, int64_t n, CsrBunches B, PlainDrift plain, double dz,
+                                      double s0_incr, double factor, int apply, int nBins, double Po) {
   chain_enter();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n || P.lost_pass[i] >= 0)
     return;
   const int b = bunch_of(i, B);
-  if (!B.mode[b])
+  if (!B.mode[b]) {
+    if (plain.now)
+      exact_drift(P, i, plain.length);
     return;
+  }
   const CsrDevState *st = B.st + b;
   double x = P.x[i], xp = P.xp[i], y = P.y[i], yp = P.yp[i], s = P.s[i], dp = P.dp[i], p, beta;
   x = x + xp * dz;
@@ -1387,15 +1406,17 @@ __global__ void csr_init_state_kernel(CsrDevState *st, int n) {
  * first kick when the drift does not start where the last CSR element ended,
  * csbend.c:3835-3848), then forward by dz; c*t = s/beta; min/max of c*t per
  * bunch (csbend.c:3876-3893) */
-__global__ void stupakov_drift_kernel(DevParticles P, int64_t n, int64_t share, CsrBunches B, double dz_back,
-                                      double dz, double Po) {
+__global__ void stupakov_drift_kernel(DevParticles P, int64_t n, int64_t share, CsrBunches B, PlainDrift plain,
+                                      double dz_back, double dz, double Po) {
   chain_enter();
   const int64_t first = blockIdx.x * share, end = min(n, first + share);
   BunchRange range(first < n ? bunch_of(first, B) : 0);
   for (int64_t i = first + threadIdx.x; i - threadIdx.x < end; i += blockDim.x) {
     const int b = i < n ? bunch_of(i, B) : B.n - 1;
-    const bool mine = i < n && P.lost_pass[i] < 0 && B.mode[b];
+    const bool alive = i < n && P.lost_pass[i] < 0, mine = alive && B.mode[b];
     double ct = 0;
+    if (alive && !mine && plain.now)
+      exact_drift(P, i, plain.length);
     if (mine) {
       double x = P.x[i], xp = P.xp[i], y = P.y[i], yp = P.yp[i], s = P.s[i];
       if (dz_back != 0) {
@@ -1737,10 +1758,7 @@ __global__ void edrift_kernel(DevParticles P, int64_t n, double L, CsrBunches B,
     return;
   if (B.mode && B.mode[bunch_of(i, B)] != mode)
     return;
-  double xp = P.xp[i], yp = P.yp[i];
-  P.x[i] = P.x[i] + xp * L;
-  P.y[i] = P.y[i] + yp * L;
-  P.s[i] = P.s[i] + L * sqrt((1 + xp * xp) + yp * yp);
+  exact_drift(P, i, L);
 }
 
 /* ------------------------------------------------------------------ host -- */
@@ -2169,13 +2187,44 @@ static void set_filter_args(WakeArgs &a, int lh, int clip, double lowCut0, doubl
   a.endLP = highCut1;
 }
 
+/* Whether the wake kicks of a CSRDRIFT go on: some candidate bunch has the two
+ * particles that a wake takes.  Where none has, the first kick's kernel has done
+ * the whole drift.  Asked between kicks without waiting for the device, which
+ * has the dipole's kernels ahead of it: a wait here drained them and took 8 % of
+ * a run of 100 kicks per drift (1,726 -> 1,865 us, 20,011 particles).  Ranks that
+ * share bunches have to agree on the number of kicks, so with a reducer the
+ * host waits. */
+struct DriftKicks {
+  bool on = true, known = false;
+};
+static int drift_goes_on(CsrState &st, const std::vector<unsigned char> &flags, bool wait, DriftKicks &k,
+                         std::string &err) {
+  if (k.known)
+    return B2E_OK;
+  const cudaError_t e = wait ? cudaEventSynchronize(st.alive_known) : cudaEventQuery(st.alive_known);
+  if (e == cudaErrorNotReady) {
+    cudaGetLastError();
+    return B2E_OK;
+  }
+  if (e != cudaSuccess) {
+    err = "CSR: alive count failed";
+    return B2E_ERR_CUDA;
+  }
+  k.known = true;
+  k.on = false;
+  for (int b = 0; b < st.n_bunches; b++)
+    k.on = k.on || (flags[st.n_bunches + b] && st.h_alive[b] > 1);
+  return B2E_OK;
+}
+
 /* CSRDRIFT with USE_STUPAKOV=1 (track_through_driftCSR_Stupakov,
- * csbend.c:3803-4159) for the bunches whose mode flag is set; the others have
- * had their exact drift.  Per kick: drift and c*t with the min/max keys, the
- * histogram of the last dipole's bin count and range factor, the wake (one
+ * csbend.c:3803-4159) for the bunches whose mode flag is set; the others get
+ * their exact drift in the first kick's drift kernel.  Per kick: drift and c*t
+ * with the min/max keys, the histogram of the last dipole's bin count and range factor, the wake (one
  * CTA per bunch), the kick; then the closing half drift. */
-static int stupakov_drift(CsrState &st, const CsrElem &ce, const CsrBunches &B, const DevParticles &P, int64_t n,
-                          double zStart, cudaStream_t stream, std::string &err, int64_t *launches) {
+static int stupakov_drift(CsrState &st, const CsrElem &ce, const CsrBunches &B,
+                          const std::vector<unsigned char> &flags, const DevParticles &P, int64_t n, double zStart,
+                          cudaStream_t stream, std::string &err, int64_t *launches) {
   if (st.last_bend < 0) {
     err = "CSRDRIFT: no dipole wake to follow";
     return B2E_ERR_STATE;
@@ -2215,6 +2264,7 @@ static int stupakov_drift(CsrState &st, const CsrElem &ce, const CsrBunches &B, 
   CSR_CUDA(cudaFuncSetAttribute(stupakov_wake_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   CsrBunches H = B; /* the histogram bins the bunches in this mode */
   H.active = B.mode;
+  DriftKicks kicks;
   for (long iKick = 0; iKick < nKicks; iKick++) {
     if (iKick == 1)
       dz = dz0;
@@ -2229,9 +2279,15 @@ static int stupakov_drift(CsrState &st, const CsrElem &ce, const CsrBunches &B, 
     sa.trapz = bend.trapz;
     csr_reset_keys_kernel<<<1, 32, 0, stream>>>(B);
     CSR_CUDA(launch_chained(stupakov_drift_kernel, dim3(sweep.grid), dim3(256), 0, stream, P, n, sweep.share, B,
-                            iKick == 0 ? dz_back : 0.0, dz, Po));
+                            PlainDrift{ce.drift_length, iKick == 0}, iKick == 0 ? dz_back : 0.0, dz, Po));
     (*launches) += 2;
     CSR_CUDA(cudaGetLastError());
+    /* a reducer is called only for wakes that are formed */
+    if (iKick > 0 || st.reducer)
+      if (int rc = drift_goes_on(st, flags, st.reducer, kicks, err))
+        return rc;
+    if (!kicks.on)
+      return B2E_OK;
     int rrc = reduce_keys(st, B, stream, err, launches);
     if (rrc)
       return rrc;
@@ -2301,11 +2357,10 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
       if (rc)
         return rc;
       if (!(ce.drift_dz > 0) && ce.drift_kicks <= 0) {
-        if (await_alive(st, err))
-          return B2E_ERR_CUDA;
-        any = false;
-        for (int b = 0; b < nbunch; b++)
-          any = any || (flags[nbunch + b] && st.h_alive[b] > 1);
+        DriftKicks kicks;
+        if (int rc2 = drift_goes_on(st, flags, true, kicks, err))
+          return rc2;
+        any = kicks.on;
       }
     }
     if (!any) {
@@ -2316,15 +2371,12 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
       CSR_CUDA(cudaGetLastError());
       return B2E_OK;
     }
-    CSR_CUDA(launch_chained(edrift_kernel, dim3(g), dim3(256), 0, stream, P, n, ce.drift_length, B, 0));
-    (*launches)++;
-    CSR_CUDA(cudaGetLastError());
     double zStart = ce.z_start;
     /* a drift behind the previous pass's dipole (csbend.c:3251-3255) */
     for (int guard = 0; zStart + 1e-12 < st.zLast && st.revolution_length > 0 && guard < (1 << 20); guard++)
       zStart += st.revolution_length;
     if (ce.stupakov)
-      return stupakov_drift(st, ce, B, P, n, zStart, stream, err, launches);
+      return stupakov_drift(st, ce, B, flags, P, n, zStart, stream, err, launches);
     int nKicks;
     if (ce.drift_dz > 0) {
       if ((nKicks = (int)(ce.drift_length / ce.drift_dz)) < 1)
@@ -2340,16 +2392,21 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
     /* csrWake.bins: bins of the last CSRCSBEND tracked (on a later pass,
      * possibly one further down the line) */
     const int lastBins = st.last_bend >= 0 ? st.elems[st.last_bend].bins : 0;
+    DriftKicks kicks;
     for (int iKick = 0; iKick < nKicks; iKick++) {
       if (iKick == 1)
         dz = dz0;
       double incr = dz + dzFirst;
       double factor = (dz0 + dzFirst) / st.ds0;
-      CSR_CUDA(launch_chained(csr_drift_kick_kernel, dim3(g), dim3(256), 0, stream, P, n, B, dz, incr, factor, 1,
-                              lastBins, Po));
+      CSR_CUDA(launch_chained(csr_drift_kick_kernel, dim3(g), dim3(256), 0, stream, P, n, B,
+                              PlainDrift{ce.drift_length, iKick == 0}, dz, incr, factor, 1, lastBins, Po));
       CSR_CUDA(launch_chained(csr_s0_add_kernel, dim3(1), dim3(32), 0, stream, B, incr));
       (*launches) += 2;
       CSR_CUDA(cudaGetLastError());
+      if (int rc = drift_goes_on(st, flags, false, kicks, err))
+        return rc;
+      if (!kicks.on)
+        return B2E_OK;
       dzFirst = 0;
     }
     dz = dz0 / 2;
