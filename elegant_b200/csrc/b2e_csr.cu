@@ -203,11 +203,9 @@ struct SliceWake {
 };
 
 /* Optional wake kick of the previous kick, one integrator slice, c*t update
- * (csbend.c:2385-2450), in the general form; out of line, for other integration
- * orders and particles near a limit. */
-static __device__ __noinline__ int csr_slice_general(SlicePart *p, const DevElem *ep, const CsrDevState *st, int nBins,
-                                                     int apply, double Po) {
-  const DevElem &e = *ep;
+ * (csbend.c:2385-2450), in the general form */
+__device__ __forceinline__ int csr_slice_general(SlicePart *p, const DevElem &e, const CsrDevState *st, int nBins,
+                                                 int apply, double Po) {
   const double *c = e.c;
   double f, Q1, Q3, Q4;
   if (apply)
@@ -224,6 +222,12 @@ static __device__ __noinline__ int csr_slice_general(SlicePart *p, const DevElem
   if (!lost)
     p->CT = p->CT + Q4 / p->beta0;
   return lost;
+}
+
+/* out of line, for particles near a limit of the straight-line form */
+static __device__ __noinline__ int csr_slice_outlier(SlicePart *p, const DevElem *e, const CsrDevState *st, int nBins,
+                                                     int apply, double Po) {
+  return csr_slice_general(p, *e, st, nBins, apply, Po);
 }
 
 static __device__ __noinline__ double divide_ieee(double a, double b) { return a / b; }
@@ -288,6 +292,7 @@ __device__ __forceinline__ void copy4_async(void *smem, const void *gmem) {
  * coordinates, then for the velocity, and every warp sent two atomics to the
  * bunch's range words; here the range stays in registers until the bunch
  * changes. */
+template <bool STRAIGHT>
 __global__ void __launch_bounds__(SLICE_THREADS, SLICE_BLOCKS_PER_SM)
     csr_slice_kernel(DevParticles P, int64_t n, int64_t tiles_per_block, const double *beta0,
                      const __grid_constant__ DevElem e, CsrBunches B, int after_first_kick, int nBins, double Po,
@@ -298,7 +303,7 @@ __global__ void __launch_bounds__(SLICE_THREADS, SLICE_BLOCKS_PER_SM)
   const int t = threadIdx.x;
   const int64_t begin = blockIdx.x * tiles_per_block * SLICE_THREADS + t;
   const int64_t end = min(n, (blockIdx.x + 1) * tiles_per_block * SLICE_THREADS);
-  const bool straight = (e.flags & EF_FAST) && e.c[CB_NSUB] == 4 && fp_within(Po, FP_HI_2M10, FP_HI_2P100);
+  const bool usual_Po = fp_within(Po, FP_HI_2M10, FP_HI_2P100);
   auto fetch = [&](int64_t i, int slot) {
     if (i < end) {
       copy8_async(&col[slot][0][t], P.x + i);
@@ -332,16 +337,21 @@ __global__ void __launch_bounds__(SLICE_THREADS, SLICE_BLOCKS_PER_SM)
       const double(*v)[SLICE_THREADS] = col[slot];
       const SliceWake w = {st->dGamma, st->ctLower, st->dct, nBins, after_first_kick && B.csr_const[bunch] != 0};
       int lost = 0;
-      p.X = v[0][t];
-      p.XP = v[1][t];
-      p.Y = v[2][t];
-      p.YP = v[3][t];
-      p.DP = v[5][t];
-      if (!(straight && (!w.apply || fp_within(w.dct, FP_HI_2M250, FP_HI_2P100)) &&
-            csr_slice_fast(p, e, w, &v[4][t], &v[6][t], Po, inv_Po))) {
-        SlicePart q = {v[0][t], v[1][t], v[2][t], v[3][t], v[4][t], v[5][t], v[6][t]};
-        lost = csr_slice_general(&q, &e, st, nBins, w.apply, Po);
-        p = q;
+      if constexpr (STRAIGHT) {
+        p.X = v[0][t];
+        p.XP = v[1][t];
+        p.Y = v[2][t];
+        p.YP = v[3][t];
+        p.DP = v[5][t];
+        if (!(usual_Po && (!w.apply || fp_within(w.dct, FP_HI_2M250, FP_HI_2P100)) &&
+              csr_slice_fast(p, e, w, &v[4][t], &v[6][t], Po, inv_Po))) {
+          SlicePart q = {v[0][t], v[1][t], v[2][t], v[3][t], v[4][t], v[5][t], v[6][t]};
+          lost = csr_slice_outlier(&q, &e, st, nBins, w.apply, Po);
+          p = q;
+        }
+      } else {
+        p = {v[0][t], v[1][t], v[2][t], v[3][t], v[4][t], v[5][t], v[6][t]};
+        lost = csr_slice_general(&p, e, st, nBins, w.apply, Po);
       }
       P.x[i] = p.X;
       P.xp[i] = p.XP;
@@ -360,6 +370,15 @@ __global__ void __launch_bounds__(SLICE_THREADS, SLICE_BLOCKS_PER_SM)
     range.add(p.CT, alive, bunch, B);
   }
   range.flush(B);
+}
+
+/* The straight-line form holds four substeps (INTEGRATION_ORDER 4) and takes
+ * elements of EF_FAST.  The others have a kernel of their own: 1e6 particles
+ * through 10 kicks per dipole at INTEGRATION_ORDER 6 took 5.89 ms with the
+ * general form called out of line from one kernel for all, 5.48 ms with it in
+ * line; 3.12 and 2.86 ms at order 2. */
+static auto slice_kernel(const DevElem &e) {
+  return (e.flags & EF_FAST) && e.c[CB_NSUB] == 4 ? csr_slice_kernel<true> : csr_slice_kernel<false>;
 }
 
 /* grid and tiles per block: as many blocks as the SMs hold at once, each with
@@ -2505,7 +2524,7 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
     }
     int64_t per_block;
     const int slice_blocks = slice_grid(n, &per_block);
-    CSR_CUDA(launch_chained(csr_slice_kernel, dim3(slice_blocks), dim3(SLICE_THREADS), 0, stream, P, n, per_block,
+    CSR_CUDA(launch_chained(slice_kernel(h_elem), dim3(slice_blocks), dim3(SLICE_THREADS), 0, stream, P, n, per_block,
                             (const double *)st.d_beta0, h_elem, B, (int)(kick > 0), ce.bins, Po, 1 / Po, pass, elem));
     (*launches)++;
     CSR_CUDA(cudaGetLastError());
@@ -2968,8 +2987,8 @@ extern "C" int b2e_csr_bend_static(double *const dev_columns[6], int32_t *dev_lo
     csr_reset_keys_kernel<<<1, 32, 0, s>>>(B);
     int64_t per_block;
     const int slice_blocks = slice_grid(n, &per_block);
-    csr_slice_kernel<<<slice_blocks, SLICE_THREADS, 0, s>>>(P, n, per_block, S->beta0, d, B, kick > 0, bins, Po, 1 / Po,
-                                                            0, 0);
+    slice_kernel(d)<<<slice_blocks, SLICE_THREADS, 0, s>>>(P, n, per_block, S->beta0, d, B, kick > 0, bins, Po,
+                                                               1 / Po, 0, 0);
     STATIC_TRY(cudaGetLastError());
     STATIC_TRY(cudaMemsetAsync(S->counts, 0, sizeof(unsigned int) * bins, s));
     int hb = hist_blocks(n, 1);
