@@ -433,16 +433,16 @@ __device__ void fiducial_without_sum(const DevParticles &P, int64_t first, int64
   fiducial_set(rs, e, tsum, nsum);
 }
 
-constexpr int FID_THREADS = 256, FID_TILE = 1024;
-
 /* gx blocks per instance; the last one to finish its share forms the result.
- * acc: one zeroed record per instance. */
-__global__ void __launch_bounds__(FID_THREADS)
+ * acc: one zeroed record per instance.  A block of one warp takes a whole
+ * instance (gx = 1) and needs none. */
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS)
     rf_fiducial_kernel(DevParticles P, const int64_t *inst_offsets, int gx, const DevElem *elems, int n_elems,
                        int elem_index, DevRfState *rf, int n_rf, double p_central, int64_t max_rows, FidAcc *acc_all,
                        unsigned int *error_flag) {
-  __shared__ double tile[FID_TILE];
-  __shared__ int last;
+  constexpr int TILE = 4 * THREADS;
+  __shared__ double tile[TILE];
   const int inst = blockIdx.x / gx, part = blockIdx.x - inst * gx;
   const DevElem &e = elems[(size_t)inst * n_elems + elem_index];
   DevRfState *rf_inst = rf + (size_t)inst * n_rf;
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(FID_THREADS)
   }
   const double sOffset = e.c[RF_SOFFSET];
   FidAcc a = {0, 0, 0, 0, 0, 0, 0};
-  for (int64_t ip = first + part * FID_THREADS + threadIdx.x; ip < end; ip += (int64_t)gx * FID_THREADS) {
+  for (int64_t ip = first + part * THREADS + threadIdx.x; ip < end; ip += (int64_t)gx * THREADS) {
     if (P.lost_pass[ip] >= 0)
       continue;
     const unsigned long long bits = (unsigned long long)__double_as_longlong(arrival_time(P, ip, sOffset, p_central));
@@ -481,35 +481,45 @@ __global__ void __launch_bounds__(FID_THREADS)
     a.e_max = max(a.e_max, __shfl_down_sync(0xffffffffu, a.e_max, off));
     a.e_min_c = max(a.e_min_c, __shfl_down_sync(0xffffffffu, a.e_min_c, off));
   }
-  FidAcc *acc = acc_all + inst;
-  if ((threadIdx.x & 31) == 0 && a.n) {
-    atomicAdd(&acc->lo, a.lo);
-    atomicAdd(&acc->hi, a.hi);
-    atomicAdd(&acc->n, a.n);
-    atomicMax(&acc->m_max, a.m_max);
-    atomicMax(&acc->e_max, a.e_max);
-    atomicMax(&acc->e_min_c, a.e_min_c);
-  }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0)
-    last = atomicAdd(&acc->done, 1ull) == (unsigned long long)(gx - 1);
-  __syncthreads();
-  if (!last)
-    return;
-  __threadfence();
-  const unsigned long long lo = __ldcg(&acc->lo), hi = __ldcg(&acc->hi), n = __ldcg(&acc->n),
-                           m_max = __ldcg(&acc->m_max);
-  const unsigned int ex = __ldcg(&acc->e_max), exc = __ldcg(&acc->e_min_c);
-  if (n && n < (1ull << 31) && ex + exc == 2047u && ex > 100 && ex < 1900 && m_max <= (1ull << 53) - 2 * n) {
+  if constexpr (THREADS > 32) {
+    __shared__ int last;
+    FidAcc *acc = acc_all + inst;
+    if ((threadIdx.x & 31) == 0 && a.n) {
+      atomicAdd(&acc->lo, a.lo);
+      atomicAdd(&acc->hi, a.hi);
+      atomicAdd(&acc->n, a.n);
+      atomicMax(&acc->m_max, a.m_max);
+      atomicMax(&acc->e_max, a.e_max);
+      atomicMax(&acc->e_min_c, a.e_min_c);
+    }
+    __threadfence();
+    __syncthreads();
     if (threadIdx.x == 0)
-      fiducial_set(rs, e, round_u128(((unsigned __int128)hi << 32) + lo, (int)ex - 1075), (int64_t)n);
+      last = atomicAdd(&acc->done, 1ull) == (unsigned long long)(gx - 1);
+    __syncthreads();
+    if (!last)
+      return;
+    __threadfence();
+    a.lo = __ldcg(&acc->lo);
+    a.hi = __ldcg(&acc->hi);
+    a.n = __ldcg(&acc->n);
+    a.m_max = __ldcg(&acc->m_max);
+    a.e_max = __ldcg(&acc->e_max);
+    a.e_min_c = __ldcg(&acc->e_min_c);
+  }
+  /* one warp has its sums in lane 0; otherwise every thread has them */
+  const unsigned long long n = THREADS > 32 ? a.n : __shfl_sync(0xffffffffu, a.n, 0);
+  const bool exact = n && n < (1ull << 31) && a.e_max + a.e_min_c == 2047u && a.e_max > 100 && a.e_max < 1900 &&
+                     a.m_max <= (1ull << 53) - 2 * n;
+  if (THREADS > 32 ? exact : __shfl_sync(0xffffffffu, exact, 0)) {
+    if (threadIdx.x == 0)
+      fiducial_set(rs, e, round_u128(((unsigned __int128)a.hi << 32) + a.lo, (int)a.e_max - 1075), (int64_t)n);
     return;
   }
   double tsum = 0, error = 0;
-  for (int64_t t0 = first; t0 < end; t0 += FID_TILE) {
-    const int len = (int)min((int64_t)FID_TILE, end - t0);
-    for (int k = threadIdx.x; k < len; k += FID_THREADS)
+  for (int64_t t0 = first; t0 < end; t0 += TILE) {
+    const int len = (int)min((int64_t)TILE, end - t0);
+    for (int k = threadIdx.x; k < len; k += THREADS)
       tile[k] = P.lost_pass[t0 + k] < 0 ? arrival_time(P, t0 + k, sOffset, p_central) : 0.0;
     __syncthreads();
     if (threadIdx.x == 0)
@@ -725,12 +735,20 @@ cudaError_t launch_fiducial(DevParticles P, const int64_t *inst_offsets, int n_i
   int64_t gx = (rows + 1023) / 1024, cap = 148 * 4 / n_inst;
   gx = gx > cap ? cap : gx;
   gx = gx < 1 ? 1 : gx;
+  /* instances of a few particles: a warp each, without the zeroed records and
+   * their atomics.  Whole calls of 20,000 instances of three: 316 us with blocks
+   * of 256 threads, 216 so; 3,000 of 64: 119 and 99 us. */
+  if (rows <= 64) {
+    rf_fiducial_kernel<32><<<(unsigned)n_inst, 32, 0, stream>>>(P, inst_offsets, 1, elems, n_elems, elem_index, rf,
+                                                                n_rf, p_central, max_rows, nullptr, error_flag);
+    return cudaGetLastError();
+  }
   cudaError_t err = cudaMemsetAsync(scratch, 0, fiducial_scratch_bytes(n_inst), stream);
   if (err != cudaSuccess)
     return err;
-  rf_fiducial_kernel<<<(unsigned)(gx * n_inst), FID_THREADS, 0, stream>>>(P, inst_offsets, (int)gx, elems, n_elems, elem_index, rf,
-                                                                       n_rf, p_central, max_rows, (FidAcc *)scratch,
-                                                                       error_flag);
+  rf_fiducial_kernel<256><<<(unsigned)(gx * n_inst), 256, 0, stream>>>(P, inst_offsets, (int)gx, elems, n_elems,
+                                                                       elem_index, rf, n_rf, p_central, max_rows,
+                                                                       (FidAcc *)scratch, error_flag);
   return cudaGetLastError();
 }
 
