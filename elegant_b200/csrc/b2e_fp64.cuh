@@ -18,19 +18,37 @@
  * (1 - e)^(-1/2), applied to D y0 for the root and to y0 for its reciprocal,
  * then Markstein's correction g + (D - g^2)/(2g) with an exact remainder
  * (P. Markstein, IBM J. Res. Dev. 34, 1990).  Quotient: q = RN(a y), remainder
- * a - q b exact under fma, RN(q + r y), with y = RN(1/b) (the same paper).
+ * a - q b exact under fma, RN(q + r y) (the same paper).
  *
- * Why the roundings are right.  Quotient: with y = RN(1/b) the last step
- * returns RN(a/b) for every a (the same paper); a result can round wrongly only
- * where a/b lies within |r| |y - 1/b| of a midpoint, q is then one of the two
- * neighbours, and half an ulp times the relative error of y is below the
- * smallest distance a quotient can have from a midpoint.  The iterations give
- * RN(1/b) but for the significand just below 2 (1/b a hair above a midpoint),
- * which fp_fix sets.  Square root: with g next to the midpoint the remainder is
- * an integer multiple of ulp(g)^2, and a relative error of the factor 1/(2g)
- * below 1.5 2^-53 (here at most 1.32) cannot move it across the rounding
- * boundary.  b2e_selftest_rounding compares all of them with the IEEE
- * operators on the device.
+ * Why the roundings are right, with b in [1, 2) for the significand of a divisor:
+ *
+ * Reciprocal, fp_polish.  y (2 - b y) is (1/b)(1 - e^2) before the last rounding,
+ * e the relative error of y; it rounds to RN(1/b) unless a midpoint lies within
+ * e^2/b below 1/b.  For b = B 2^-52 and a midpoint M 2^-54 (M odd) the distance is
+ * k 2^-106/b with k = 2^106 - M B odd, so with e below sqrt(3) 2^-53 only k = 1
+ * remains, and the only divisor of 2^106 - 1 = 3 107 6361 69431 20394401
+ * 28059810762433 in [2^52, 2^53) is 2^53 - 1, the significand of all ones, which
+ * fp_fix sets.
+ *
+ * Reciprocal, fp_recip.  The series is short of e^4 and its sum rounds at
+ * 2^-53 e, e at most 2^-19 of the seed, so y is within 0.5 + 2^-20 ulp of 1/b: not
+ * always RN(1/b): six divisors in 1e8 have its neighbour.
+ *
+ * Quotient.  With y = (1/b)(1 + e) the last fma rounds a/b - (q - a/b) e.  Let a/b
+ * (a in [1, 2) too) lie next to a midpoint: its distance is |k| 2^-105/b for a >= b,
+ * |k| 2^-106/b for a < b, k an integer other than 0, and half an ulp is 2^-53 or
+ * 2^-54.  |e| is at most 2^-54 b (1 + 2^-19).  For b below 2 - 2^-18 q is one of the
+ * midpoint's neighbours, half an ulp away, and a wrong rounding would take |e| >=
+ * |k| 2^-52/b, which is more.  Above, q can be the next one to it, three halves
+ * away, so |k| up to 3 comes into question: at most ten numerators per divisor,
+ * and b2e_selftest_quotient divides them all.
+ *
+ * Square root: with g next to the midpoint the remainder is an integer multiple
+ * of ulp(g)^2, and a relative error of the factor 1/(2g) below 1.5 2^-53 (here at
+ * most 1.32) cannot move it across the rounding boundary.
+ *
+ * b2e_selftest_rounding and b2e_selftest_quotient compare fp_polish, the quotients
+ * and the square roots with the IEEE operators on the device.
  */
 #ifndef B2E_FP64_CUH
 #define B2E_FP64_CUH
@@ -64,16 +82,16 @@ __device__ __forceinline__ double fp_rsqrt_seed(double d) {
   return y;
 }
 
-/* RN(1/b) from y within two ulp of it */
+/* RN(1/b) from y within sqrt(3) 2^-53 of it, relative */
 __device__ __forceinline__ double fp_polish(double b, double y) { return fp_fix(b, fma(fma(-b, y, 1.0), y, y)); }
 
-/* RN(1/b): four operations behind the seed */
+/* 1/b within 0.5 + 2^-20 ulp, enough for fp_quot: four operations behind the seed */
 __device__ __forceinline__ double fp_recip(double b) {
   const double y0 = fp_rcp_seed(b), e = fma(-b, y0, 1.0), p = fma(e, e, e);
   return fp_fix(b, fma(y0, fma(p, e, e), y0));
 }
 
-/* RN(a/b) from y = 1/b, b > 0.  The remainder is formed with its sign turned
+/* RN(a/b), b > 0, from y = RN(1/b) or fp_recip(b).  The remainder is formed with its sign turned
  * over, so that an exact quotient adds a zero of the opposite sign to q and
  * keeps q, signed zeros included. */
 __device__ __forceinline__ double fp_quot(double a, double b, double y) {

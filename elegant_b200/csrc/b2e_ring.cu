@@ -889,7 +889,8 @@ __device__ __forceinline__ double rounding_operand(uint64_t z, int kind) {
 }
 
 /* counts[0]: quotients through fp_recip, [1]: square roots, [2]: quotients
- * through a root's reciprocal, [3]: fp_polish(fp_recip) against 1/b.  Every
+ * through a root's reciprocal, [3]: polished reciprocals, fp_polish(fp_recip)
+ * against 1/b.  Every
  * second numerator is placed next to the midpoint of two quotients, every
  * second radicand next to the square of a midpoint. */
 __global__ void rounding_selftest_kernel(int64_t samples, uint64_t seed, unsigned long long *counts) {
@@ -938,5 +939,96 @@ extern "C" int b2e_selftest_rounding(int64_t samples, uint64_t seed, int64_t mis
     return B2E_ERR_CUDA;
   for (int c = 0; c < 4; c++)
     mismatches[c] = (int64_t)hm[c];
+  return B2E_OK;
+}
+
+/* ---- quotients next to midpoints (b2e_selftest_quotient) ---------------- */
+namespace b2e {
+
+/* whether fp_quot(a, b, y) rounds every a of [1, 2) right whose quotient by b =
+ * B 2^-52 lies next to a midpoint: A 2^s - M B = k with |k| up to 3, s = 53 for a >=
+ * b (midpoints M 2^-53) and 54 for a < b (M 2^-54), M odd in [2^53, 2^54) */
+__device__ __forceinline__ bool hardest_quotients_right(uint64_t B, double y) {
+  const double b = __longlong_as_double((long long)((B & 0xfffffffffffffull) | 0x3ff0000000000000ull));
+  const int v = B & 1 ? 0 : 1;
+  if (v && !(B & 2)) /* multiples of 4: so is k */
+    return true;
+  uint64_t inv = B >> v; /* of B / 2^v modulo 2^64: Newton doubles the right bits, 3 to begin with */
+  for (int i = 0; i < 5; i++)
+    inv *= 2 - (B >> v) * inv;
+  bool right = true;
+#pragma unroll 1
+  for (int k = -3; k <= 3; k++) {
+    if (k == 0 || (v ? k != 2 && k != -2 : (k & 1) == 0))
+      continue;
+    for (int s = 53; s <= 54; s++) {
+      const uint64_t step = 1ull << (s - v);
+      for (uint64_t M = (0 - (uint64_t)(int64_t)(v ? k / 2 : k) * inv) & (step - 1); M < 1ull << 54; M += step) {
+        const __int128 n = (__int128)((unsigned __int128)M * B) + k; /* A 2^s */
+        const uint64_t A = (uint64_t)(n >> s);
+        if (M >> 53 != 1 || A >> 52 != 1)
+          continue;
+        const double a = __longlong_as_double((long long)((A & 0xfffffffffffffull) | 0x3ff0000000000000ull));
+        right = right && __double_as_longlong(fp_quot(a, b, y)) == __double_as_longlong(a / b);
+      }
+    }
+  }
+  return right;
+}
+
+__global__ void quotient_selftest_kernel(int64_t samples, uint64_t seed, unsigned long long *counts) {
+  unsigned long long n[5] = {0, 0, 0, 0, 0};
+  const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  /* seeds: they follow from the high word, so both ends of its low words bound
+   * the error (and every exponent gives the same significand) */
+  for (int64_t k = first; k < (1 << 21); k += stride) {
+    const uint64_t bits = 0x3ff0000000000000ull | (uint64_t)(k >> 1) << 32 | (k & 1 ? 0xffffffffull : 0);
+    const double b = __longlong_as_double((long long)bits), y0 = fp_rcp_seed(b);
+    const int ex = (int)(rounding_hash(seed ^ bits) % 401) - 200;
+    n[0] += !(fabs(fma(-b, y0, 1.0)) <= 0x1p-19) || fp_rcp_seed(ldexp(b, ex)) != ldexp(y0, -ex) ||
+            y0 != fp_rcp_seed(__longlong_as_double((long long)(bits & ~0xffffffffull)));
+  }
+  /* every significand of the last 2^-18 below 2 */
+  for (int64_t k = first; k < (1ll << 34); k += stride) {
+    const uint64_t B = (1ull << 53) - 1 - (uint64_t)k;
+    const double b = __longlong_as_double((long long)((B & 0xfffffffffffffull) | 0x3ff0000000000000ull));
+    const double y = fp_recip(b);
+    n[1] += __double_as_longlong(y) != __double_as_longlong(1.0 / b);
+    n[2] += !hardest_quotients_right(B, y);
+  }
+  for (int64_t k = first; k < samples; k += stride) {
+    const uint64_t B = (rounding_hash(seed + 0x9E3779B97F4A7C15ull * (uint64_t)(k + 1)) >> 11) | (1ull << 52);
+    const double b = __longlong_as_double((long long)((B & 0xfffffffffffffull) | 0x3ff0000000000000ull));
+    const double y = fp_recip(b);
+    n[3] += __double_as_longlong(y) != __double_as_longlong(1.0 / b);
+    n[4] += !hardest_quotients_right(B, y);
+  }
+  for (int c = 0; c < 5; c++) {
+    for (int off = 16; off > 0; off >>= 1)
+      n[c] += __shfl_down_sync(0xffffffffu, n[c], off);
+    if ((threadIdx.x & 31) == 0 && n[c])
+      atomicAdd(counts + c, n[c]);
+  }
+}
+
+} // namespace b2e
+
+extern "C" int b2e_selftest_quotient(int64_t samples, uint64_t seed, int64_t counts[5]) {
+  using namespace b2e;
+  if (samples < 1 || !counts)
+    return B2E_ERR_ARG;
+  unsigned long long *dm = nullptr, hm[5] = {0, 0, 0, 0, 0};
+  if (cudaMalloc(&dm, sizeof(hm)) != cudaSuccess)
+    return B2E_ERR_NOMEM;
+  cudaMemset(dm, 0, sizeof(hm));
+  quotient_selftest_kernel<<<148 * 8, 256>>>(samples, seed, dm);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaMemcpy(hm, dm, sizeof(hm), cudaMemcpyDeviceToHost);
+  cudaFree(dm);
+  if (e != cudaSuccess)
+    return B2E_ERR_CUDA;
+  for (int c = 0; c < 5; c++)
+    counts[c] = (int64_t)hm[c];
   return B2E_OK;
 }

@@ -564,8 +564,19 @@ int b2e_selftest_division(const double *host_b, int32_t n_b, int64_t samples, ui
  * significands, ones around 1 and around powers of two, short ones, and
  * numerators and radicands placed next to rounding boundaries.  mismatches[0]:
  * quotients by a reciprocal, [1] square roots, [2] quotients by a square root
- * through its reciprocal, [3] reciprocals.  No counterpart in the reference. */
+ * through its reciprocal, [3] reciprocals after the correction that the square
+ * roots' get.  No counterpart in the reference. */
 int b2e_selftest_rounding(int64_t samples, uint64_t seed, int64_t mismatches[4]);
+
+/* ---- quotient self-test --------------------------------------------------
+ * Quotients through the uncorrected reciprocal, which is within 0.5 + 2^-20 ulp
+ * but not always the nearest, where they lie as near to a rounding boundary as
+ * quotients can.  counts[0]: hardware seeds further than 2^-19 from 1/b, over all
+ * their inputs; [1], [2]: every significand within 2^-18 below 2, where the
+ * quotients are in question: reciprocals that are not the nearest, and divisors
+ * with a wrong quotient; [3], [4]: the same for `samples` random significands.
+ * All but [1] and [3] have to be zero.  No counterpart in the reference. */
+int b2e_selftest_quotient(int64_t samples, uint64_t seed, int64_t counts[5]);
 
 /* ---- allocation-free CSR dipole ---------------------------------------
  * No counterpart in the reference: an addition for callers that cannot
