@@ -186,6 +186,18 @@ __device__ __forceinline__ float gelu_grad_at(const float *table, unsigned h, bo
   return table[(h >> 15) * (GG_N + 1) + min(max(k, 0), GG_N)];
 }
 
+/* every BF16 value: the table's float against the formula's, and `beyond`
+ * against |z| >= 8 or not a number */
+__global__ void gelu_grad_selftest_kernel(const float *table, unsigned long long *bad) {
+  const unsigned h = blockIdx.x * blockDim.x + threadIdx.x;
+  const float z = bf16_value(h);
+  bool beyond = false;
+  const float t = gelu_grad_at(table, h, beyond);
+  const bool wrong = beyond != !(fabsf(z) < 8.f) || (!beyond && __float_as_uint(t) != __float_as_uint(gelu_grad_f(z)));
+  if (wrong)
+    atomicAdd(bad, 1ull);
+}
+
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t *>(&h);
@@ -613,6 +625,30 @@ cudaError_t launch_wgrad(const CUtensorMap &t_in, const CUtensorMap &t_dz, const
 } // namespace b2e
 
 using namespace b2e;
+
+extern "C" int b2e_selftest_gelu_grad(int64_t *mismatches) {
+  if (!mismatches)
+    return B2E_ERR_ARG;
+  float *table = nullptr;
+  unsigned long long *dm = nullptr, hm = 0;
+  if (cudaMalloc(&table, GG_BYTES) != cudaSuccess || cudaMalloc(&dm, sizeof(hm)) != cudaSuccess) {
+    cudaFree(table);
+    return B2E_ERR_NOMEM;
+  }
+  cudaError_t e = cudaMemset(dm, 0, sizeof(hm));
+  if (e == cudaSuccess)
+    e = launch_gelu_grad_table(table, 0);
+  if (e == cudaSuccess) {
+    gelu_grad_selftest_kernel<<<256, 256>>>(table, dm);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess)
+    e = cudaMemcpy(&hm, dm, sizeof(hm), cudaMemcpyDeviceToHost);
+  cudaFree(table);
+  cudaFree(dm);
+  *mismatches = (int64_t)hm;
+  return e == cudaSuccess ? B2E_OK : B2E_ERR_CUDA;
+}
 
 extern "C" int b2e_umma_selftest(int mode, const void *dev_a, const void *dev_b, float *dev_d, void *stream) {
   if (mode < 0 || mode > 2 || (mode < 2 && (!dev_a || !dev_b || !dev_d)))

@@ -568,6 +568,13 @@ int b2e_selftest_division(const double *host_b, int32_t n_b, int64_t samples, ui
  * roots' get.  No counterpart in the reference. */
 int b2e_selftest_rounding(int64_t samples, uint64_t seed, int64_t mismatches[4]);
 
+/* ---- wake network's GELU' table self-test ---------------------------------
+ * Compares the table from which the backward pass takes GELU' of BF16 values with
+ * the formula, for all 65,536 of them, bit for bit; *mismatches counts those that
+ * differ, or whose |z| >= 8 or NaN is not told apart.  No counterpart in the
+ * reference. */
+int b2e_selftest_gelu_grad(int64_t *mismatches);
+
 /* ---- quotient self-test --------------------------------------------------
  * Quotients through the uncorrected reciprocal, which is within 0.5 + 2^-20 ulp
  * but not always the nearest, where they lie as near to a rounding boundary as
