@@ -33,6 +33,10 @@ def lattice_spec(lattice) -> str:
     return ";".join(items)
 
 
+class ReferenceMissing(FileNotFoundError):
+    """elegant's own code has not been compiled on this machine."""
+
+
 class RefOracle:
     def __init__(self, math: str = "libm", private: bool = False):
         """private=True loads a fresh copy of the library, so that file-static
@@ -42,7 +46,7 @@ class RefOracle:
         name = "libb2e_ref.so" if math == "libm" else "libb2e_ref_b2emath.so"
         path = os.path.join(REF_DIR, name)
         if not os.path.exists(path):
-            raise FileNotFoundError(path)
+            raise ReferenceMissing(path)
         if private:
             import shutil
             import tempfile
