@@ -85,9 +85,9 @@ __device__ __forceinline__ void expand_range(double *lower, double *upper, doubl
 
 /* Range of c*t per bunch, for kernels whose threads take particles of rising
  * index: each thread keeps the range of the warp's current bunch in registers,
- * and a warp sends its two atomics when the bunch changes and at the end.  One
- * pair per warp of particles, as it was, made 62,500 atomics on two words of a
- * million-particle bunch. */
+ * and a warp sends its two atomics when the bunch changes and at the end.  A pair
+ * for every 32 particles would be 62,500 atomics on two words for a bunch of a
+ * million. */
 struct BunchRange {
   unsigned long long kmin = ~0ull, kmax = 0ull;
   int cur;
@@ -287,11 +287,10 @@ __device__ __forceinline__ void copy4_async(void *smem, const void *gmem) {
  * integrates the current one.  Bound by the FP64 pipe and its register ports:
  * of about 920 warp instructions per 32 particles 430 are FP64, and an fma of
  * three different registers issues every third cycle, not every second.  20 to
- * 32 warps per SM, and two particles per thread, all measured within 2 %.
- * Before, a block per 256 particles waited for the loss word, then for the
- * coordinates, then for the velocity, and every warp sent two atomics to the
- * bunch's range words; here the range stays in registers until the bunch
- * changes. */
+ * 32 warps per SM, and two particles per thread, all measured within 2 %.  48.6 us
+ * for 1e6 particles under ncu; 59.3 us with a block per 256 particles that waits
+ * for the loss word, then for the coordinates, then for the velocity, and two
+ * atomics per warp. */
 template <bool STRAIGHT>
 __global__ void __launch_bounds__(SLICE_THREADS, SLICE_BLOCKS_PER_SM)
     csr_slice_kernel(DevParticles P, int64_t n, int64_t tiles_per_block, const double *beta0,
@@ -516,7 +515,7 @@ __global__ void csr_hist_kernel(DevParticles P, int64_t n, CsrBunches B, unsigne
 }
 
 struct WakeArgs {
-  int nBins, sgHalf, sgdHalf, trapz, steady, correct;
+  int nBins, sgHalf, sgdHalf, trapz, steady;
   /* Savitzky-Golay weights of smoothing and derivative (sg_table) */
   const double *sg_w, *sgd_w;
   double slippage, slippage13, c1, c2, csr_constant;
@@ -622,9 +621,9 @@ __device__ __forceinline__ void sg_apply(const double *in, double *out, int nb, 
   }
 }
 
-/* ((v[0] + v[1]) + v[2]) + ... in index order, as a serial loop forms it: one
- * addition's latency a value (8.4 cycles), eight values loading while eight are
- * added */
+/* ((v[0] + v[1]) + v[2]) + ... in index order, as a serial loop forms it, eight
+ * values loading while eight are added: 10.6 cycles a value measured (600 bins),
+ * 8.4 being the latency of a dependent addition */
 __device__ __forceinline__ double ordered_sum(const double *v, int n) {
   double s = 0, r[8], q[8];
   auto load = [&](double(&to)[8], int from) {
@@ -1265,9 +1264,10 @@ __global__ void __launch_bounds__(BATCH_THREADS, 3)
 
 /* Blocks of the kernels that collect ranges, and the run of particles each
  * takes: an equal share of the whole 256-particle tiles, one tile per block
- * while eight blocks per SM hold them all.  A million particles send 18,944
- * atomics on the bunch's two words instead of 62,500: chicane of 1e6 particles
- * 5.86 -> 5.78 ms, a train of 64 bunches 18.2 -> 17.7 ms. */
+ * while eight blocks per SM hold them all.  A million particles send 15,632
+ * atomics to the bunch's two words instead of the 62,500 of one tile per block:
+ * chicane of 1e6 particles 5.80 ms against 5.87, a train of five bunches 17.72
+ * against 17.99 ms. */
 struct Sweep {
   int grid;
   int64_t share;
@@ -1584,10 +1584,10 @@ __device__ __forceinline__ long long clamp_bins(double d, int nb) {
 
 /* wake of one Stupakov kick, one CTA per bunch (csbend.c:3950-4054): the
  * histogram filters of the last dipole, phi solutions (one warp, each starting
- * from the previous one: the latency of that chain bounds the kernel, 64 us
- * before and about 16 (30,000 cycles) now for 300 bins, with the scan
- * tabulated, the values of a Newton pass side by side and all that is no part
- * of the chain formed by the whole block), then per bin case C, case D's
+ * from the previous one: the latency of that chain bounds the kernel, about 16 us
+ * (30,000 cycles) for 300 bins with the scan tabulated, the values of a Newton
+ * pass side by side and all that is no part of the chain formed by the whole
+ * block; 64 us on one thread), then per bin case C, case D's
  * boundary term and its integral in the reference's order, times -4/rho
  * GSConstant dz0.  Shared memory: 4 nBins + 8 doubles for the filters, nBins
  * for phi. */
@@ -2239,8 +2239,8 @@ static int drift_goes_on(CsrState &st, const std::vector<unsigned char> &flags, 
 /* CSRDRIFT with USE_STUPAKOV=1 (track_through_driftCSR_Stupakov,
  * csbend.c:3803-4159) for the bunches whose mode flag is set; the others get
  * their exact drift in the first kick's drift kernel.  Per kick: drift and c*t
- * with the min/max keys, the histogram of the last dipole's bin count and range factor, the wake (one
- * CTA per bunch), the kick; then the closing half drift. */
+ * with the min/max keys, the histogram of the last dipole's bin count and range
+ * factor, the wake (one CTA per bunch), the kick; then the closing half drift. */
 static int stupakov_drift(CsrState &st, const CsrElem &ce, const CsrBunches &B,
                           const std::vector<unsigned char> &flags, const DevParticles &P, int64_t n, double zStart,
                           cudaStream_t stream, std::string &err, int64_t *launches) {
@@ -2275,7 +2275,6 @@ static int stupakov_drift(CsrState &st, const CsrElem &ce, const CsrBunches &B,
   a.sgHalf = bend.sgHalf;
   a.sgdHalf = bend.sgdHalf;
   a.trapz = bend.trapz;
-  a.correct = bend.sgHalf > 0;
   a.sg_w = sgw;
   a.sgd_w = sgw + sg_width(bend.sgHalf, nb) * sg_width(bend.sgHalf, nb);
   set_filter_args(a, bend.lh, bend.clip, bend.lowCut0, bend.lowCut1, bend.highCut0, bend.highCut1);
@@ -2556,7 +2555,6 @@ int csr_track_element(CsrState &st, const DevElem *d_elems, const DevElem &h_ele
     a.sgdHalf = ce.sgdHalf;
     a.trapz = ce.trapz;
     a.steady = ce.steady;
-    a.correct = ce.sgHalf > 0;
     a.sg_w = sgw;
     a.sgd_w = sgw + sg_width(ce.sgHalf, ce.bins) * sg_width(ce.sgHalf, ce.bins);
     a.slippage = slippage;
@@ -3002,7 +3000,6 @@ extern "C" int b2e_csr_bend_static(double *const dev_columns[6], int32_t *dev_lo
     a.sgdHalf = sgdHalf;
     a.trapz = p[B2E_BEND_TRAPAZOID_INTEGRATION] != 0;
     a.steady = p[B2E_BEND_STEADY_STATE] != 0;
-    a.correct = sgHalf > 0;
     a.sg_w = S->sg_w;
     a.sgd_w = S->sg_w + sg_width(sgHalf, bins) * sg_width(sgHalf, bins);
     a.slippage = slippage;
@@ -3163,7 +3160,6 @@ extern "C" int b2e_csr_wake_batch(const double *dev_counts, const double *dev_sl
   a.sgdHalf = sgd_halfwidth;
   a.trapz = trapezoid != 0;
   a.steady = steady != 0;
-  a.correct = sg_halfwidth > 0;
   a.sg_w = w;
   a.sgd_w = w ? w + w0 * w0 : nullptr;
   a.slippage = 0;

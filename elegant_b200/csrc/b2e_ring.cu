@@ -344,8 +344,8 @@ cudaError_t launch_history_merge(const double *partials, int hist_passes, const 
  * RN(q sum m_i), an integer sum that any order gives.  Arrival times of a bunch
  * behind the first metres of a line nearly always qualify; where they do not,
  * one thread runs the reference's loop on tiles of terms formed by the block.
- * (The loop with its own two divisions and square root per step took 530 ns
- * per particle, 5.3 ms for 10,000.) */
+ * 11 us for 10,000 particles; 28 ns a particle in the loop, 400 ns with the two
+ * divisions and the square root of each term inside it. */
 struct FidAcc {
   unsigned long long lo, hi; /* sums of the significands' low 32 bits and of the rest */
   unsigned long long n, done, m_max;
