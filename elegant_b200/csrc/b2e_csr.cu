@@ -1063,8 +1063,13 @@ __global__ void __launch_bounds__(1024, 1) csr_wake_kernel(CsrBunches B, unsigne
     st->ct_min_key = ~0ull;
     st->ct_max_key = 0ull;
   }
-  if (!active)
+  if (!active) {
+    /* a bunch of a train without a wake on this kick: zeros in the log */
+    if (a.wakelog)
+      for (int b = threadIdx.x; b < a.nBins; b += blockDim.x)
+        a.wakelog[(size_t)bunch * a.nBins + b] = 0;
     return;
+  }
   WakeArgs w = a;
   w.csr_constant = csr_constant;
   w.c1 = csr_constant * a.length / a.nSlices;
@@ -1158,8 +1163,14 @@ __global__ void __launch_bounds__(1024, 1) csr_sur_combine_kernel(CsrBunches B, 
                                        unsigned long long *counters) {
   extern __shared__ double sm[];
   const int b = blockIdx.x, nb = a.nBins;
-  if (!B.active[b])
+  if (!B.active[b]) {
+    if (a.wakelog)
+      for (int i = threadIdx.x; i < nb; i += blockDim.x)
+        a.wakelog[(size_t)b * nb + i] = 0;
+    if (threadIdx.x == 0)
+      gate_log[b] = 0;
     return;
+  }
   CsrDevState *st = B.st + b;
   double *hist = sm, *deriv = sm + nb, *denom = sm + 2 * nb, *red = sm + 3 * nb;
   const double *t = tab + (size_t)b * 3 * B2E_CSR_MAX_BINS;
@@ -1180,6 +1191,8 @@ __global__ void __launch_bounds__(1024, 1) csr_sur_combine_kernel(CsrBunches B, 
       if (wl)
         wl[ib] = 0;
     }
+    if (threadIdx.x == 0)
+      gate_log[b] = 0;
     return;
   }
   long long diS, diS4;
